@@ -39,6 +39,8 @@
 namespace opsec {
 void launch_project_simt(const ProjectArgs& a, cudaStream_t s, long long* launches);
 bool project_tc_supported(const ProjectArgs& a);
+// whether the projection's arc-run tables hold this grid's arcs (else the general key gather)
+bool project_arc_run_ok(const KeySpace& ks);
 void launch_project_tc(const ProjectArgs& a, cudaStream_t s, long long* launches);
 size_t project_tc_work_bytes(const ProjectArgs& a);
 void launch_fisher64(const FisherArgs& a, const double* Dp64, cudaStream_t s, long long* launches);

@@ -170,7 +170,9 @@ struct Step1Params {
 // N3 >= 16) once per slice into its own buffer and expands its rows of the tile from there.
 // Entry e = ((ra (BK/N3) + ca) nf + df) of slice k's table is the word of row arc a0/N3 + ra,
 // column arc k BK/N3 + ca and offset df (zero past the last arc: padding rows and columns).
-constexpr int kArcTab = 288;  // (BM/16) (BK/16) 9 words at N3 = 16, the smallest arc run allowed
+// The run is all of |f_a - f_b|: nf = N3/2 + 1 words on a full-sky grid, N3 words on part of the
+// sky, where N3 = 16 would need 512 words (project_arc_run_ok sends it to the key gather).
+constexpr int kArcTab = 288;  // (BM/16) (BK/16) 9 words at N3 = 16 on the full sky, the largest table
 
 __device__ __forceinline__ int arc_table_size(const KeySpace& ks, int n3) { return (BM / n3) * (BK / n3) * ks.nf; }
 
@@ -654,6 +656,12 @@ Layout layout_of(const ProjectArgs& a) {
 }
 
 }  // namespace
+
+bool project_arc_run_ok(const KeySpace& ks) {
+    const int n3 = ks.N3;
+    return (n3 == 16 || n3 == 32 || n3 == 64) && (BM / n3) * (BK / n3) * ks.nf <= kArcTab &&
+           (long long)(BM / n3) * ks.H * ks.nf < (1LL << 23);
+}
 
 bool project_tc_supported(const ProjectArgs& a) {
     return a.ncells >= 1 && a.nmodes >= 1 && a.nbands >= 1 && a.ncells < (1 << 28);
