@@ -148,9 +148,10 @@ struct XiTableArgs {
     double* r;              // [n] out
     double* xi64;           // [1+nbands][n] out
     float* xi32;            // [1+nbands][n] out
-    double* scratch;        // >= 3 (32769 + nbands*8193) doubles: Simpson weights, weights / k, and
-                            // weights / k as (hi, lo) float pairs
+    double band_wmax;       // widest band, max |band_hi - band_lo|
+    double* scratch;        // xi_scratch_doubles() doubles
 };
+size_t xi_scratch_doubles(const XiTableArgs& a);  // reads xl, nbands and band_wmax
 void launch_xi_tables(const XiTableArgs& a, cudaStream_t s, long long* launches);
 
 // Expand Q[t][key] into the square table Qsq[t][(ha*H+hb)*nf + df] (spherical)

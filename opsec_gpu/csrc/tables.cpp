@@ -26,10 +26,12 @@ void build_tables(opsec_gpu* c) {
     OPSEC_CUDA(cudaMemcpyAsync(c->r_grid.p, r.data(), sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
     c->xi64.alloc((size_t)ntab * n);
     c->xi32.alloc((size_t)ntab * n);
-    c->scratch.alloc(3 * ((size_t)32769 + (size_t)nb * 8193));  // weights, weights / k, (weights / k) as float pairs
     XiTableArgs a;
     a.xl = c->xl;
     a.nbands = nb;
+    a.band_wmax = 0.0;
+    for (int p = 0; p < nb; p++) a.band_wmax = std::max(a.band_wmax, std::fabs(c->band_hi[p] - c->band_lo[p]));
+    c->scratch.alloc(xi_scratch_doubles(a));
     a.pk_x = c->pk_dev.p;
     a.pk_y = a.pk_x + npk;
     a.pk_b = a.pk_y + npk;
