@@ -6,10 +6,7 @@
 // solves the blocks: every eigenvalue of every block (the global top-M cut needs them all), but
 // eigenvectors only for the block eigenvalues that can survive the cut.
 //
-//   1. tridiag_kernel: Householder reduction A = Q T Q^T of every block, one cluster of four CTAs
-//      per block (the lower triangle stays in L2; each step is a fused pass that applies the
-//      previous reflector's rank-2 update and forms the next reflector's product A v).  It runs
-//      in double-FP32 (df64.h) but the reflectors' scalars (FP64, one warp).
+//   1. tridiag.cu: Householder reduction A = Q T Q^T of every block, in double-FP32 (df64.h).
 //   2. spectrum_kernel: every eigenvalue of every T by bisection on FP32 Sturm counts of the
 //      power-of-two-scaled T (to ~1e-6 of the block norm): enough to decide which block
 //      eigenvalues can reach the global cut.
@@ -23,23 +20,16 @@
 //      block norm, where separately computed vectors need not be orthogonal.
 //   6. backtransform_kernel: x = Q z by the stored reflectors (double-FP32), written as the
 //      block's eigenvector column (ascending eigenvalue order, the layout of LAPACK's syevd).
-#include <cooperative_groups.h>
-
 #include <cfloat>
 #include <cmath>
 
 #include "df64.h"
 #include "engine.h"
 
-namespace cg = cooperative_groups;
-
 namespace opsec {
 namespace {
 
-constexpr int kCl = 4;            // CTAs per block in the reduction (one thread-block cluster)
-constexpr int kTT = 512;          // threads per CTA
-constexpr int kTW = kTT / 32;     // warps per CTA
-constexpr int kMaxN = 1024;       // largest block the reduction keeps its per-warp rows for
+constexpr int kMaxN = 1024;  // largest block of the batched form
 
 // Deterministic CTA-wide sum: the same inputs give the same bits in every CTA of the cluster.
 __device__ double cta_sum(double x, double* red) {
@@ -58,222 +48,6 @@ __device__ double cta_sum(double x, double* red) {
     const double r = red[32];
     __syncthreads();
     return r;
-}
-
-// Deterministic CTA-wide double-FP32 sum (lane 0's butterfly result of each warp, then warp
-// 0's): the same inputs give the same bits in every CTA of the cluster.
-__device__ df cta_sum_df(df x, float2* red) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o; o >>= 1)
-        x = df_add(x, df{__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)});
-    if (lane == 0) red[warp] = df_pack(x);
-    __syncthreads();
-    if (warp == 0) {
-        df y = lane < (int)(blockDim.x >> 5) ? df_unpack(red[lane]) : df{0.f, 0.f};
-#pragma unroll
-        for (int o = 16; o; o >>= 1)
-            y = df_add(y, df{__shfl_xor_sync(0xffffffffu, y.h, o), __shfl_xor_sync(0xffffffffu, y.l, o)});
-        if (lane == 0) red[32] = df_pack(y);
-    }
-    __syncthreads();
-    const df r = df_unpack(red[32]);
-    __syncthreads();
-    return r;
-}
-
-// Householder reflector of the pivot column c held in col[c..n) (double-FP32): H = I - tau v v^T
-// with v[c+1] = 1 maps col[c+1..n) onto beta e_{c+1}.  The sum of squares and v in double-FP32,
-// the scalars in FP64 by warp 0 alone (the FP64 pipe issues at 1/64 of the FP32 rate: once per
-// CTA, not in every warp).  sc: tau, beta (FP64); sc2: tau, 1/(x0 - beta) as (hi, lo) pairs.
-// Every CTA of the cluster computes it from the same data and gets the same bits.
-__device__ void householder_df(int n, int c, const float2* col, float2* v, double* sc, float2* sc2, float2* red) {
-    const int t = threadIdx.x;
-    df s{0.f, 0.f};
-    for (int i = c + 2 + t; i < n; i += blockDim.x) {
-        const df x = df_unpack(col[i]);
-        s = df_fma(s, x, x);
-    }
-    const df s2 = cta_sum_df(s, red);
-    if (t < 32) {
-        const double x0 = df_to(df_unpack(col[c + 1])), s2d = df_to(s2);
-        double tau = 0.0, beta = x0, scal = 0.0;
-        if (s2d > 0.0) {
-            const double nrm = sqrt(x0 * x0 + s2d);
-            beta = x0 >= 0.0 ? -nrm : nrm;
-            tau = (beta - x0) / beta;
-            scal = 1.0 / (x0 - beta);
-        }
-        if (t == 0) {
-            sc[0] = tau;
-            sc[1] = beta;
-            sc2[0] = df_pack(df_from(tau));
-            sc2[1] = df_pack(df_from(scal));
-        }
-    }
-    __syncthreads();
-    const df scal = df_unpack(sc2[1]);
-    for (int i = c + 2 + t; i < n; i += blockDim.x) v[i] = df_pack(df_mul(df_unpack(col[i]), scal));
-    if (t == 0) v[c + 1] = make_float2(1.f, 0.f);
-}
-
-// One fused pass over the columns j in [j0, n) of the lower triangle, in double-FP32 (the
-// FP64 pipe is the bound otherwise): a -= v_i w_j + w_i v_j (when upd), then the partial
-// products p += A vn into this warp's row of pw (when sym).  conv: the column still holds FP64
-// values (the first pass), which are read as doubles and written back as (hi, lo) pairs in the
-// same 8 bytes.
-__device__ void fused_pass(int n, int j0, double* __restrict__ A, const float2* vk, const float2* wk,
-                           const float2* vn, float2* pw, bool upd, bool sym, bool conv, int gwarp, int nwarps) {
-    const int lane = threadIdx.x & 31;
-    const int L = n - j0;
-    float2* A2 = reinterpret_cast<float2*>(A);
-    for (int q0 = 0; q0 < L; q0 += nwarps) {
-        // snake order: the long columns at the front go to alternate ends of the warp list
-        const int odd = (q0 / nwarps) & 1;
-        const int q = q0 + (odd ? nwarps - 1 - gwarp : gwarp);
-        if (q >= L) continue;
-        const int j = j0 + q;
-        const size_t cj = (size_t)j * n;
-        const df vkj = upd ? df_unpack(vk[j]) : df{0.f, 0.f}, wkj = upd ? df_unpack(wk[j]) : df{0.f, 0.f};
-        const df vnj = sym ? df_unpack(vn[j]) : df{0.f, 0.f};
-        df cacc{0.f, 0.f};
-        for (int i = j + lane; i < n; i += 32) {
-            df a = conv ? df_from(A[cj + i]) : df_unpack(A2[cj + i]);
-            if (upd) {
-                a = df_fms(a, df_unpack(vk[i]), wkj);
-                a = df_fms(a, df_unpack(wk[i]), vkj);
-            }
-            if (upd || conv) A2[cj + i] = df_pack(a);
-            if (sym) {
-                pw[i] = df_pack(df_fma(df_unpack(pw[i]), a, vnj));
-                if (i != j) cacc = df_fma(cacc, a, df_unpack(vn[i]));
-            }
-        }
-        if (sym) {
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                const df other{__shfl_xor_sync(0xffffffffu, cacc.h, o), __shfl_xor_sync(0xffffffffu, cacc.l, o)};
-                cacc = df_add(cacc, other);
-            }
-            if (lane == 0) pw[j] = df_pack(df_add(df_unpack(pw[j]), cacc));
-        }
-    }
-}
-
-// this CTA's partial A v for rows [i0, n): the warps' rows summed in a fixed order
-__device__ void reduce_warp_rows(int n, int i0, const float2* pw, float2* out) {
-    for (int i = i0 + (int)threadIdx.x; i < n; i += kTT) {
-        df s{0.f, 0.f};
-        for (int w = 0; w < kTW; w++) s = df_add(s, df_unpack(pw[(size_t)w * n + i]));
-        out[i] = df_pack(s);
-    }
-}
-
-// Householder tridiagonalisation of block b = blockIdx.x / kCl (column-major, lower triangle
-// read and updated; n >= 3).  Outputs T (dg, eg), the reflectors V[b][c][i] as (hi, lo) float
-// pairs (v[c+1] = 1) and tau.  Everything runs in double-FP32 but the reflector's scalars
-// (FP64, one warp): the O(n^2) fused pass and the O(n) work of each step (p = A v from the
-// cluster, w, the pivot column, v).
-__global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kTT, 1)
-tridiag_kernel(int n, double* __restrict__ Aall, double* __restrict__ Vall, double* __restrict__ tau,
-               double* __restrict__ dg, double* __restrict__ eg) {
-    extern __shared__ double sm[];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    const int b = blockIdx.x / kCl;
-    const int t = threadIdx.x, warp = t >> 5;
-    double* A = Aall + (size_t)b * n * n;
-    float2* V = reinterpret_cast<float2*>(Vall) + (size_t)b * n * n;
-    float2* vk2 = reinterpret_cast<float2*>(sm);  // (hi, lo): v and w of the step being applied,
-    float2* wk2 = vk2 + n;                        // the next reflector, the pivot column
-    float2* vn2 = wk2 + n;
-    float2* col2 = vn2 + n;
-    float2* buf = col2 + n;           // [2][n] this CTA's partial A v, read by the whole cluster
-    float2* pw = buf + 2 * n;         // [kTW][n] per-warp partial rows
-    float2* red = pw + (size_t)kTW * n;  // 40 pairs
-    double* sc = reinterpret_cast<double*>(red + 40);  // tau, beta of the next reflector
-    float2* sc2 = reinterpret_cast<float2*>(sc + 2);   // tau, 1/(x0 - beta) as pairs
-    float2* pw_mine = pw + (size_t)warp * n;
-    const int gwarp = rank * kTW + warp, nwarps = kCl * kTW;
-    const float2* A2 = reinterpret_cast<const float2*>(A);
-
-    // pivot column 0 and the first reflector
-    for (int i = t; i < n; i += kTT) col2[i] = df_pack(df_from(A[i]));
-    __syncthreads();
-    householder_df(n, 0, col2, vn2, sc, sc2, red);
-    __syncthreads();
-    if (rank == 0) {
-        for (int i = 1 + t; i < n; i += kTT) V[i] = vn2[i];
-        if (t == 0) {
-            dg[(size_t)b * n] = df_to(df_unpack(col2[0]));
-            eg[(size_t)b * n] = sc[1];
-            tau[(size_t)b * n] = sc[0];
-        }
-    }
-    for (int i = 1 + (t & 31); i < n; i += 32) pw_mine[i] = make_float2(0.f, 0.f);
-    __syncthreads();
-    fused_pass(n, 1, A, vk2, wk2, vn2, pw_mine, false, true, true, gwarp, nwarps);
-    __syncthreads();
-    reduce_warp_rows(n, 1, pw, buf);  // parity 0
-    cluster.sync();
-
-    for (int c = 0; c <= n - 3; c++) {
-        const df tc = df_unpack(sc2[0]);
-        // (a) v_c, p_c = A v_c from the four CTAs (fixed order), w_c = y - (tau/2)(y.v) v
-        const float2* rb[kCl];
-#pragma unroll
-        for (int r = 0; r < kCl; r++) rb[r] = cluster.map_shared_rank(buf + (size_t)(c & 1) * n, r);
-        df part{0.f, 0.f};
-        for (int i = c + 1 + t; i < n; i += kTT) {
-            df p = df_unpack(rb[0][i]);
-#pragma unroll
-            for (int r = 1; r < kCl; r++) p = df_add(p, df_unpack(rb[r][i]));
-            const df y = df_mul(tc, p);
-            const float2 v = vn2[i];
-            vk2[i] = v;
-            wk2[i] = df_pack(y);
-            part = df_fma(part, y, df_unpack(v));
-        }
-        const df yv = cta_sum_df(part, red);
-        const df alpha = df_mul(tc, df{0.5f * yv.h, 0.5f * yv.l});
-        for (int i = c + 1 + t; i < n; i += kTT)
-            wk2[i] = df_pack(df_fms(df_unpack(wk2[i]), alpha, df_unpack(vk2[i])));
-        __syncthreads();
-        // (b) pivot column c+1 under the update, the next reflector
-        const int c1 = c + 1;
-        const df vkc = df_unpack(vk2[c1]), wkc = df_unpack(wk2[c1]);
-        for (int i = c1 + t; i < n; i += kTT) {
-            df a = df_unpack(A2[(size_t)c1 * n + i]);
-            a = df_fms(a, df_unpack(vk2[i]), wkc);
-            a = df_fms(a, df_unpack(wk2[i]), vkc);
-            col2[i] = df_pack(a);
-        }
-        __syncthreads();
-        householder_df(n, c1, col2, vn2, sc, sc2, red);
-        __syncthreads();
-        if (rank == 0) {
-            for (int i = c1 + 1 + t; i < n; i += kTT) V[(size_t)c1 * n + i] = vn2[i];
-            if (t == 0) {
-                dg[(size_t)b * n + c1] = df_to(df_unpack(col2[c1]));
-                eg[(size_t)b * n + c1] = sc[1];
-                tau[(size_t)b * n + c1] = sc[0];
-            }
-        }
-        // (c) columns c+2 .. n-1: update by (v_c, w_c); partial A v_{c+1} for the next step
-        const bool sym = c1 <= n - 3;
-        if (sym)
-            for (int i = c1 + 1 + (t & 31); i < n; i += 32) pw_mine[i] = make_float2(0.f, 0.f);
-        __syncthreads();
-        fused_pass(n, c1 + 1, A, vk2, wk2, vn2, pw_mine, true, sym, false, gwarp, nwarps);
-        __syncthreads();
-        if (sym) reduce_warp_rows(n, c1 + 1, pw, buf + (size_t)(c1 & 1) * n);
-        cluster.sync();
-    }
-    if (rank == 0 && t == 0) {
-        dg[(size_t)b * n + n - 1] = df_to(df_unpack(A2[(size_t)(n - 1) * n + n - 1]));
-        eg[(size_t)b * n + n - 1] = 0.0;
-        tau[(size_t)b * n + n - 1] = 0.0;
-    }
 }
 
 // ---------------------------------------------------------------- spectrum (FP32 bisection)
@@ -648,21 +422,7 @@ __global__ void __launch_bounds__(kBT) backtransform_kernel(VecArgs a, const dou
 
 }  // namespace
 
-size_t blockeig_tridiag_smem(int n) { return sizeof(double) * ((size_t)(6 + kTW) * n + 48); }
-
-bool blockeig_supported(int n) {
-    return n >= 3 && n <= kMaxN && blockeig_tridiag_smem(n) <= (size_t)max_dynamic_smem((const void*)tridiag_kernel);
-}
-
-void launch_blockeig_tridiag(int n, int nblk, double* A, double* V, double* tau, double* dg, double* eg,
-                             cudaStream_t s, long long* launches) {
-    const size_t smem = blockeig_tridiag_smem(n);
-    OPSEC_CUDA(cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    max_dynamic_smem((const void*)tridiag_kernel)));
-    tridiag_kernel<<<nblk * kCl, kTT, smem, s>>>(n, A, V, tau, dg, eg);
-    OPSEC_CUDA(cudaGetLastError());
-    ++*launches;
-}
+bool blockeig_supported(int n) { return n >= 3 && n <= kMaxN; }
 
 void launch_blockeig_spectrum(int n, int nblk, const double* dg, const double* eg, double* w, double* scale,
                               cudaStream_t s, long long* launches) {

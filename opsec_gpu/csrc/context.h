@@ -151,7 +151,8 @@ struct opsec_gpu {
     DevBuf<double> nba_dev;      // Nbar per arc
     DevBuf<unsigned char> syev_ws;  // batched eigensolver workspace
     DevBuf<double> bev_V, bev_T, bev_vec;  // hand-written block eigensolver: reflectors, T, vectors
-    DevBuf<int> bev_i;
+    DevBuf<int> bev_i, bev_err;
+    DevBuf<unsigned char> bev_D;  // its working matrix
     DevBuf<int> probe;  // opsec_gpu_wait_probe's status word
     std::string cfg_text;        // the configuration the context was created with
     // learned far-field surrogate: 4 networks (FP32 master weights) and the target scale

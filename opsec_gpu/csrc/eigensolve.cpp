@@ -66,13 +66,20 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     double* eg = dg + (size_t)nblk * n;
     double* scale = eg + (size_t)nblk * n;
     if (g_clock) g_clock->begin("blockeig_tridiag", c->stream, 4.0 / 3.0 * n * nn * nblk);
-    launch_blockeig_tridiag(n, nblk, c->S.p, c->bev_V.p, tau, dg, eg, c->stream, &c->launches);
+    c->bev_D.alloc(tridiag_work_bytes(n, nblk));
+    c->bev_err.alloc(1);
+    OPSEC_CUDA(cudaMemsetAsync(c->bev_err.p, 0, sizeof(int), c->stream));
+    launch_tridiag(n, nblk, c->S.p, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
+                   &c->launches);
     if (g_clock) g_clock->end(c->stream);
     launch_blockeig_spectrum(n, nblk, dg, eg, c->W.p, scale, c->stream, &c->launches);
     std::vector<double> w((size_t)nblk * n), sc(nblk);
     OPSEC_CUDA(cudaMemcpyAsync(w.data(), c->W.p, sizeof(double) * w.size(), cudaMemcpyDeviceToHost, c->stream));
     OPSEC_CUDA(cudaMemcpyAsync(sc.data(), scale, sizeof(double) * nblk, cudaMemcpyDeviceToHost, c->stream));
+    int err = 0;
+    OPSEC_CUDA(cudaMemcpyAsync(&err, c->bev_err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     sync(c);
+    if (err) fail(OPSEC_ERR_CUDA, "tridiagonalisation: a wait between CTAs timed out");
     // the M-th largest approximate eigenvalue, counting the (cos, sin) pairs of 0 < m < Nphi/2 twice
     std::vector<double> all;
     all.reserve((size_t)2 * nblk * n);

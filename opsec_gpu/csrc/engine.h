@@ -205,8 +205,13 @@ void launch_assemble_modes(int H, int Nphi, int Nmu, int npar, int nmodes, const
 // eigenvalue to ~1e-6 of the block scale, then FP64 eigenpairs of the top kc[b] of each block
 // written as columns n-1-c of out (ascending order, as LAPACK's syevd).
 bool blockeig_supported(int n);
-void launch_blockeig_tridiag(int n, int nblk, double* A, double* V, double* tau, double* dg, double* eg,
-                             cudaStream_t s, long long* launches);
+// Householder tridiagonalisation (tridiag.cu) of nblk blocks of order n >= 3 (FP64, column-major,
+// lower triangle read): T = (dg, eg), the reflectors V[block][c][i] as (hi, lo) float pairs
+// (v[c+1] = 1) and tau, each [block][n].  work: tridiag_work_bytes() bytes.  *err (zeroed by the
+// caller) is set when a wait between CTAs ran out.
+size_t tridiag_work_bytes(int n, int nblk);
+void launch_tridiag(int n, int nblk, const double* A, double* V, double* tau, double* dg, double* eg, void* work,
+                    int* err, long long wait_cycles, cudaStream_t s, long long* launches);
 void launch_blockeig_spectrum(int n, int nblk, const double* dg, const double* eg, double* w, double* scale,
                               cudaStream_t s, long long* launches);
 struct BlockEigVectors {
