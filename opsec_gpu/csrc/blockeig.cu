@@ -11,16 +11,18 @@
 //      power-of-two-scaled T (to ~1e-6 of the block norm): enough to decide which block
 //      eigenvalues can reach the global cut.
 //   3. (host) the candidates: per block, the eigenvalues within a safe margin of the cut.
-//   4. vectors_kernel: each candidate's eigenvalue from its FP32 bracket (confirmed by two FP64
-//      Sturm counts, bisected until it holds this eigenvalue alone) by Rayleigh-quotient
-//      iteration on twisted factorisations (the stationary top-down and bottom-up LDL^T
-//      factorisations of T - s I meet at the index where the residual is smallest), then its
-//      eigenvector of T from the last one.
+//   4. vectors_kernel: each candidate's eigenvalue from its FP32 bracket (confirmed by two Sturm
+//      counts, narrowed until it holds this eigenvalue alone) by Rayleigh-quotient iteration on
+//      twisted factorisations (the solutions of (T - s I) x = 0 from the top and from the bottom
+//      meet at the row where the residual is smallest), in double-FP32 and at the end in FP64,
+//      then its eigenvector of T from the last one.
 //   5. cluster_kernel: Gram-Schmidt (twice) inside clusters of candidates closer than 1e-6 of the
 //      block norm, where separately computed vectors need not be orthogonal.
 //   6. backtransform_kernel: x = Q z by the stored reflectors (double-FP32), written as the
 //      block's eigenvector column (ascending eigenvalue order, the layout of LAPACK's syevd).
+#include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 
 #include "df64.h"
@@ -50,17 +52,42 @@ __device__ double cta_sum(double x, double* red) {
     return r;
 }
 
+// ---------------------------------------------------------------- the three-term recurrence
+// Everything below follows the solutions of (T' - s I) x = 0 row by row, T' the block's T with its
+// off-diagonals made -|e_i| (a similarity by signs):
+//   x_{i+1} = ((d_i - s) x_i - |e_{i-1}| x_{i-1}) / |e_i|
+// x_i is the leading i x i minor of T - s I over prod |e|, so its sign changes count the eigenvalues
+// below s (Sturm), and the two solutions from the top and from the bottom are the two halves of a
+// twisted factorisation's eigenvector.  With a_i = (d_i - s) / |e_i| and the ratio |e_{i-1}| / |e_i|
+// tabulated per block a row is three instructions and one FMA of latency; the pivots' form of the
+// same recurrence, q_{i+1} = d - s - e^2 / q_i, waits for a division in every row (FP32 some 60
+// cycles, FP64 several hundred at this part's 1/64 rate).  Solutions grow and decay far beyond the
+// exponent range, so they are rescaled by powers of two every few rows.  |e_i| is held at or above
+// eps/4 of the block's scale, below the rounding of the reduction, which bounds the growth per row.
+constexpr int kGrp32 = 4, kGrp64 = 8;  // rows between rescalings: 27 and 62 bits of growth a row
+
+__device__ __forceinline__ int round_up(int n, int g) { return (n + g - 1) / g * g; }
+
 // ---------------------------------------------------------------- spectrum (FP32 bisection)
-__device__ __forceinline__ int sturm32(int n, const float* d, const float* e2, float s, float pivmin) {
-    float q = d[0] - s;
-    if (fabsf(q) < pivmin) q = -pivmin;
-    int cnt = q < 0.0f;
-    for (int i = 1; i < n; i++) {
-        q = d[i] - s - e2[i - 1] / q;
-        if (fabsf(q) < pivmin) q = -pivmin;
-        cnt += q < 0.0f;
+// row: (d / |e|, 1 / |e|, -|e_{i-1}| / |e|), n a multiple of kGrp32 (rows past the end keep x)
+__device__ __forceinline__ int sturm32(int n, const float4* row, float s) {
+    float x = 1.f, xp = 0.f;
+    unsigned cnt = 0;
+    for (int i = 0; i < n; i += kGrp32) {
+#pragma unroll
+        for (int k = 0; k < kGrp32; k++) {
+            const float4 t = row[i + k];
+            const float y = fmaf(fmaf(-s, t.y, t.x), x, t.z * xp);
+            cnt += (__float_as_uint(y) ^ __float_as_uint(x)) >> 31;
+            xp = x;
+            x = y;
+        }
+        const unsigned e = __float_as_uint(fmaxf(fabsf(x), fabsf(xp))) & 0x7f800000u;
+        const float sc = __uint_as_float(0x7f000000u - e);  // 2^-exponent
+        x *= sc;
+        xp *= sc;
     }
-    return cnt;
+    return (int)cnt;
 }
 
 // Power-of-two scale of a block (>= its Gershgorin bound), so that scaling is exact.
@@ -87,45 +114,37 @@ __device__ double block_scale(int n, const double* d, const double* e, double* r
 __global__ void __launch_bounds__(256) spectrum_kernel(int n, const double* __restrict__ dg,
                                                        const double* __restrict__ eg, double* __restrict__ w,
                                                        double* __restrict__ scale_out) {
-    __shared__ float d[kMaxN], e2[kMaxN];
+    extern __shared__ float4 rows32[];
     __shared__ double red[32];
-    const int b = blockIdx.x;
+    const int b = blockIdx.x, np = round_up(n, kGrp32);
     const double* db = dg + (size_t)b * n;
     const double* ebk = eg + (size_t)b * n;
     const double sc = block_scale(n, db, ebk, red);
     const double inv = 1.0 / sc;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        d[i] = (float)(db[i] * inv);
-        const float ei = (float)(ebk[i] * inv);
-        e2[i] = ei * ei;
+    constexpr float kMinE = 1.4901161193847656e-8f;  // 2^-26
+    for (int i = threadIdx.x; i < np; i += blockDim.x) {
+        float4 t = make_float4(1.f, 0.f, 0.f, 0.f);
+        if (i < n) {
+            const float e = i + 1 < n ? fmaxf(fabsf((float)(ebk[i] * inv)), kMinE) : 1.f;
+            const float ep = i > 0 ? fmaxf(fabsf((float)(ebk[i - 1] * inv)), kMinE) : 0.f;
+            t = make_float4((float)(db[i] * inv) / e, 1.f / e, -ep / e, 0.f);
+        }
+        rows32[i] = t;
     }
     __syncthreads();
     if (blockIdx.y == 0 && threadIdx.x == 0) scale_out[b] = sc;
     const int j = blockIdx.y * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const float pivmin = 1e-30f;
     float lo = -1.0f, hi = 1.0f;  // the scaled spectrum lies in (-1, 1)
     for (int it = 0; it < 40 && hi - lo > 2.5e-7f; it++) {
         const float mid = 0.5f * (lo + hi);
-        if (sturm32(n, d, e2, mid, pivmin) > j) hi = mid;
+        if (sturm32(np, rows32, mid) > j) hi = mid;
         else lo = mid;
     }
     w[(size_t)b * n + j] = 0.5 * ((double)lo + (double)hi) * sc;
 }
 
 // ---------------------------------------------------------------- candidate eigenpairs (FP64)
-__device__ __forceinline__ int sturm64(int n, const double* d, const double* e2, double s, double pivmin) {
-    double q = d[0] - s;
-    if (fabs(q) < pivmin) q = -pivmin;
-    int cnt = q < 0.0;
-    for (int i = 1; i < n; i++) {
-        q = d[i] - s - e2[i - 1] / q;
-        if (fabs(q) < pivmin) q = -pivmin;
-        cnt += q < 0.0;
-    }
-    return cnt;
-}
-
 struct VecArgs {
     int n, nblk, ktot;
     const int* kc;       // [nblk] candidates per block (the top kc[b] eigenvalues)
@@ -135,192 +154,540 @@ struct VecArgs {
     const double* scale; // [nblk] power-of-two scale of each block
     double* w;           // [nblk][n] ascending: approximate in, candidates refined out
     double* Z;           // [n][ktot] eigenvectors of T, then of the block
-    double* L;           // [n][ktot] scratch: top-down multipliers
-    double* U;           // [n][ktot] scratch: bottom-up multipliers
-    double* G;           // [n][ktot] scratch: top-down pivots
+    int* KX;             // scratch: exponents of groups of rows of X, then of Y ([ceil(n/2)][ktot] each)
+    double* X;           // [n][ktot] scratch: the solution from the top
+    double* Y;           // [n][ktot] scratch: the solution from the bottom
     int* status;         // [nblk]: 0, or 1 when a bracket could not be confirmed, 2 when a cluster degenerated
 };
 
-// Twisted factorisation of T - s I (scaled T).  The stationary top-down pivots G_i (with the
-// multipliers L_i = e_i / G_i) and the bottom-up pivots H_i (U_i = e_{i-1} / H_i) meet at the
-// twist index r where |gamma_r| = |G_r + H_r - (d_r - s)| is least; the vector with z_r = 1
-// has z_i = -L_i z_{i+1} above r and z_i = -U_i z_{i-1} below it.  Its squared norm at every
-// twist follows from two recurrences, S_{i+1} = L_i^2 (1 + S_i) from the top and
-// B_{i-1} = U_i^2 (1 + B_i) from the bottom, so |z|^2 = S_r + 1 + B_r without forming z.
-// rq_step: one pass each way; returns the Rayleigh-quotient correction gamma_r / |z|^2.  The
-// top-down pass keeps G and S in the scratch columns (they are read back, in an order that
-// does not depend on the recurrence, by the bottom-up pass).
-__device__ double rq_step(int n, const double* d, const double* e, double s, double pivmin, size_t K,
-                          double* __restrict__ Gc, double* __restrict__ Sc, int* r_out) {
-    double g = d[0] - s, sn = 0.0;
-    if (fabs(g) < pivmin) g = -pivmin;
-    for (int i = 0; i + 1 < n; i++) {
-        Gc[i * K] = g;
-        Sc[i * K] = sn;
-        const double l = e[i] / g;
-        sn = l * l * (1.0 + sn);
-        g = d[i + 1] - s - l * e[i];
-        if (fabs(g) < pivmin) g = -pivmin;
+// Per block, in shared memory: the rows of both recurrences (np = n rounded up to kGrp64).
+struct Rows64 {
+    const double *ff, *fi, *fb;  // from the top: d/|e_i|, 1/|e_i|, -|e_{i-1}|/|e_i|
+    const double *bf, *bb;       // from the bottom: d/|e_{i-1}|, -|e_i|/|e_{i-1}| (1/|e_{i-1}| is fi[i-1])
+};
+
+// 2^-e for the exponent e of x (x normal), and e
+__device__ __forceinline__ double exp_scale(double x, int* e) {
+    const int h = (__double2hiint(x) >> 20) & 0x7ff;
+    *e = h - 1023;
+    return __hiloint2double((2046 - h) << 20, 0);
+}
+__device__ __forceinline__ unsigned hi_xor(double a, double b) { return (unsigned)(__double2hiint(a) ^ __double2hiint(b)); }
+
+constexpr int kShifts = 2;  // Sturm counts at a time: independent recurrences under one row's latency
+
+// eigenvalues below each shift
+__device__ void sturm64(int np, const Rows64& t, const double (&s)[kShifts], int (&cnt)[kShifts]) {
+    double x[kShifts], xp[kShifts];
+    unsigned c[kShifts];
+#pragma unroll
+    for (int q = 0; q < kShifts; q++) {
+        x[q] = 1.0;
+        xp[q] = 0.0;
+        c[q] = 0;
     }
-    // twist at n-1: gamma = G_{n-1}, |z|^2 = S_{n-1} + 1
-    int r = n - 1;
-    double gam_r = g, best = fabs(g), nz = sn + 1.0;
-    double h = d[n - 1] - s, bn = 0.0;
-    if (fabs(h) < pivmin) h = -pivmin;
-    double gnext = Gc[(size_t)(n - 2) * K], snext = Sc[(size_t)(n - 2) * K];
-    for (int i = n - 1; i >= 1; i--) {
-        const double gi = gnext, si = snext;  // G_{i-1}, S_{i-1}
-        if (i >= 2) {
-            gnext = Gc[(size_t)(i - 2) * K];
-            snext = Sc[(size_t)(i - 2) * K];
+    for (int i = 0; i < np; i += kGrp64) {
+#pragma unroll
+        for (int k = 0; k < kGrp64; k++) {
+            const double f = t.ff[i + k], g = t.fi[i + k], b = t.fb[i + k];
+#pragma unroll
+            for (int q = 0; q < kShifts; q++) {
+                const double y = fma(fma(-s[q], g, f), x[q], b * xp[q]);
+                c[q] += hi_xor(y, x[q]) >> 31;
+                xp[q] = x[q];
+                x[q] = y;
+            }
         }
-        const double u = e[i - 1] / h;
-        bn = u * u * (1.0 + bn);
-        h = d[i - 1] - s - u * e[i - 1];
-        if (fabs(h) < pivmin) h = -pivmin;
-        const double gam = gi + h - (d[i - 1] - s);
-        if (fabs(gam) < best) {
-            best = fabs(gam);
-            gam_r = gam;
-            r = i - 1;
-            nz = si + 1.0 + bn;
+#pragma unroll
+        for (int q = 0; q < kShifts; q++) {
+            int e;
+            const double sc = exp_scale(fmax(fabs(x[q]), fabs(xp[q])), &e);
+            x[q] *= sc;
+            xp[q] *= sc;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kShifts; q++) cnt[q] = (int)c[q];
+}
+
+// The same counts in double-FP32 (47 bits; rescaled every row, FP32's exponent range being short):
+// FP64 instructions take 64 cycles a warp on one scheduler's pipe, three of them a row.
+struct RowsDf {
+    const float2 *f, *g, *b;  // d/|e_i|, 1/|e_i|, -|e_{i-1}|/|e_i| as (hi, lo) pairs
+};
+__device__ void sturm_df(int np, const RowsDf& t, const double (&s)[kShifts], int (&cnt)[kShifts]) {
+    df x[kShifts], xp[kShifts], ms[kShifts];
+    unsigned c[kShifts];
+#pragma unroll
+    for (int q = 0; q < kShifts; q++) {
+        x[q] = df{1.f, 0.f};
+        xp[q] = df{0.f, 0.f};
+        ms[q] = df_from(-s[q]);
+        c[q] = 0;
+    }
+#pragma unroll 2
+    for (int i = 0; i < np; i++) {
+        const df f = df_unpack(t.f[i]), g = df_unpack(t.g[i]), b = df_unpack(t.b[i]);
+#pragma unroll
+        for (int q = 0; q < kShifts; q++) {
+            const df y = df_fma(df_mul(b, xp[q]), df_fma(f, ms[q], g), x[q]);
+            c[q] += (__float_as_uint(y.h) ^ __float_as_uint(x[q].h)) >> 31;
+            const unsigned e = __float_as_uint(fmaxf(fabsf(y.h), fabsf(x[q].h))) & 0x7f800000u;
+            const float sc = __uint_as_float(0x7f000000u - e);  // 2^-exponent
+            xp[q] = df{x[q].h * sc, x[q].l * sc};
+            x[q] = df{y.h * sc, y.l * sc};
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kShifts; q++) cnt[q] = (int)c[q];
+}
+
+// One step of the search for eigenvalue j in (lo, hi), which hold clo and chi eigenvalues below
+// them: the bracket's interior shifts, evenly spaced.  False when they no longer separate.
+template <class Count>
+__device__ bool narrow(Count count, int j, double* lo, double* hi, int* clo, int* chi) {
+    double s[kShifts];
+    int c[kShifts];
+    bool apart = true;
+#pragma unroll
+    for (int q = 0; q < kShifts; q++) {
+        s[q] = *lo + (*hi - *lo) * ((q + 1) / (double)(kShifts + 1));
+        apart = apart && s[q] > (q ? s[q - 1] : *lo);
+    }
+    if (!apart || !(s[kShifts - 1] < *hi)) return false;
+    count(s, c);
+    double l = *lo, h = *hi;
+    int cl = *clo, ch = *chi;
+#pragma unroll
+    for (int q = kShifts - 1; q >= 0; q--)
+        if (c[q] > j) {
+            h = s[q];
+            ch = c[q];
+        }
+#pragma unroll
+    for (int q = 0; q < kShifts; q++)
+        if (c[q] <= j && s[q] < h) {
+            l = s[q];
+            cl = c[q];
+        }
+    *lo = l;
+    *hi = h;
+    *clo = cl;
+    *chi = ch;
+    return true;
+}
+
+// 2^k, zero far below the smallest normal
+__device__ __forceinline__ double pow2i(int k) { return k < -1000 ? 0.0 : __hiloint2double((min(k, 1000) + 1023) << 20, 0); }
+
+// Twisted factorisation at s: the solutions from the top (X) and from the bottom (Y), meeting at
+// the row r where |x_r y_r| is largest: (T - s I)^{-1}_{rr} is x_r y_r over their (constant)
+// Wronskian, so that is where the residual gamma_r of z = (x_i / x_r above, 1, y_i / y_r below) is
+// least.  Entries carry the exponent of their group of kGrp64 rows.  Returns the
+// Rayleigh-quotient correction gamma_r / |z|^2; |z|^2 in *nz_out.
+__device__ double rq_step(int n, const Rows64& t, const double* __restrict__ d, const double* __restrict__ e, double inv,
+                          double s, const VecArgs& a, int col, int* r_out, double* nz_out) {
+    const size_t K = (size_t)a.ktot;
+    double* X = a.X + col;
+    double* Y = a.Y + col;
+    const int ngrp = (n + kGrp64 - 1) / kGrp64;
+    int* KX = a.KX + col;
+    int* KY = KX + (size_t)ngrp * K;
+    double x = 1.0, xp = 0.0, y = 1.0, yp = 0.0;
+    int kx = 0, ky = 0;
+    for (int g = 0; g < ngrp; g++) {
+        // from the top rows of group g, from the bottom rows of group ngrp-1-g (rows past n keep y = 1)
+        KX[g * K] = kx;
+        KY[(ngrp - 1 - g) * K] = ky;
+#pragma unroll
+        for (int k = 0; k < kGrp64; k++) {
+            const int i = g * kGrp64 + k, j = (ngrp - g) * kGrp64 - 1 - k;
+            if (i < n) X[i * K] = x;
+            if (j < n) Y[j * K] = y;
+            const double xn = fma(fma(-s, t.fi[i], t.ff[i]), x, t.fb[i] * xp);
+            const double yn = fma(fma(-s, t.fi[max(j - 1, 0)], t.bf[j]), y, t.bb[j] * yp);
+            xp = x;
+            x = xn;
+            yp = y;
+            y = j < n ? yn : y;
+        }
+        int ex, ey;
+        const double sx = exp_scale(fmax(fabs(x), fabs(xp)), &ex), sy = exp_scale(fmax(fabs(y), fabs(yp)), &ey);
+        x *= sx;
+        xp *= sx;
+        y *= sy;
+        yp *= sy;
+        kx += ex;
+        ky += ey;
+    }
+    // the twist: log2 |x_r y_r| to 0.1 from the high words; kB rows' loads at a time, without branches
+    constexpr int kB = 4 * kGrp64;
+    int r = 0, best = INT_MIN;
+    for (int i0 = 0; i0 < n; i0 += kB) {
+        int l[kB], kg[kB / kGrp64];
+#pragma unroll
+        for (int u = 0; u < kB / kGrp64; u++) {
+            const int g = min(i0 / kGrp64 + u, ngrp - 1);
+            kg[u] = (KX[g * K] + KY[g * K]) << 10;
+        }
+#pragma unroll
+        for (int k = 0; k < kB; k++) {
+            const size_t o = (size_t)min(i0 + k, n - 1) * K;
+            l[k] = ((__double2hiint(X[o]) & 0x7fffffff) >> 10) + ((__double2hiint(Y[o]) & 0x7fffffff) >> 10);
+        }
+#pragma unroll
+        for (int k = 0; k < kB; k++) {
+            const int v = l[k] + kg[k / kGrp64];
+            if (i0 + k < n && v > best) {
+                best = v;
+                r = i0 + k;
+            }
+        }
+    }
+    // entries above and below r relative to it
+    const double xr = 1.0 / X[r * K], yr = 1.0 / Y[r * K];
+    const int kxr = KX[(r / kGrp64) * K], kyr = KY[(r / kGrp64) * K];
+    double gamma = d[r] * inv - s;
+    if (r > 0) gamma -= fabs(e[r - 1]) * inv * (X[(r - 1) * K] * xr * pow2i(KX[((r - 1) / kGrp64) * K] - kxr));
+    if (r + 1 < n) gamma -= fabs(e[r]) * inv * (Y[(r + 1) * K] * yr * pow2i(KY[((r + 1) / kGrp64) * K] - kyr));
+    double nz = 1.0;
+    for (int i0 = 0; i0 < n; i0 += kB) {
+        double v[kB], fx[kB / kGrp64], fy[kB / kGrp64];
+#pragma unroll
+        for (int u = 0; u < kB / kGrp64; u++) {
+            const int g = min(i0 / kGrp64 + u, ngrp - 1);
+            fx[u] = pow2i(KX[g * K] - kxr);
+            fy[u] = pow2i(KY[g * K] - kyr);
+        }
+#pragma unroll
+        for (int k = 0; k < kB; k++) {
+            const int i = min(i0 + k, n - 1);
+            v[k] = (i < r ? X : Y)[(size_t)i * K];
+        }
+#pragma unroll
+        for (int u = 0; u < kB / kGrp64; u++) {
+            fx[u] *= xr;
+            fy[u] *= yr;
+        }
+#pragma unroll
+        for (int k = 0; k < kB; k++) {
+            const int i = i0 + k;
+            const double zi = v[k] * (i < r ? fx[k / kGrp64] : fy[k / kGrp64]);
+            nz = fma(zi, i < n && i != r ? zi : 0.0, nz);
         }
     }
     *r_out = r;
-    return gam_r / nz;
+    *nz_out = nz;
+    return gamma / nz;
 }
 
-// The eigenvector at s with twist r into column Zc (stride K), unnormalised, |z|^2 in *nrm_out;
-// Lc, Uc scratch columns.
-__device__ void twisted_vector(int n, const double* d, const double* e, double s, double pivmin, int r, size_t K,
-                               double* __restrict__ Lc, double* __restrict__ Uc, double* __restrict__ Zc,
-                               double* nrm_out) {
-    double g = d[0] - s;
-    if (fabs(g) < pivmin) g = -pivmin;
-    for (int i = 0; i < r; i++) {
-        const double l = e[i] / g;
-        Lc[i * K] = l;
-        g = d[i + 1] - s - l * e[i];
-        if (fabs(g) < pivmin) g = -pivmin;
+// The first step of the iteration in double-FP32: the same solutions from both ends (exponents per
+// kGrpDf rows), the twist row r, |z|^2 there in FP32 (it only scales the correction) and the
+// correction.  tb: the rows of the recurrence from the bottom.
+constexpr int kGrpDf = 2;
+struct RowsDfB {
+    const float2 *f, *b;  // d/|e_{i-1}|, -|e_i|/|e_{i-1}| (1/|e_{i-1}| is RowsDf::g[i-1])
+};
+__device__ __forceinline__ df rescaled(df v, float sc) { return df{v.h * sc, v.l * sc}; }
+__device__ __forceinline__ float exp_scale(df a, df b, int* e) {
+    const unsigned h = __float_as_uint(fmaxf(fabsf(a.h), fabsf(b.h))) & 0x7f800000u;
+    *e = (int)(h >> 23) - 127;
+    return __uint_as_float(0x7f000000u - h);
+}
+// d_r - s - |e_{r-1}| x_{r-1}/x_r - |e_r| y_{r+1}/y_r, the ratios given
+__device__ __forceinline__ double gamma_of(int n, const double* d, const double* e, double inv, double s, int r, double tx,
+                                           double ty) {
+    double g = d[r] * inv - s;
+    if (r > 0) g -= fabs(e[r - 1]) * inv * tx;
+    if (r + 1 < n) g -= fabs(e[r]) * inv * ty;
+    return g;
+}
+__device__ double rq_first(int n, const RowsDf& t, const RowsDfB& tb, const double* __restrict__ d,
+                           const double* __restrict__ e, double inv, double s, const VecArgs& a, int col, int* r_out,
+                           double* nz_out) {
+    const size_t K = (size_t)a.ktot;
+    float2* X = reinterpret_cast<float2*>(a.X) + col;
+    float2* Y = reinterpret_cast<float2*>(a.Y) + col;
+    const int ngrp = (n + kGrpDf - 1) / kGrpDf;
+    int* KX = a.KX + col;
+    int* KY = KX + (size_t)ngrp * K;
+    const df ms = df_from(-s);
+    df x{1.f, 0.f}, xp{0.f, 0.f}, y{1.f, 0.f}, yp{0.f, 0.f};
+    int kx = 0, ky = 0;
+    for (int g = 0; g < ngrp; g++) {
+        KX[g * K] = kx;
+        KY[(ngrp - 1 - g) * K] = ky;
+#pragma unroll
+        for (int k = 0; k < kGrpDf; k++) {
+            const int i = g * kGrpDf + k, j = (ngrp - g) * kGrpDf - 1 - k;
+            if (i < n) X[i * K] = df_pack(x);
+            if (j < n) Y[j * K] = df_pack(y);
+            const df xn = df_fma(df_mul(df_unpack(t.b[i]), xp), df_fma(df_unpack(t.f[i]), ms, df_unpack(t.g[i])), x);
+            const df yn = df_fma(df_mul(df_unpack(tb.b[j]), yp),
+                                 df_fma(df_unpack(tb.f[j]), ms, df_unpack(t.g[max(j - 1, 0)])), y);
+            xp = x;
+            x = xn;
+            yp = y;
+            if (j < n) y = yn;
+        }
+        int ex, ey;
+        const float sx = exp_scale(x, xp, &ex), sy = exp_scale(y, yp, &ey);
+        x = rescaled(x, sx);
+        xp = rescaled(xp, sx);
+        y = rescaled(y, sy);
+        yp = rescaled(yp, sy);
+        kx += ex;
+        ky += ey;
     }
-    double h = d[n - 1] - s;
-    if (fabs(h) < pivmin) h = -pivmin;
-    for (int i = n - 1; i > r; i--) {
-        const double u = e[i - 1] / h;
-        Uc[i * K] = u;
-        h = d[i - 1] - s - u * e[i - 1];
-        if (fabs(h) < pivmin) h = -pivmin;
+    constexpr int kB = 32;  // rows' loads at a time, without branches
+    int r = 0, best = INT_MIN;
+    for (int i0 = 0; i0 < n; i0 += kB) {
+        int l[kB];
+#pragma unroll
+        for (int k = 0; k < kB; k++) {
+            const int i = min(i0 + k, n - 1);
+            const size_t o = (size_t)i * K, og = (size_t)(i / kGrpDf) * K;
+            l[k] = ((KX[og] + KY[og]) << 10) + ((__float_as_int(X[o].x) & 0x7fffffff) >> 13) +
+                   ((__float_as_int(Y[o].x) & 0x7fffffff) >> 13);
+        }
+#pragma unroll
+        for (int k = 0; k < kB; k++)
+            if (i0 + k < n && l[k] > best) {
+                best = l[k];
+                r = i0 + k;
+            }
     }
-    double nrm = 1.0, z = 1.0;
-    Zc[(size_t)r * K] = 1.0;
-    for (int i = r - 1; i >= 0; i--) {
-        z = -Lc[i * K] * z;
-        Zc[i * K] = z;
-        nrm += z * z;
+    auto pow2f = [](int k) { return k < -126 ? 0.f : __int_as_float((min(k, 126) + 127) << 23); };
+    const int kxr = KX[(r / kGrpDf) * K], kyr = KY[(r / kGrpDf) * K];
+    const float xr = 1.0f / X[r * K].x, yr = 1.0f / Y[r * K].x;
+    float nz = 1.f;
+    for (int i0 = 0; i0 < n; i0 += kB) {
+        float v[kB], f[kB];
+#pragma unroll
+        for (int k = 0; k < kB; k++) {
+            const int i = min(i0 + k, n - 1);
+            const bool top = i < r;
+            v[k] = (top ? X : Y)[(size_t)i * K].x;
+            f[k] = pow2f((top ? KX : KY)[(size_t)(i / kGrpDf) * K] - (top ? kxr : kyr));
+        }
+#pragma unroll
+        for (int k = 0; k < kB; k++) {
+            const int i = i0 + k;
+            const float zi = v[k] * (i < r ? xr : yr) * f[k];
+            if (i < n && i != r) nz = fmaf(zi, zi, nz);
+        }
     }
-    z = 1.0;
-    for (int i = r + 1; i < n; i++) {
-        z = -Uc[i * K] * z;
-        Zc[i * K] = z;
-        nrm += z * z;
-    }
-    *nrm_out = nrm;
+    double tx = 0.0, ty = 0.0;
+    if (r > 0)
+        tx = df_to(df_unpack(X[(r - 1) * K])) / df_to(df_unpack(X[r * K])) * pow2i(KX[((r - 1) / kGrpDf) * K] - kxr);
+    if (r + 1 < n)
+        ty = df_to(df_unpack(Y[(r + 1) * K])) / df_to(df_unpack(Y[r * K])) * pow2i(KY[((r + 1) / kGrpDf) * K] - kyr);
+    *r_out = r;
+    *nz_out = (double)nz;
+    return gamma_of(n, d, e, inv, s, r, tx, ty) / (double)nz;
 }
 
-// grid (nblk, ceil(n/32)), 32 threads: candidate c (0 = largest) of block b per thread.
-// The FP32 estimate's bracket is confirmed by two FP64 Sturm counts.  An eigenvalue alone in
+// gamma_r at s for a given twist row: the solution from the top down to r, then the one from the
+// bottom up to r, in double-FP32; nothing is stored.
+__device__ double gamma_df(int n, const RowsDf& t, const RowsDfB& tb, const double* __restrict__ d,
+                           const double* __restrict__ e, double inv, double s, int r) {
+    const df ms = df_from(-s);
+    df x{1.f, 0.f}, xp{0.f, 0.f};
+    double tx = 0.0;
+    for (int q = 0; q < n - 1; q++) {
+        const bool top = q < r;
+        if (q == r) {  // x holds row r of the solution from the top
+            tx = r > 0 ? df_to(xp) / df_to(x) : 0.0;
+            x = df{1.f, 0.f};
+            xp = df{0.f, 0.f};
+        }
+        const int i = top ? q : n - 1 - (q - r);
+        const df f = df_unpack((top ? t.f : tb.f)[i]), b = df_unpack((top ? t.b : tb.b)[i]);
+        const df g = df_unpack(t.g[top ? i : i - 1]);
+        const df y = df_fma(df_mul(b, xp), df_fma(f, ms, g), x);
+        int ex;
+        const float sc = exp_scale(y, x, &ex);
+        xp = rescaled(x, sc);
+        x = rescaled(y, sc);
+    }
+    const double ratio = df_to(xp) / df_to(x);
+    return gamma_of(n, d, e, inv, s, r, r == n - 1 ? ratio : tx, r == n - 1 ? 0.0 : ratio);
+}
+
+// grid (nblk, parts of kc), 4 warps of `per` candidates each, one per thread: candidate c (0 =
+// largest) of block b.  An FP64 instruction takes a warp 64 cycles of its scheduler's pipe however
+// many of its lanes work, so the candidates are dealt over all schedulers of the chip.
+// The FP32 estimate's bracket is confirmed by FP64 Sturm counts.  An eigenvalue alone in
 // its bracket is refined by Rayleigh-quotient iteration on twisted factorisations (cubic
 // convergence; the iterate must stay in the bracket); an eigenvalue sharing its bracket is
-// bisected to full precision first.  The last twisted factorisation gives the vector.
-__global__ void __launch_bounds__(32) vectors_kernel(VecArgs a) {
-    __shared__ double d[kMaxN], e[kMaxN], e2[kMaxN];
-    const int b = blockIdx.x, n = a.n;
+// narrowed down first.  The last twisted factorisation gives the vector.
+// Bound by the FP64 pipe (64 cycles an instruction, measured, with nothing to overlap) and by loads of the stored solutions (32 rows at a time: row by row their latency was half the kernel).
+// Candidates of 34 blocks of 512^2 (4,351): 4.51 -> 1.15 ms against FP64 pivots with a division in
+// every row; 34 of 1024^2 25.5 -> 3.77, 10 of 555^2 12.5 -> 2.01, 18 of 64^2 0.406 -> 0.092.
+__global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, int per) {
+    extern __shared__ double rows64[];
+    const int b = blockIdx.x, n = a.n, np = round_up(n, kGrp64);
     const int kc = a.kc[b];
-    if ((int)blockIdx.y * 32 >= kc) return;
+    if ((int)blockIdx.y * 4 * per >= kc) return;
     const double sc = a.scale[b], inv = 1.0 / sc;
-    for (int i = threadIdx.x; i < n; i += 32) {
-        d[i] = a.dg[(size_t)b * n + i] * inv;
-        e[i] = a.eg[(size_t)b * n + i] * inv;
-        e2[i] = e[i] * e[i];
+    const double* dgb = a.dg + (size_t)b * n;
+    const double* egb = a.eg + (size_t)b * n;
+    const Rows64 t{rows64, rows64 + np, rows64 + 2 * np, rows64 + 3 * np, rows64 + 4 * np};
+    float2* rowsf = reinterpret_cast<float2*>(rows64 + 5 * np);
+    const RowsDf tf{rowsf, rowsf + np, rowsf + 2 * np};
+    const RowsDfB tfb{rowsf + 3 * np, rowsf + 4 * np};
+    constexpr double kMinE = 8.673617379884035e-19;  // 2^-60
+    for (int i = threadIdx.x; i < np; i += 128) {
+        double ff = 1.0, fi = 0.0, fb = 0.0, bf = 0.0, bb = 0.0;  // rows past the end keep x
+        if (i < n) {
+            const double d = dgb[i] * inv;
+            const double e = i + 1 < n ? fmax(fabs(egb[i] * inv), kMinE) : 1.0;
+            const double ep = i > 0 ? fmax(fabs(egb[i - 1] * inv), kMinE) : 1.0;
+            fi = 1.0 / e;
+            ff = d * fi;
+            fb = i > 0 ? -ep * fi : 0.0;
+            bf = d / ep;
+            bb = i + 1 < n ? -e / ep : 0.0;
+        }
+        rows64[i] = ff;
+        rows64[np + i] = fi;
+        rows64[2 * np + i] = fb;
+        rows64[3 * np + i] = bf;
+        rows64[4 * np + i] = bb;
+        rowsf[i] = df_pack(df_from(ff));
+        rowsf[np + i] = df_pack(df_from(fi));
+        rowsf[2 * np + i] = df_pack(df_from(fb));
+        rowsf[3 * np + i] = df_pack(df_from(bf));
+        rowsf[4 * np + i] = df_pack(df_from(bb));
     }
     __syncthreads();
-    const int c = blockIdx.y * 32 + threadIdx.x;
-    if (c >= kc) return;
+    const int lane = threadIdx.x & 31, c = (blockIdx.y * 4 + (threadIdx.x >> 5)) * per + lane;
+    if (lane >= per || c >= kc) return;
     const int j = n - 1 - c;  // ascending index
     const int col = a.koff[b] + c;
     const size_t K = (size_t)a.ktot;
-    const double pivmin = 1e-290;
     const double x = a.w[(size_t)b * n + j] * inv;
-    double del = 8.0 * FLT_EPSILON, lo = x - del, hi = x + del;
-    int clo = 0, chi = 0;
-    bool ok = false;
-    for (int k = 0; k < 8 && !ok; k++) {
-        lo = x - del;
-        hi = x + del;
-        clo = sturm64(n, d, e2, lo, pivmin);
-        chi = sturm64(n, d, e2, hi, pivmin);
-        ok = clo <= j && chi > j;
-        del *= 8.0;
+    auto count_df = [&](const double (&sh)[kShifts], int (&cn)[kShifts]) { sturm_df(np, tf, sh, cn); };
+    auto count64 = [&](const double (&sh)[kShifts], int (&cn)[kShifts]) { sturm64(np, t, sh, cn); };
+    // the FP32 estimate's bracket, confirmed
+    double del = 8.0 * FLT_EPSILON, lo = -1.0, hi = 1.0;  // the scaled spectrum lies inside (-1, 1)
+    int clo = 0, chi = n;
+    for (int k = 0; k < 8 && (lo == -1.0 || hi == 1.0); k++, del *= 8.0) {
+        const double sh[kShifts] = {x - del, x + del};
+        int cn[kShifts];
+        count_df(sh, cn);
+        if (cn[0] <= j && sh[0] > lo) {
+            lo = sh[0];
+            clo = cn[0];
+        }
+        if (cn[1] > j && sh[1] < hi) {
+            hi = sh[1];
+            chi = cn[1];
+        }
     }
-    if (!ok) {
-        lo = -1.0;
-        hi = 1.0;
-        clo = sturm64(n, d, e2, lo, pivmin);
-        chi = sturm64(n, d, e2, hi, pivmin);
-        if (!(clo <= j && chi > j)) atomicMax(&a.status[b], 1);
-    }
-    double* Gc = a.G + col;
-    double* Sc = a.L + col;
-    double lam = x, vs = x;  // the eigenvalue, and the shift whose twist r gives the vector
+    if (lo == -1.0 || hi == 1.0) atomicMax(&a.status[b], 1);
+    double lam = x, nz = 1.0;
     int r = n - 1;
     bool done = false;
-    // a bracket holding several eigenvalues is bisected until it holds this one alone
-    for (int it = 0; it < 60 && chi - clo > 1 && hi - lo > 4.0 * DBL_EPSILON; it++) {
-        const double mid = 0.5 * (lo + hi);
-        const int cm = sturm64(n, d, e2, mid, pivmin);
-        if (cm > j) {
-            hi = mid;
-            chi = cm;
-        } else {
-            lo = mid;
-            clo = cm;
-        }
+    // a bracket holding several eigenvalues is narrowed until it holds this one alone: in double-FP32
+    // down to well above its rounding, then in FP64
+    for (int it = 0; it < 40 && chi - clo > 1 && hi - lo > 1e-12; it++)
+        if (!narrow(count_df, j, &lo, &hi, &clo, &chi)) break;
+    if (chi - clo > 1) {
+        lo -= 1e-13;  // a double-FP32 count may be off this close to an eigenvalue
+        hi += 1e-13;
+        const double sh[kShifts] = {lo, hi};
+        int cn[kShifts];
+        count64(sh, cn);
+        clo = cn[0];
+        chi = cn[1];
+        for (int it = 0; it < 40 && chi - clo > 1 && hi - lo > 4.0 * DBL_EPSILON; it++)
+            if (!narrow(count64, j, &lo, &hi, &clo, &chi)) break;
     }
     if (chi - clo == 1) {
         // converged when the correction is below 1e-14 of the block scale (T is scaled to norm
         // < 1), or when it stops shrinking at a level below 1e-10 (the rounding floor of gamma)
         double s = fmin(fmax(x, lo), hi), prev = 1.0;
-        for (int it = 0; it < 8; it++) {
-            const double dl = rq_step(n, d, e, s, pivmin, K, Gc, Sc, &r);
-            const double s1 = s + dl;
-            if (!(s1 > lo && s1 < hi)) break;  // left the bracket: bisect instead
-            if (fabs(dl) <= 1e-14 || (fabs(dl) <= 1e-10 && fabs(dl) > 0.25 * prev)) {
-                lam = s1;
-                vs = s;  // the twist r belongs to s
-                done = true;
-                break;
+        {
+            // most of the way in double-FP32, at one twist row: an FP64 step costs four times as much
+            double s1 = s, dl = rq_first(n, tf, tfb, dgb, egb, inv, s, a, col, &r, &nz), pl = 1.0;
+            for (int it = 0;; it++) {
+                s1 += dl;
+                if (!(s1 > lo && s1 < hi) || it == 4 || !(fabs(dl) < pl)) break;
+                s = s1;
+                if (fabs(dl) <= 1e-13) break;
+                pl = fabs(dl);
+                dl = gamma_df(n, tf, tfb, dgb, egb, inv, s, r) / nz;
             }
-            prev = fabs(dl);
-            s = s1;
+        }
+        // FP64 from there; an iterate that left the bracket starts again from the bracket narrowed to
+        // double-FP32's resolution
+        for (int att = 0; att < 2 && !done; att++) {
+            if (att) {
+                for (int it = 0; it < 40 && hi - lo > 1e-12; it++)
+                    if (!narrow(count_df, j, &lo, &hi, &clo, &chi)) break;
+                lo -= 1e-13;
+                hi += 1e-13;
+                s = 0.5 * (lo + hi);
+                prev = 1.0;
+            }
+            for (int it = 0; it < 8; it++) {
+                const double dl = rq_step(n, t, dgb, egb, inv, s, a, col, &r, &nz);
+                const double s1 = s + dl;
+                if (!(s1 > lo && s1 < hi)) break;  // left the bracket
+                if (fabs(dl) <= 1e-14 || (fabs(dl) <= 1e-10 && fabs(dl) > 0.25 * prev)) {
+                    lam = s1;
+                    done = true;  // the stored solutions belong to s
+                    break;
+                }
+                prev = fabs(dl);
+                s = s1;
+            }
         }
     }
     if (!done) {
-        for (int it = 0; it < 96; it++) {
-            const double mid = 0.5 * (lo + hi);
-            if (!(hi - lo > 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + 4.0 * pivmin) || mid <= lo || mid >= hi)
-                break;
-            if (sturm64(n, d, e2, mid, pivmin) > j) hi = mid;
-            else lo = mid;
-        }
-        lam = vs = 0.5 * (lo + hi);
-        rq_step(n, d, e, vs, pivmin, K, Gc, Sc, &r);
+        for (int it = 0; it < 48 && hi - lo > 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + 1e-300; it++)
+            if (!narrow(count64, j, &lo, &hi, &clo, &chi)) break;
+        lam = 0.5 * (lo + hi);
+        rq_step(n, t, dgb, egb, inv, lam, a, col, &r, &nz);
     }
-    double nrm2 = 1.0;
-    twisted_vector(n, d, e, vs, pivmin, r, K, a.L + col, a.U + col, a.Z + col, &nrm2);
     a.w[(size_t)b * n + j] = lam * sc;
-    const double s = 1.0 / sqrt(nrm2);
+    const double s = 1.0 / sqrt(nz);
     if (!isfinite(s) || !(s > 0.0)) atomicMax(&a.status[b], 3);
-    for (int i = 0; i < n; i++) a.Z[i * K + col] *= s;
+    // the vector, normalised, with the signs of T's own off-diagonals (entry r positive)
+    const int ngrp = (n + kGrp64 - 1) / kGrp64;
+    const int* KX = a.KX + col;
+    const int* KY = KX + (size_t)ngrp * K;
+    const double* X = a.X + col;
+    const double* Y = a.Y + col;
+    const double xr = s / X[r * K], yr = s / Y[r * K];
+    const int kxr = KX[(r / kGrp64) * K], kyr = KY[(r / kGrp64) * K];
+    int neg = 0;  // parity of the sign flips between row i and row r
+    for (int i = 0; i < r; i++) neg ^= !(egb[i] < 0.0);
+    constexpr int kU = 4;  // groups loaded at a time
+    for (int g0 = 0; g0 < ngrp; g0 += kU) {
+        double v[kU * kGrp64], fx[kU], fy[kU];
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            const int g = min(g0 + u, ngrp - 1);
+            fx[u] = xr * pow2i(KX[g * K] - kxr);
+            fy[u] = yr * pow2i(KY[g * K] - kyr);
+        }
+#pragma unroll
+        for (int k = 0; k < kU * kGrp64; k++) {
+            const int i = g0 * kGrp64 + k;
+            v[k] = i < n ? (i < r ? X : Y)[i * K] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kU * kGrp64; k++) {
+            const int i = g0 * kGrp64 + k;
+            if (i < n) {
+                const double zi = v[k] * (i < r ? fx[k / kGrp64] : fy[k / kGrp64]);
+                a.Z[i * K + col] = neg ? -zi : zi;
+                if (i + 1 < n) neg ^= !(egb[i] < 0.0);
+            }
+        }
+    }
 }
 
 // Gram-Schmidt, twice, inside clusters of close candidates of block b (one CTA per block).
@@ -426,16 +793,27 @@ bool blockeig_supported(int n) { return n >= 3 && n <= kMaxN; }
 
 void launch_blockeig_spectrum(int n, int nblk, const double* dg, const double* eg, double* w, double* scale,
                               cudaStream_t s, long long* launches) {
-    spectrum_kernel<<<dim3(nblk, (n + 255) / 256), 256, 0, s>>>(n, dg, eg, w, scale);
+    const size_t smem = sizeof(float4) * (size_t)((n + kGrp32 - 1) / kGrp32 * kGrp32);
+    OPSEC_CUDA(cudaFuncSetAttribute(spectrum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    max_dynamic_smem((const void*)spectrum_kernel)));
+    spectrum_kernel<<<dim3(nblk, (n + 255) / 256), 256, smem, s>>>(n, dg, eg, w, scale);
     OPSEC_CUDA(cudaGetLastError());
     ++*launches;
 }
 
 void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long* launches) {
-    VecArgs a{p.n, p.nblk, p.ktot, p.kc, p.koff, p.dg, p.eg, p.scale, p.w, p.Z, p.L, p.U, p.G, p.status};
-    const dim3 grid(p.nblk, (p.n + 31) / 32);
+    VecArgs a{p.n, p.nblk, p.ktot, p.kc, p.koff, p.dg, p.eg, p.scale, p.w, p.Z, p.K, p.X, p.Y, p.status};
+    int dev = 0, nsm = 0;
+    OPSEC_CUDA(cudaGetDevice(&dev));
+    OPSEC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    const int per = std::min(32, std::max(1, (p.ktot + 4 * nsm - 1) / (4 * nsm)));
+    const dim3 grid(p.nblk, (p.kmax + 4 * per - 1) / (4 * per));
     if (g_clock) g_clock->begin("blockeig_pairs", s);
-    vectors_kernel<<<grid, 32, 0, s>>>(a);
+    const size_t rows = sizeof(double) * 10 * (size_t)((p.n + kGrp64 - 1) / kGrp64 * kGrp64);
+    OPSEC_CUDA(cudaFuncSetAttribute(vectors_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    max_dynamic_smem((const void*)vectors_kernel)));
+    vectors_kernel<<<grid, 128, rows, s>>>(a, per);
+    OPSEC_CUDA(cudaGetLastError());
     if (g_clock) g_clock->end(s);
     cluster_kernel<<<p.nblk, 256, 0, s>>>(a, 1e-6);
     if (g_clock) g_clock->begin("blockeig_back", s, 2.0 * p.n * (double)p.n * p.ktot);

@@ -115,11 +115,12 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     OPSEC_CUDA(cudaMemcpyAsync(c->bev_i.p, hi.data(), sizeof(int) * 2 * nblk, cudaMemcpyHostToDevice, c->stream));
     OPSEC_CUDA(cudaMemsetAsync(c->bev_i.p + 2 * nblk, 0, sizeof(int) * nblk, c->stream));
     const size_t per = (size_t)n * ktot;
-    c->bev_vec.alloc(4 * per);
+    c->bev_vec.alloc(3 * per + (size_t)((n + 1) / 2) * ktot);
     BlockEigVectors p{};
     p.n = n;
     p.nblk = nblk;
     p.ktot = ktot;
+    p.kmax = *std::max_element(kc.begin(), kc.end());
     p.kc = c->bev_i.p;
     p.koff = c->bev_i.p + nblk;
     p.status = c->bev_i.p + 2 * nblk;
@@ -128,9 +129,9 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     p.scale = scale;
     p.w = c->W.p;
     p.Z = c->bev_vec.p;
-    p.L = p.Z + per;
-    p.U = p.L + per;
-    p.G = p.U + per;
+    p.X = p.Z + per;
+    p.Y = p.X + per;
+    p.K = reinterpret_cast<int*>(p.Y + per);
     p.V = c->bev_V.p;
     p.tau = tau;
     p.out = c->S.p;

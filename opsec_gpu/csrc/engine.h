@@ -216,13 +216,15 @@ void launch_blockeig_spectrum(int n, int nblk, const double* dg, const double* e
                               cudaStream_t s, long long* launches);
 struct BlockEigVectors {
     int n, nblk, ktot;
+    int kmax;             // largest kc
     const int* kc;        // [nblk] candidates per block
     const int* koff;      // [nblk] prefix sums of kc
     const double* dg;     // [nblk][n] diagonal of T
     const double* eg;     // [nblk][n] off-diagonal of T
     const double* scale;  // [nblk] power-of-two scale
     double* w;            // [nblk][n] eigenvalues, ascending (candidates refined in place)
-    double *Z, *L, *U, *G;  // [n][ktot] each
+    double *Z, *X, *Y;    // [n][ktot] each: the vectors, and scratch
+    int* K;               // scratch, 2 ceil(n/2) ktot
     int* status;          // [nblk], zeroed by the caller
     const double* V;      // [nblk][n][n] reflectors
     const double* tau;    // [nblk][n]
