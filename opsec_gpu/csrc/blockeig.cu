@@ -18,8 +18,10 @@
 //      then its eigenvector of T from the last one.
 //   5. cluster_kernel: Gram-Schmidt (twice) inside clusters of candidates closer than 1e-6 of the
 //      block norm, where separately computed vectors need not be orthogonal.
-//   6. backtransform_kernel: x = Q z by the stored reflectors (double-FP32), written as the
-//      block's eigenvector column (ascending eigenvalue order, the layout of LAPACK's syevd).
+//   6. backtransform_kernel: x = Q z by the stored reflectors, four at a time (double-FP32), written
+//      as the block's eigenvector column (ascending eigenvalue order, the layout of LAPACK's syevd):
+//      34 blocks of 512^2 1.85 -> 1.10 ms, 34 of 1024^2 16.2 -> 10.2, 10 of 555^2 1.40 -> 0.68 against
+//      one reflector at a time by CTAs of 16 vectors.
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -725,69 +727,238 @@ __global__ void __launch_bounds__(256) cluster_kernel(VecArgs a, double tol) {
     }
 }
 
-// x = H_0 H_1 ... H_{n-3} z for G candidates of block b per CTA (grid (nblk, ceil(n/G)), 256
-// threads), in double-FP32.  The G vectors live in shared memory ([row][G] (hi, lo) pairs),
-// each reflector row is staged once per CTA, thread t works on vector t % G over the rows
-// t / G + R k, and the G dot products are summed over the R = 256 / G row groups in a fixed
-// order.  Writes column n-1-c of the block in FP64 (ascending order, column-major).
-constexpr int kBT = 256;
-template <int G>
-__global__ void __launch_bounds__(kBT) backtransform_kernel(VecArgs a, const double* __restrict__ Vall,
-                                                            const double* __restrict__ tau, double* __restrict__ out) {
-    extern __shared__ double bsm[];
-    constexpr int R = kBT / G;  // row groups
-    const int b = blockIdx.x, n = a.n, kc = a.kc[b];
-    const int c0 = blockIdx.y * G;
-    if (c0 >= kc) return;
-    float2* z = reinterpret_cast<float2*>(bsm);  // [n][G]
-    float2* v = z + (size_t)n * G;                // [n] reflector row
-    float2* part = v + n;                         // [R][G]
-    float2* f = part + R * G;                     // [G]
-    float2* tau2 = f + G;                         // [n] tau as (hi, lo) pairs
-    const int t = threadIdx.x, g = t % G, rg = t / G;
-    const size_t K = (size_t)a.ktot;
-    const int ng = min(G, kc - c0);
-    for (int idx = t; idx < n * G; idx += kBT) {
-        const int i = idx / G, gg = idx % G;
-        z[idx] = df_pack(df_from(gg < ng ? a.Z[(size_t)i * K + a.koff[b] + c0 + gg] : 0.0));
+// ---------------------------------------------------------------- back-transformation
+// x = H_0 H_1 ... H_{n-3} z.  Reflectors are applied kR at a time, H_c .. H_{c+kR-1} = I - V T V^T
+// (the compact form of Schreiber and Van Loan, SIAM J. Sci. Stat. Comput. 10 (1989) 53): one pass
+// over the rows forms V^T z, a kR x kR product and one pass subtracts V (T V^T z).
+constexpr int kR = 4;
+constexpr int kT = kR * (kR + 1) / 2;  // T's upper triangle, column by column
+
+__device__ __forceinline__ df shfl_df(df x, int src) {
+    return df{__shfl_sync(0xffffffffu, x.h, src), __shfl_sync(0xffffffffu, x.l, src)};
+}
+__device__ __forceinline__ df shfl_xor_df(df x, int o) {
+    return df{__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)};
+}
+// acc + x y, the low parts only added up (renormalised where the sum is used)
+__device__ __forceinline__ df df_mac(df acc, df x, df y) {
+    const float p = __fmul_rn(x.h, y.h);
+    float e = fmaf(x.h, y.h, -p);
+    e = fmaf(x.h, y.l, e);
+    e = fmaf(x.l, y.h, e);
+    float t;
+    const float s = two_sum(acc.h, p, t);
+    return df{s, acc.l + (t + e)};
+}
+
+// T of every group of kR reflectors: one warp each.  Reflectors past the last (n - 3) become zero
+// rows.  V row c: zero from its group's first row + 1 to c (tridiag.cu), then v.
+__global__ void __launch_bounds__(128) compact_kernel(int n, int nblk, float2* __restrict__ Vall,
+                                                      const double* __restrict__ tau, float2* __restrict__ T) {
+    const int ngrp = (n - 2 + kR - 1) / kR, lane = threadIdx.x & 31;
+    const int w = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (w >= ngrp * nblk) return;
+    const int b = w / ngrp, c0 = (w % ngrp) * kR;
+    float2* V = Vall + (size_t)b * n * n;
+    df tv[kR], g[kR][kR];
+#pragma unroll
+    for (int q = 0; q < kR; q++) {
+        tv[q] = c0 + q <= n - 3 ? df_from(tau[(size_t)b * n + c0 + q]) : df{0.f, 0.f};
+#pragma unroll
+        for (int p = 0; p < kR; p++) g[p][q] = df{0.f, 0.f};
     }
-    const float2* V = reinterpret_cast<const float2*>(Vall) + (size_t)b * n * n;
-    const double* tb = tau + (size_t)b * n;
-    for (int i = t; i < n; i += kBT) tau2[i] = df_pack(df_from(tb[i]));
-    __syncthreads();
-    for (int c2 = n - 3; c2 >= 0; c2--) {
-        const float2 tc2 = tau2[c2];
-        if (tc2.x == 0.f) continue;  // uniform over the CTA
-        __syncthreads();          // the previous update is done with v and f
-        for (int i = c2 + 1 + t; i < n; i += kBT) v[i] = V[(size_t)c2 * n + i];
-        __syncthreads();
-        df s0{0.f, 0.f}, s1{0.f, 0.f};
-        int i = c2 + 1 + rg;
-        for (; i + R < n; i += 2 * R) {
-            s0 = df_fma(s0, df_unpack(v[i]), df_unpack(z[(size_t)i * G + g]));
-            s1 = df_fma(s1, df_unpack(v[i + R]), df_unpack(z[(size_t)(i + R) * G + g]));
+    for (int i = c0 + 1 + lane; i < n; i += 32) {
+        df v[kR];
+#pragma unroll
+        for (int q = 0; q < kR; q++) {
+            if (c0 + q <= n - 3) {
+                v[q] = df_unpack(V[(size_t)(c0 + q) * n + i]);
+            } else {
+                v[q] = df{0.f, 0.f};
+                if (c0 + q < n) V[(size_t)(c0 + q) * n + i] = make_float2(0.f, 0.f);
+            }
         }
-        if (i < n) s0 = df_fma(s0, df_unpack(v[i]), df_unpack(z[(size_t)i * G + g]));
-        part[rg * G + g] = df_pack(df_add(s0, s1));
-        __syncthreads();
-        if (t < G) {
-            df s = df_unpack(part[t]);
-            for (int r = 1; r < R; r++) s = df_add(s, df_unpack(part[r * G + t]));
-            f[t] = df_pack(df_mul(df_unpack(tc2), s));
-        }
-        __syncthreads();
-        const df fg = df_unpack(f[g]);
-        for (i = c2 + 1 + rg; i < n; i += R)
-            z[(size_t)i * G + g] = df_pack(df_fms(df_unpack(z[(size_t)i * G + g]), fg, df_unpack(v[i])));
+#pragma unroll
+        for (int q = 1; q < kR; q++)
+#pragma unroll
+            for (int p = 0; p < q; p++) g[p][q] = df_mac(g[p][q], v[p], v[q]);
     }
-    __syncthreads();
-    for (int gg = 0; gg < ng; gg++) {
-        double* o = out + (size_t)b * n * n + (size_t)(n - 1 - (c0 + gg)) * n;
-        for (int i2 = t; i2 < n; i2 += kBT) o[i2] = df_to(df_unpack(z[(size_t)i2 * G + gg]));
+#pragma unroll
+    for (int q = 1; q < kR; q++)
+#pragma unroll
+        for (int p = 0; p < q; p++)
+#pragma unroll
+            for (int o = 16; o; o >>= 1) g[p][q] = df_add(g[p][q], shfl_xor_df(g[p][q], o));
+    // T_qq = tau_q, T_pq = -tau_q sum_{p <= k < q} T_pk g_kq
+    df t[kR][kR];
+#pragma unroll
+    for (int q = 0; q < kR; q++) {
+        t[q][q] = tv[q];
+#pragma unroll
+        for (int p = 0; p < q; p++) {
+            df s{0.f, 0.f};
+#pragma unroll
+            for (int k = p; k < q; k++) s = df_fma(s, t[p][k], g[k][q]);
+            t[p][q] = df_mul(df{-tv[q].h, -tv[q].l}, s);
+        }
+    }
+    if (lane == 0) {
+        float2* o = T + (size_t)w * kT;
+#pragma unroll
+        for (int q = 0; q < kR; q++)
+#pragma unroll
+            for (int p = 0; p <= q; p++) o[q * (q + 1) / 2 + p] = df_pack(t[p][q]);
     }
 }
 
+// NV candidates of block b per warp, their rows in the warp's shared memory; warps work alone (no
+// barriers).  The reflectors come from L2 twice per group, as one stream of asynchronous copies
+// kPipe steps ahead (each lane copies what it will read), which runs on over the ends of passes and
+// groups: with plain loads every step of 32 rows waited for L2.  More vectors a warp read the
+// reflectors less often, fewer keep more warps in flight (launch_blockeig_vectors); the CTAs of a
+// block are neighbours, so that its reflectors stay in L2.  Writes candidate c in FP64: as column
+// n-1-c of the block (ascending order, column-major), or, with rows set, as row c of out while c <
+// rows.
+constexpr int kPipe = 8;
+constexpr int kRing = kPipe * kR * 32;  // pairs per warp
+template <int NV>
+__global__ void __launch_bounds__(128) backtransform_kernel(VecArgs a, const float2* __restrict__ Vall,
+                                                            const float2* __restrict__ Tall, double* __restrict__ out,
+                                                            int rows) {
+    extern __shared__ float2 zsm[];
+    const int b = blockIdx.y, n = a.n, kc = a.kc[b];
+    const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c0 = (blockIdx.x * W + warp) * NV;
+    if (c0 >= kc) return;
+    float2* ring = zsm + (size_t)warp * (kRing + NV * n) + lane;  // [kPipe][kR][32], this lane's slots
+    float2* z = zsm + (size_t)warp * (kRing + NV * n) + kRing;    // [NV][n]
+    const size_t K = (size_t)a.ktot;
+    const int nv = min(NV, kc - c0);
+    for (int i = lane; i < n; i += 32) {
+        const double* src = a.Z + (size_t)i * K + a.koff[b] + c0;
+#pragma unroll
+        for (int v = 0; v < NV; v++) z[v * n + i] = df_pack(df_from(v < nv ? src[v] : 0.0));
+    }
+    __syncwarp();
+    const float2* V = Vall + (size_t)b * n * n;
+    const int ngrp = (n - 2 + kR - 1) / kR;
+    constexpr int NS = NV * kR;  // sums a group: (vector, reflector)
+    // the stream: groups downwards, each twice, rows r0 + 1 + lane, + 32, ...
+    int sg = ngrp - 1, sp = 0, si = 0, slot = 0;  // next step to issue: group, pass, row offset
+    auto issue = [&]() {
+        if (sg >= 0) {
+            const int i = sg * kR + 1 + si + lane;
+            if (i < n) {
+                const float2* src = V + (size_t)(sg * kR) * n + i;
+#pragma unroll
+                for (int q = 0; q < kR; q++) {
+                    const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + (slot * kR + q) * 32);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src + (size_t)q * n) : "memory");
+                }
+            }
+            si += 32;
+            if (sg * kR + 1 + si >= n) {
+                si = 0;
+                sg -= sp;
+                sp ^= 1;
+            }
+        }
+        slot = slot + 1 == kPipe ? 0 : slot + 1;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int k = 0; k < kPipe - 1; k++) issue();
+    int rd = 0;
+    auto step = [&](df (&v)[kR]) {  // the next step's reflector entries
+        asm volatile("cp.async.wait_group %0;" ::"n"(kPipe - 2) : "memory");
+#pragma unroll
+        for (int q = 0; q < kR; q++) v[q] = df_unpack(ring[(rd * kR + q) * 32]);
+        rd = rd + 1 == kPipe ? 0 : rd + 1;
+        issue();
+    };
+    for (int g = ngrp - 1; g >= 0; g--) {
+        const int r0 = g * kR;
+        df acc[NS];
+#pragma unroll
+        for (int k = 0; k < NS; k++) acc[k] = df{0.f, 0.f};
+        for (int i0 = r0 + 1; i0 < n; i0 += 32) {
+            const int i = i0 + lane;
+            df v[kR];
+            step(v);
+            if (i < n) {
+#pragma unroll
+                for (int u = 0; u < NV; u++) {
+                    const df x = df_unpack(z[u * n + i]);
+#pragma unroll
+                    for (int q = 0; q < kR; q++) acc[u * kR + q] = df_mac(acc[u * kR + q], v[q], x);
+                }
+            }
+        }
+        // sum over the lanes, halving the sums held: lane l ends with sum l / (32 / NS)
+        int o = 16;
+#pragma unroll
+        for (int h = NS / 2; h >= 1; h /= 2, o /= 2) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int k = 0; k < h; k++) {
+                const df keep = up ? acc[k + h] : acc[k], give = up ? acc[k] : acc[k + h];
+                acc[k] = df_add(keep, shfl_xor_df(give, o));
+            }
+        }
+#pragma unroll
+        for (int e = 16 / NS; e; e >>= 1) acc[0] = df_add(acc[0], shfl_xor_df(acc[0], e));
+        // f = T d: this lane's row p of its vector u
+        constexpr int kL = 32 / NS;  // lanes per sum
+        const int mine = lane / kL, u0 = mine / kR, p0 = mine % kR;
+        const float2* Tg = Tall + ((size_t)b * ngrp + g) * kT;
+        df f{0.f, 0.f};
+#pragma unroll
+        for (int q = 0; q < kR; q++) {
+            const df d = shfl_df(acc[0], (u0 * kR + q) * kL);
+            if (q >= p0) f = df_fma(f, df_unpack(__ldg(Tg + q * (q + 1) / 2 + p0)), d);
+        }
+        df fs[NS];
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+            const df t = shfl_df(f, k * kL);
+            fs[k] = df{-t.h, -t.l};
+        }
+        for (int i0 = r0 + 1; i0 < n; i0 += 32) {
+            const int i = i0 + lane;
+            df v[kR];
+            step(v);
+            if (i < n) {
+#pragma unroll
+                for (int u = 0; u < NV; u++) {
+                    df x = df_unpack(z[u * n + i]);
+#pragma unroll
+                    for (int q = 0; q < kR; q++) x = df_mac(x, v[q], fs[u * kR + q]);
+                    z[u * n + i] = df_pack(fast_two_sum(x.h, x.l));
+                }
+            }
+        }
+        __syncwarp();  // a lane's rows shift by kR from group to group
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    for (int u = 0; u < nv; u++) {
+        if (rows > 0 && c0 + u >= rows) break;
+        double* o = rows > 0 ? out + (size_t)(c0 + u) * n : out + (size_t)b * n * n + (size_t)(n - 1 - (c0 + u)) * n;
+        for (int i = lane; i < n; i += 32) o[i] = df_to(df_unpack(z[u * n + i]));
+    }
+}
+
+template <int NV>
+void launch_back(const VecArgs& a, const BlockEigVectors& p, int warps, cudaStream_t s) {
+    auto k = backtransform_kernel<NV>;
+    const size_t per = sizeof(float2) * (kRing + (size_t)NV * p.n);
+    OPSEC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem((const void*)k)));
+    k<<<dim3((p.kmax + warps * NV - 1) / (warps * NV), p.nblk), 32 * warps, per * warps, s>>>(
+        a, reinterpret_cast<const float2*>(p.V), reinterpret_cast<const float2*>(p.T), p.out, p.rows);
+    OPSEC_CUDA(cudaGetLastError());
+}
+
 }  // namespace
+
+size_t blockeig_compact_doubles(int n, int nblk) { return (size_t)((n - 2 + kR - 1) / kR) * nblk * kT; }
 
 bool blockeig_supported(int n) { return n >= 3 && n <= kMaxN; }
 
@@ -816,23 +987,30 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     OPSEC_CUDA(cudaGetLastError());
     if (g_clock) g_clock->end(s);
     cluster_kernel<<<p.nblk, 256, 0, s>>>(a, 1e-6);
-    if (g_clock) g_clock->begin("blockeig_back", s, 2.0 * p.n * (double)p.n * p.ktot);
-    if (p.n <= 256) {  // 16 vectors per CTA above: twice the CTAs, two per SM
-        constexpr int G = 32;
-        const size_t smem = sizeof(double) * ((size_t)p.n * G + 2 * p.n + kBT + G);
-        OPSEC_CUDA(cudaFuncSetAttribute(backtransform_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        max_dynamic_smem((const void*)backtransform_kernel<G>)));
-        backtransform_kernel<G><<<dim3(p.nblk, (p.n + G - 1) / G), kBT, smem, s>>>(a, p.V, p.tau, p.out);
-    } else {
-        constexpr int G = 16;
-        const size_t smem = sizeof(double) * ((size_t)p.n * G + 2 * p.n + kBT + G);
-        OPSEC_CUDA(cudaFuncSetAttribute(backtransform_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        max_dynamic_smem((const void*)backtransform_kernel<G>)));
-        backtransform_kernel<G><<<dim3(p.nblk, (p.n + G - 1) / G), kBT, smem, s>>>(a, p.V, p.tau, p.out);
-    }
-    if (g_clock) g_clock->end(s);
     OPSEC_CUDA(cudaGetLastError());
-    *launches += 3;
+    if (g_clock) g_clock->begin("blockeig_back", s, 2.0 * p.n * (double)p.n * p.ktot);
+    const int groups = (p.n - 2 + kR - 1) / kR * p.nblk;
+    compact_kernel<<<(groups + 3) / 4, 128, 0, s>>>(p.n, p.nblk, reinterpret_cast<float2*>(p.V), p.tau,
+                                                    reinterpret_cast<float2*>(p.T));
+    OPSEC_CUDA(cudaGetLastError());
+    // Vectors per warp.  One while the warps do not fill the chip four times over (10 blocks of 555^2,
+    // 1,390 vectors: 0.68 ms, two 0.84, four 1.07); two beyond (34 of 1024^2: 10.2 ms, four 13.4: a
+    // warp's 40 KB leave five warps an SM); four where their rows still leave nine warps an SM and
+    // reading the reflectors half as often counts (34 of 512^2, 4,351 vectors: 1.10 ms, two 1.43, one
+    // 1.42; 66 of 256^2: two 0.35, four 0.41).
+    const int cap = max_dynamic_smem((const void*)backtransform_kernel<4>);
+    const size_t vec = sizeof(float2) * (size_t)p.n;
+    auto warps_of = [&](int nv) { return (int)std::min<size_t>(4, (size_t)cap / (vec * nv + sizeof(float2) * kRing)); };
+    int nv = p.ktot < 16 * nsm ? 1 : p.ktot >= 24 * nsm && p.n > 384 && p.n <= 576 ? 4 : 2;
+    while (nv > 1 && warps_of(nv) < 1) nv /= 2;
+    if (nv == 4)
+        launch_back<4>(a, p, warps_of(4), s);
+    else if (nv == 2)
+        launch_back<2>(a, p, warps_of(2), s);
+    else
+        launch_back<1>(a, p, warps_of(1), s);
+    if (g_clock) g_clock->end(s);
+    *launches += 4;
 }
 
 }  // namespace opsec

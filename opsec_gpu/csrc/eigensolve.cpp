@@ -52,7 +52,11 @@ void drop_eig_graph(opsec_gpu* c) {
     c->eig_key = {};
 }
 
-// The hand-written block eigensolver (blockeig.cu) on the nblk blocks of order n in c->S:
+// Surveys whose Fisher matrix moves by over 1e-9 with the eigensolver's rounding (blockeig_small.cu):
+// few cells, or blocks that keep the modes even and odd in mu together (npar = 1) and not many cells.
+bool small_survey(int npar, long long cells) { return cells < 1024 || (npar == 1 && cells < 8192); }
+
+// The hand-written block eigensolver (blockeig.cu, blockeig_small.cu) on the nblk blocks of order n in c->S:
 // every eigenvalue (ascending per block) into c->W, and the eigenvectors of the block
 // eigenvalues that can reach the global top-M cut as columns of c->S.  kc[b] = the number of
 // top eigenpairs of block b computed.  Returns false (and leaves a warning) when a check in the
@@ -65,14 +69,21 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     double* dg = tau + (size_t)nblk * n;
     double* eg = dg + (size_t)nblk * n;
     double* scale = eg + (size_t)nblk * n;
-    if (g_clock) g_clock->begin("blockeig_tridiag", c->stream, 4.0 / 3.0 * n * nn * nblk);
-    c->bev_D.alloc(tridiag_work_bytes(n, nblk));
+    const bool small = small_survey(npar, (long long)n * npar * Nphi);
     c->bev_err.alloc(1);
     OPSEC_CUDA(cudaMemsetAsync(c->bev_err.p, 0, sizeof(int), c->stream));
-    launch_tridiag(n, nblk, c->S.p, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
-                   &c->launches);
+    if (!small) c->bev_D.alloc(tridiag_work_bytes(n, nblk));
+    if (g_clock) g_clock->begin("blockeig_tridiag", c->stream, 4.0 / 3.0 * n * nn * nblk);
+    if (small)
+        launch_small_tridiag(n, nblk, c->S.p, c->bev_V.p, tau, dg, eg, c->stream, &c->launches);
+    else
+        launch_tridiag(n, nblk, c->S.p, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
+                       &c->launches);
     if (g_clock) g_clock->end(c->stream);
-    launch_blockeig_spectrum(n, nblk, dg, eg, c->W.p, scale, c->stream, &c->launches);
+    if (small)
+        launch_small_spectrum(n, nblk, dg, eg, c->W.p, scale, c->stream, &c->launches);
+    else
+        launch_blockeig_spectrum(n, nblk, dg, eg, c->W.p, scale, c->stream, &c->launches);
     std::vector<double> w((size_t)nblk * n), sc(nblk);
     OPSEC_CUDA(cudaMemcpyAsync(w.data(), c->W.p, sizeof(double) * w.size(), cudaMemcpyDeviceToHost, c->stream));
     OPSEC_CUDA(cudaMemcpyAsync(sc.data(), scale, sizeof(double) * nblk, cudaMemcpyDeviceToHost, c->stream));
@@ -115,31 +126,44 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     OPSEC_CUDA(cudaMemcpyAsync(c->bev_i.p, hi.data(), sizeof(int) * 2 * nblk, cudaMemcpyHostToDevice, c->stream));
     OPSEC_CUDA(cudaMemsetAsync(c->bev_i.p + 2 * nblk, 0, sizeof(int) * nblk, c->stream));
     const size_t per = (size_t)n * ktot;
-    c->bev_vec.alloc(3 * per + (size_t)((n + 1) / 2) * ktot);
-    BlockEigVectors p{};
-    p.n = n;
-    p.nblk = nblk;
-    p.ktot = ktot;
-    p.kmax = *std::max_element(kc.begin(), kc.end());
-    p.kc = c->bev_i.p;
-    p.koff = c->bev_i.p + nblk;
-    p.status = c->bev_i.p + 2 * nblk;
-    p.dg = dg;
-    p.eg = eg;
-    p.scale = scale;
-    p.w = c->W.p;
-    p.Z = c->bev_vec.p;
-    p.X = p.Z + per;
-    p.Y = p.X + per;
-    p.K = reinterpret_cast<int*>(p.Y + per);
-    p.V = c->bev_V.p;
-    p.tau = tau;
-    p.out = c->S.p;
-    if (g_clock) g_clock->begin("blockeig_vectors", c->stream, 2.0 * nn * ktot);
-    launch_blockeig_vectors(p, c->stream, &c->launches);
-    if (g_clock) g_clock->end(c->stream);
+    int* status = c->bev_i.p + 2 * nblk;
+    if (small) {
+        c->bev_vec.alloc(4 * per);
+        double* Z = c->bev_vec.p;
+        const SmallEigVectors p{n, nblk, ktot, c->bev_i.p, c->bev_i.p + nblk, dg, eg, scale, c->W.p, Z, Z + per,
+                                Z + 2 * per, Z + 3 * per, status, c->bev_V.p, tau, c->S.p};
+        if (g_clock) g_clock->begin("blockeig_vectors", c->stream, 2.0 * nn * ktot);
+        launch_small_vectors(p, c->stream, &c->launches);
+        if (g_clock) g_clock->end(c->stream);
+    } else {
+        c->bev_vec.alloc(3 * per + (size_t)((n + 1) / 2) * ktot);
+        c->bev_C.alloc(blockeig_compact_doubles(n, nblk));
+        BlockEigVectors p{};
+        p.n = n;
+        p.nblk = nblk;
+        p.ktot = ktot;
+        p.kmax = *std::max_element(kc.begin(), kc.end());
+        p.kc = c->bev_i.p;
+        p.koff = c->bev_i.p + nblk;
+        p.status = status;
+        p.dg = dg;
+        p.eg = eg;
+        p.scale = scale;
+        p.w = c->W.p;
+        p.Z = c->bev_vec.p;
+        p.X = p.Z + per;
+        p.Y = p.X + per;
+        p.K = reinterpret_cast<int*>(p.Y + per);
+        p.V = c->bev_V.p;
+        p.tau = tau;
+        p.T = c->bev_C.p;
+        p.out = c->S.p;
+        if (g_clock) g_clock->begin("blockeig_vectors", c->stream, 2.0 * nn * ktot);
+        launch_blockeig_vectors(p, c->stream, &c->launches);
+        if (g_clock) g_clock->end(c->stream);
+    }
     std::vector<int> st(nblk);
-    OPSEC_CUDA(cudaMemcpyAsync(st.data(), p.status, sizeof(int) * nblk, cudaMemcpyDeviceToHost, c->stream));
+    OPSEC_CUDA(cudaMemcpyAsync(st.data(), status, sizeof(int) * nblk, cudaMemcpyDeviceToHost, c->stream));
     sync(c);
     for (int b = 0; b < nblk; b++)
         if (st[b]) {

@@ -226,11 +226,35 @@ struct BlockEigVectors {
     double *Z, *X, *Y;    // [n][ktot] each: the vectors, and scratch
     int* K;               // scratch, 2 ceil(n/2) ktot
     int* status;          // [nblk], zeroed by the caller
+    double* V;            // [nblk][n][n] reflectors, (hi, lo) float pairs
+    const double* tau;    // [nblk][n]
+    double* T;            // scratch, blockeig_compact_doubles()
+    double* out;          // [nblk][n][n] eigenvector columns, or with rows > 0 (one block) [rows][n], largest first
+    int rows;
+};
+size_t blockeig_compact_doubles(int n, int nblk);
+void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long* launches);
+
+// The same for small surveys (blockeig_small.cu): A is overwritten.
+void launch_small_tridiag(int n, int nblk, double* A, double* V, double* tau, double* dg, double* eg, cudaStream_t s,
+                          long long* launches);
+void launch_small_spectrum(int n, int nblk, const double* dg, const double* eg, double* w, double* scale,
+                           cudaStream_t s, long long* launches);
+struct SmallEigVectors {
+    int n, nblk, ktot;
+    const int* kc;        // [nblk] candidates per block
+    const int* koff;      // [nblk] prefix sums of kc
+    const double* dg;     // [nblk][n] diagonal of T
+    const double* eg;     // [nblk][n] off-diagonal of T
+    const double* scale;  // [nblk] power-of-two scale
+    double* w;            // [nblk][n] eigenvalues, ascending (candidates refined in place)
+    double *Z, *L, *U, *G;  // [n][ktot] each
+    int* status;          // [nblk], zeroed by the caller
     const double* V;      // [nblk][n][n] reflectors
     const double* tau;    // [nblk][n]
     double* out;          // [nblk][n][n] eigenvector columns
 };
-void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long* launches);
+void launch_small_vectors(const SmallEigVectors& p, cudaStream_t s, long long* launches);
 
 // Projection C_p = B'^T Q_p B' for all bands; B' = diag(sqrt Nbar) B.
 struct ProjectArgs {

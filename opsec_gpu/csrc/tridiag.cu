@@ -119,7 +119,7 @@ struct TridiagArgs {
     int kres;          // a warp's rows k >= kres live in shared memory
     int nres;          // resident rows per CTA
     float* D;          // [block][n][2 ld] the matrix in double-FP32, both triangles, zero past column n
-    float2* V;         // [block][n][n] reflector c in row c (v[c+1] = 1)
+    float2* V;         // [block][n][n] reflector c in row c (v[c+1] = 1), zeros from entry (c & ~3) + 1 on before it
     double *tau, *dg, *eg;  // [block][n]
     // whole-chip form: exchange of p, and the barrier between CTAs
     float2* pbuf;      // [2][n]
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
         reflect(c1, s, vnxt);
         __syncthreads();
         if (rank == c1 % C)
-            for (int i = c1 + 1 + t; i < n; i += T) V[(size_t)c1 * n + i] = df_pack(get(vnxt, i));
+            for (int i = (c1 & ~3) + 1 + t; i < n; i += T) V[(size_t)c1 * n + i] = df_pack(get(vnxt, i));
         if (c < n - 3)
             pass(c + 2, par ^ 1, yes{}, yes{});
         else

@@ -8,9 +8,11 @@ from opsec_gpu import api, synth
 pytestmark = pytest.mark.gpu
 
 
-# (nr, nmu, nphi): odd nmu keeps one block of nr nmu per azimuthal order, even nmu two of half that
-@pytest.mark.parametrize("dims", [(1, 3, 6), (4, 1, 5), (9, 7, 8), (8, 16, 6), (13, 5, 9), (19, 5, 6), (32, 3, 4),
-                                  (97, 1, 4), (43, 3, 5), (7, 37, 6), (4, 6, 128), (27, 38, 4), (31, 33, 4)])
+# (nr, nmu, nphi): odd nmu keeps one block of nr nmu per azimuthal order, even nmu two of half that.
+# The first four are small surveys, which keep their own kernels.
+@pytest.mark.parametrize("dims", [(1, 3, 6), (4, 1, 5), (13, 5, 9), (40, 5, 40), (1, 6, 172), (2, 4, 130), (1, 10, 103),
+                                  (4, 6, 128), (9, 14, 9), (8, 16, 8), (13, 10, 8), (19, 10, 6), (32, 6, 6), (97, 2, 6),
+                                  (43, 6, 5), (37, 14, 4), (27, 38, 4), (31, 66, 4), (91, 11, 9)])
 def test_eigenpairs_of_every_block_shape(dims):
     sv, cells = synth.shell_survey(*dims)
     k, P = synth.pk_table()
