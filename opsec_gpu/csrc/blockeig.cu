@@ -516,6 +516,40 @@ __device__ double gamma_df(int n, const RowsDf& t, const RowsDfB& tb, const doub
     return gamma_of(n, d, e, inv, s, r, r == n - 1 ? ratio : tx, r == n - 1 ? 0.0 : ratio);
 }
 
+// The rows of the recurrences of every block, five FP64 arrays and their double-FP32 pairs, each of
+// np = n rounded up to kGrp64 entries: Rows64's ff, fi, fb, bf, bb, then RowsDf's and RowsDfB's f, g,
+// b, f, b.
+__global__ void rows_kernel(int n, int nblk, const double* __restrict__ dg, const double* __restrict__ eg,
+                            const double* __restrict__ scale, double* __restrict__ R) {
+    const int np = round_up(n, kGrp64);
+    constexpr double kMinE = 8.673617379884035e-19;  // 2^-60
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < np * nblk; t += gridDim.x * blockDim.x) {
+        const int b = t / np, i = t % np;
+        const double inv = 1.0 / scale[b];
+        const double* dgb = dg + (size_t)b * n;
+        const double* egb = eg + (size_t)b * n;
+        double* r = R + (size_t)b * 10 * np;
+        double v[5] = {1.0, 0.0, 0.0, 0.0, 0.0};  // rows past the end keep x
+        if (i < n) {
+            const double d = dgb[i] * inv;
+            const double e = i + 1 < n ? fmax(fabs(egb[i] * inv), kMinE) : 1.0;
+            const double ep = i > 0 ? fmax(fabs(egb[i - 1] * inv), kMinE) : 1.0;
+            v[1] = 1.0 / e;
+            v[0] = d * v[1];
+            v[2] = i > 0 ? -ep * v[1] : 0.0;
+            v[3] = d / ep;
+            v[4] = i + 1 < n ? -e / ep : 0.0;
+        }
+        float2* f = reinterpret_cast<float2*>(r + 5 * np);
+        for (int q = 0; q < 5; q++) r[q * np + i] = v[q];
+        f[i] = df_pack(df_from(v[0]));
+        f[np + i] = df_pack(df_from(v[1]));
+        f[2 * np + i] = df_pack(df_from(v[2]));
+        f[3 * np + i] = df_pack(df_from(v[3]));
+        f[4 * np + i] = df_pack(df_from(v[4]));
+    }
+}
+
 // grid (nblk, parts of kc), 4 warps of `per` candidates each, one per thread: candidate c (0 =
 // largest) of block b.  An FP64 instruction takes a warp 64 cycles of its scheduler's pipe however
 // many of its lanes work, so the candidates are dealt over all schedulers of the chip.
@@ -526,7 +560,9 @@ __device__ double gamma_df(int n, const RowsDf& t, const RowsDfB& tb, const doub
 // Bound by the FP64 pipe (64 cycles an instruction, measured, with nothing to overlap) and by loads of the stored solutions (32 rows at a time: row by row their latency was half the kernel).
 // Candidates of 34 blocks of 512^2 (4,351): 4.51 -> 1.15 ms against FP64 pivots with a division in
 // every row; 34 of 1024^2 25.5 -> 3.77, 10 of 555^2 12.5 -> 2.01, 18 of 64^2 0.406 -> 0.092.
-__global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, int per) {
+// LOCAL: the block's rows in shared memory; otherwise (orders whose rows do not fit) read through L1.
+template <bool LOCAL>
+__global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* __restrict__ R, int per) {
     extern __shared__ double rows64[];
     const int b = blockIdx.x, n = a.n, np = round_up(n, kGrp64);
     const int kc = a.kc[b];
@@ -534,35 +570,16 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, int per) {
     const double sc = a.scale[b], inv = 1.0 / sc;
     const double* dgb = a.dg + (size_t)b * n;
     const double* egb = a.eg + (size_t)b * n;
-    const Rows64 t{rows64, rows64 + np, rows64 + 2 * np, rows64 + 3 * np, rows64 + 4 * np};
-    float2* rowsf = reinterpret_cast<float2*>(rows64 + 5 * np);
+    const double* rows = R + (size_t)b * 10 * np;
+    if (LOCAL) {
+        for (int i = threadIdx.x; i < 10 * np; i += 128) rows64[i] = rows[i];
+        rows = rows64;
+        __syncthreads();
+    }
+    const Rows64 t{rows, rows + np, rows + 2 * np, rows + 3 * np, rows + 4 * np};
+    const float2* rowsf = reinterpret_cast<const float2*>(rows + 5 * np);
     const RowsDf tf{rowsf, rowsf + np, rowsf + 2 * np};
     const RowsDfB tfb{rowsf + 3 * np, rowsf + 4 * np};
-    constexpr double kMinE = 8.673617379884035e-19;  // 2^-60
-    for (int i = threadIdx.x; i < np; i += 128) {
-        double ff = 1.0, fi = 0.0, fb = 0.0, bf = 0.0, bb = 0.0;  // rows past the end keep x
-        if (i < n) {
-            const double d = dgb[i] * inv;
-            const double e = i + 1 < n ? fmax(fabs(egb[i] * inv), kMinE) : 1.0;
-            const double ep = i > 0 ? fmax(fabs(egb[i - 1] * inv), kMinE) : 1.0;
-            fi = 1.0 / e;
-            ff = d * fi;
-            fb = i > 0 ? -ep * fi : 0.0;
-            bf = d / ep;
-            bb = i + 1 < n ? -e / ep : 0.0;
-        }
-        rows64[i] = ff;
-        rows64[np + i] = fi;
-        rows64[2 * np + i] = fb;
-        rows64[3 * np + i] = bf;
-        rows64[4 * np + i] = bb;
-        rowsf[i] = df_pack(df_from(ff));
-        rowsf[np + i] = df_pack(df_from(fi));
-        rowsf[2 * np + i] = df_pack(df_from(fb));
-        rowsf[3 * np + i] = df_pack(df_from(bf));
-        rowsf[4 * np + i] = df_pack(df_from(bb));
-    }
-    __syncthreads();
     const int lane = threadIdx.x & 31, c = (blockIdx.y * 4 + (threadIdx.x >> 5)) * per + lane;
     if (lane >= per || c >= kc) return;
     const int j = n - 1 - c;  // ascending index
@@ -692,22 +709,19 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, int per) {
     }
 }
 
-// Gram-Schmidt, twice, inside clusters of close candidates of block b (one CTA per block).
+// Gram-Schmidt, twice, inside clusters of close candidates: grid (nblk, kmax), the CTA of a
+// cluster's first candidate takes the cluster.
 __global__ void __launch_bounds__(256) cluster_kernel(VecArgs a, double tol) {
     __shared__ double red[40];
-    const int b = blockIdx.x, n = a.n, kc = a.kc[b];
+    const int b = blockIdx.x, n = a.n, kc = a.kc[b], start = blockIdx.y;
     const size_t K = (size_t)a.ktot;
     const double* wb = a.w + (size_t)b * n;
     const double sc = a.scale[b];
     const int c0 = a.koff[b];
-    int start = 0;
-    for (int c = 1; c < kc; c++) {
-        // wb is ascending: candidate c has index n-1-c
-        const bool close = wb[n - c] - wb[n - 1 - c] < tol * sc;
-        if (!close) {
-            start = c;
-            continue;
-        }
+    // wb is ascending: candidate c has index n-1-c
+    auto close = [&](int c) { return wb[n - c] - wb[n - 1 - c] < tol * sc; };  // candidates c-1 and c
+    if (start + 1 >= kc || !close(start + 1) || (start > 0 && close(start))) return;
+    for (int c = start + 1; c < kc && close(c); c++) {
         for (int pass = 0; pass < 2; pass++) {
             for (int k = start; k < c; k++) {
                 double s = 0.0;
@@ -946,6 +960,28 @@ __global__ void __launch_bounds__(128) backtransform_kernel(VecArgs a, const flo
     }
 }
 
+// ---------------------------------------------------------------- polish of a dense solve
+// E of X <- X (I + E) and the Rayleigh quotients, from G = X^T X and H = X^T S X (Ogita and Aishima,
+// Japan J. Indust. Appl. Math. 35 (2018) 1007): with R = I - G, E_ij = (H_ij + l_j R_ij) / (l_j - l_i),
+// E_jj = R_jj / 2; eigenvalues too close to tell apart only have their vectors orthogonalised.
+__global__ void polish_kernel(int k, int m, const double* __restrict__ G, const double* __restrict__ H, double tol,
+                              double* __restrict__ E, double* __restrict__ lam) {
+    const long long n = (long long)k * m;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        const int i = (int)(t % k), j = (int)(t / k);
+        const double li = H[(size_t)i * k + i] / G[(size_t)i * k + i], lj = H[(size_t)j * k + j] / G[(size_t)j * k + j];
+        const size_t o = i >= j ? (size_t)j * k + i : (size_t)i * k + j;  // lower triangles
+        const double r = (i == j ? 1.0 : 0.0) - G[o];
+        double e = 0.5 * r;
+        if (i != j && fabs(lj - li) > tol) {
+            const double v = (H[o] + lj * r) / (lj - li);
+            if (fabs(v) < 1e-5) e = v;
+        }
+        E[t] = e;
+        if (i == j) lam[j] = lj;
+    }
+}
+
 template <int NV>
 void launch_back(const VecArgs& a, const BlockEigVectors& p, int warps, cudaStream_t s) {
     auto k = backtransform_kernel<NV>;
@@ -957,6 +993,16 @@ void launch_back(const VecArgs& a, const BlockEigVectors& p, int warps, cudaStre
 }
 
 }  // namespace
+
+void launch_polish_coefficients(int k, int m, const double* G, const double* H, double tol, double* E, double* lam,
+                                cudaStream_t s, long long* launches) {
+    const long long n = (long long)k * m;
+    polish_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 65536), 256, 0, s>>>(k, m, G, H, tol, E, lam);
+    OPSEC_CUDA(cudaGetLastError());
+    ++*launches;
+}
+
+size_t blockeig_rows_doubles(int n, int nblk) { return (size_t)10 * ((n + kGrp64 - 1) / kGrp64 * kGrp64) * nblk; }
 
 size_t blockeig_compact_doubles(int n, int nblk) { return (size_t)((n - 2 + kR - 1) / kR) * nblk * kT; }
 
@@ -980,13 +1026,20 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     const int per = std::min(32, std::max(1, (p.ktot + 4 * nsm - 1) / (4 * nsm)));
     const dim3 grid(p.nblk, (p.kmax + 4 * per - 1) / (4 * per));
     if (g_clock) g_clock->begin("blockeig_pairs", s);
-    const size_t rows = sizeof(double) * 10 * (size_t)((p.n + kGrp64 - 1) / kGrp64 * kGrp64);
-    OPSEC_CUDA(cudaFuncSetAttribute(vectors_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    max_dynamic_smem((const void*)vectors_kernel)));
-    vectors_kernel<<<grid, 128, rows, s>>>(a, per);
+    const int np = (p.n + kGrp64 - 1) / kGrp64 * kGrp64;
+    rows_kernel<<<(np * p.nblk + 127) / 128, 128, 0, s>>>(p.n, p.nblk, p.dg, p.eg, p.scale, p.R);
+    OPSEC_CUDA(cudaGetLastError());
+    const size_t rows = sizeof(double) * 10 * (size_t)np;
+    const size_t room = (size_t)max_dynamic_smem((const void*)vectors_kernel<true>);
+    if (rows <= room) {
+        OPSEC_CUDA(cudaFuncSetAttribute(vectors_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+        vectors_kernel<true><<<grid, 128, rows, s>>>(a, p.R, per);
+    } else {
+        vectors_kernel<false><<<grid, 128, 0, s>>>(a, p.R, per);
+    }
     OPSEC_CUDA(cudaGetLastError());
     if (g_clock) g_clock->end(s);
-    cluster_kernel<<<p.nblk, 256, 0, s>>>(a, 1e-6);
+    cluster_kernel<<<dim3(p.nblk, p.kmax), 256, 0, s>>>(a, 1e-6);
     OPSEC_CUDA(cudaGetLastError());
     if (g_clock) g_clock->begin("blockeig_back", s, 2.0 * p.n * (double)p.n * p.ktot);
     const int groups = (p.n - 2 + kR - 1) / kR * p.nblk;
@@ -1001,7 +1054,9 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     const int cap = max_dynamic_smem((const void*)backtransform_kernel<4>);
     const size_t vec = sizeof(float2) * (size_t)p.n;
     auto warps_of = [&](int nv) { return (int)std::min<size_t>(4, (size_t)cap / (vec * nv + sizeof(float2) * kRing)); };
-    int nv = p.ktot < 16 * nsm ? 1 : p.ktot >= 24 * nsm && p.n > 384 && p.n <= 576 ? 4 : 2;
+    // On one dense matrix the reflectors leave L2 behind: two from 2,400 rows on (2730^2, 890 vectors: 14.3
+    // ms, one 17.5, four 22.4; 1728^2, 530 vectors: one 3.6, two 5.8).
+    int nv = p.n >= 2400 ? 2 : p.ktot < 16 * nsm ? 1 : p.ktot >= 24 * nsm && p.n > 384 && p.n <= 576 ? 4 : 2;
     while (nv > 1 && warps_of(nv) < 1) nv /= 2;
     if (nv == 4)
         launch_back<4>(a, p, warps_of(4), s);
@@ -1010,7 +1065,7 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     else
         launch_back<1>(a, p, warps_of(1), s);
     if (g_clock) g_clock->end(s);
-    *launches += 4;
+    *launches += 5;
 }
 
 }  // namespace opsec

@@ -150,7 +150,7 @@ struct opsec_gpu {
     DevBuf<double> nba_band;     // per-arc Nbar read by the band-block transforms
     DevBuf<double> nba_dev;      // Nbar per arc
     DevBuf<unsigned char> syev_ws;  // batched eigensolver workspace
-    DevBuf<double> bev_V, bev_T, bev_vec, bev_C;  // hand-written block eigensolver: reflectors, T, vectors
+    DevBuf<double> bev_V, bev_T, bev_vec, bev_C, bev_R, bev_X;  // hand-written block eigensolver: reflectors, T, vectors
     DevBuf<int> bev_i, bev_err;
     DevBuf<unsigned char> bev_D;  // its working matrix
     DevBuf<int> probe;  // opsec_gpu_wait_probe's status word

@@ -52,6 +52,13 @@ void drop_eig_graph(opsec_gpu* c) {
     c->eig_key = {};
 }
 
+// Dense problems of this order on (to tridiag_chip_supported's limit, 4,096) take the engine's own
+// kernels, open box with all else equal, top 29 %: 512 cells 14.9 -> 4.3 ms, 990 31.5 -> 10.4, 1,728
+// 67.7 -> 30.4, 2,730 156.6 -> 85.  Smaller ones gain as much (294 cells 9.0 -> 2.3 ms) but stay with
+// cuSOLVER: their C_p, rounded to FP32 in few modes, moves q by up to 1e-9 with any other rounding
+// of the vectors.  So do exactly degenerate S (exchange_symmetric), whose basis rounding picks.
+constexpr int kOwnDenseMin = 512;
+
 // Surveys whose Fisher matrix moves by over 1e-9 with the eigensolver's rounding (blockeig_small.cu):
 // few cells, or blocks that keep the modes even and odd in mu together (npar = 1) and not many cells.
 bool small_survey(int npar, long long cells) { return cells < 1024 || (npar == 1 && cells < 8192); }
@@ -77,7 +84,7 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     if (small)
         launch_small_tridiag(n, nblk, c->S.p, c->bev_V.p, tau, dg, eg, c->stream, &c->launches);
     else
-        launch_tridiag(n, nblk, c->S.p, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
+        launch_tridiag(n, nblk, false, c->S.p, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
                        &c->launches);
     if (g_clock) g_clock->end(c->stream);
     if (small)
@@ -157,6 +164,8 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
         p.V = c->bev_V.p;
         p.tau = tau;
         p.T = c->bev_C.p;
+        c->bev_R.alloc(blockeig_rows_doubles(n, nblk));
+        p.R = c->bev_R.p;
         p.out = c->S.p;
         if (g_clock) g_clock->begin("blockeig_vectors", c->stream, 2.0 * nn * ktot);
         launch_blockeig_vectors(p, c->stream, &c->launches);
@@ -175,6 +184,103 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     return true;
 }
 
+// Dense S of order n (c->S, kept) by the same steps on the whole GPU: the top M eigenpairs into
+// c->evals (descending) and c->modes.  False when a check in the kernels failed.
+bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
+    const size_t nn = (size_t)n * n;
+    c->bev_V.alloc(nn);
+    c->bev_T.alloc((size_t)3 * n + 1);
+    double* tau = c->bev_T.p;
+    double* dg = tau + n;
+    double* eg = dg + n;
+    double* scale = eg + n;
+    c->W.alloc(n);
+    c->bev_D.alloc(tridiag_work_bytes(n, 1));
+    c->bev_err.alloc(1);
+    OPSEC_CUDA(cudaMemsetAsync(c->bev_err.p, 0, sizeof(int), c->stream));
+    if (g_clock) g_clock->begin("blockeig_tridiag", c->stream, 4.0 / 3.0 * n * nn);
+    launch_tridiag(n, 1, true, c->S.p, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
+                   &c->launches);
+    if (g_clock) g_clock->end(c->stream);
+    launch_blockeig_spectrum(n, 1, dg, eg, c->W.p, scale, c->stream, &c->launches);
+    std::vector<double> w(n);
+    double sc = 1.0;
+    int err = 0;
+    OPSEC_CUDA(cudaMemcpyAsync(w.data(), c->W.p, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+    OPSEC_CUDA(cudaMemcpyAsync(&sc, scale, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    OPSEC_CUDA(cudaMemcpyAsync(&err, c->bev_err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    sync(c);
+    if (err) fail(OPSEC_ERR_CUDA, "tridiagonalisation: a wait between CTAs timed out");
+    // the same margin as for the blocks: every eigenvalue that can be among the top M once refined
+    const double cut = w[n - M] - 64.0 * FLT_EPSILON * sc;
+    int kc = M;
+    while (kc < n && w[n - 1 - kc] >= cut) kc++;
+    kc = std::min(n, std::max(kc, M + std::max(32, M / 8)));  // a margin below the cut for the polish
+    c->eig_stats[4] = kc;
+    const int hi[3] = {kc, 0, 0};
+    c->bev_i.alloc(3);
+    OPSEC_CUDA(cudaMemcpyAsync(c->bev_i.p, hi, sizeof hi, cudaMemcpyHostToDevice, c->stream));
+    const size_t per = (size_t)n * kc;
+    c->bev_vec.alloc(3 * per + (size_t)((n + 1) / 2) * kc);
+    c->bev_C.alloc(blockeig_compact_doubles(n, 1));
+    c->bev_R.alloc(blockeig_rows_doubles(n, 1));
+    BlockEigVectors p{};
+    p.n = n;
+    p.nblk = 1;
+    p.ktot = p.kmax = kc;
+    p.kc = c->bev_i.p;
+    p.koff = c->bev_i.p + 1;
+    p.status = c->bev_i.p + 2;
+    p.dg = dg;
+    p.eg = eg;
+    p.scale = scale;
+    p.w = c->W.p;
+    p.Z = c->bev_vec.p;
+    p.X = p.Z + per;
+    p.Y = p.X + per;
+    p.K = reinterpret_cast<int*>(p.Y + per);
+    p.V = c->bev_V.p;
+    p.tau = tau;
+    p.T = c->bev_C.p;
+    p.R = c->bev_R.p;
+    c->bev_X.alloc(2 * per + (size_t)2 * kc * kc + (size_t)kc * M);
+    double* X = c->bev_X.p;
+    double *SX = X + per, *G = SX + per, *H = G + (size_t)kc * kc, *E = H + (size_t)kc * kc;
+    p.out = X;
+    p.rows = kc;
+    if (g_clock) g_clock->begin("blockeig_vectors", c->stream, 2.0 * nn * kc);
+    launch_blockeig_vectors(p, c->stream, &c->launches);
+    if (g_clock) g_clock->end(c->stream);
+    // The reduction and the back-transformation are good to 48 bits: vectors of neighbouring
+    // eigenvalues are off by 1e-12 of each other.  One first-order correction in FP64 over the kept
+    // vectors and the margin brings them to what an FP64 solve gives.
+    if (!c->blas) blas_check(cublasCreate(&c->blas), "cublasCreate");
+    blas_check(cublasSetStream(c->blas, c->stream), "cublasSetStream");
+    const double one = 1.0, zero = 0.0;
+    if (g_clock) g_clock->begin("dense_polish", c->stream, 2.0 * nn * kc + 2.0 * n * (double)kc * (1.5 * kc + M));
+    blas_check(cublasDgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, n, kc, n, &one, c->S.p, n, X, n, &zero, SX, n), "dgemm");
+    blas_check(cublasDsyrk(c->blas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, kc, n, &one, X, n, &zero, G, kc), "dsyrk");
+    blas_check(cublasDgemm(c->blas, CUBLAS_OP_T, CUBLAS_OP_N, kc, kc, n, &one, X, n, SX, n, &zero, H, kc), "dgemm");
+    launch_polish_coefficients(kc, M, G, H, 1e-12 * sc, E, c->evals.p, c->stream, &c->launches);
+    OPSEC_CUDA(cudaMemcpyAsync(c->modes.p, X, sizeof(double) * (size_t)n * M, cudaMemcpyDeviceToDevice, c->stream));
+    blas_check(cublasDgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, n, M, kc, &one, X, n, E, kc, &one, c->modes.p, n), "dgemm");
+    c->launches += 4;
+    if (g_clock) g_clock->end(c->stream);
+    int st = 0;
+    std::vector<double> ev(M);
+    OPSEC_CUDA(cudaMemcpyAsync(ev.data(), c->evals.p, sizeof(double) * M, cudaMemcpyDeviceToHost, c->stream));
+    OPSEC_CUDA(cudaMemcpyAsync(&st, p.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    sync(c);
+    if (st) {
+        c->warning = "dense eigensolver check " + std::to_string(st) + " failed; solved by cuSOLVER instead";
+        return false;
+    }
+    std::stable_sort(ev.begin(), ev.end(), std::greater<double>());  // refined one by one: equal to rounding
+    OPSEC_CUDA(cudaMemcpyAsync(c->evals.p, ev.data(), sizeof(double) * M, cudaMemcpyHostToDevice, c->stream));
+    sync(c);
+    return true;
+}
+
 // After a failed device allocation a buffer may have been released without being replaced:
 // nothing cached on the device is trusted, so the next call rebuilds what it needs.
 void forget_device_state(opsec_gpu* c) {
@@ -184,6 +290,32 @@ void forget_device_state(opsec_gpu* c) {
     if (!c->xi64.p || !c->xi32.p) c->tables_ok = false;
     c->az_valid = false;
     drop_eig_graph(c);
+}
+
+// True when a Cartesian survey looks the same with two of its axes exchanged (equal cell counts and
+// sizes, and Nbar): S then has exactly degenerate eigenvalues.  Only a full grid can.
+bool exchange_symmetric(const opsec_gpu* c, int ncells, const opsec_cell* cells) {
+    const Geometry& g = c->geo;
+    const int* n = g.n;
+    if (g.coordsys != 1 || (long long)ncells != (long long)n[0] * n[1] * n[2]) return false;
+    std::vector<double> nb(ncells, -1.0);
+    auto at = [&](int x, int y, int z) { return ((size_t)x * n[1] + y) * n[2] + z; };
+    for (int a = 0; a < ncells; a++) nb[at(cells[a].d1, cells[a].d2, cells[a].d3)] = cells[a].Nbar;
+    auto same = [](double x, double y) { return std::fabs(x - y) <= 1e-9 * std::max(std::fabs(x), std::fabs(y)); };
+    for (int p = 0; p < 3; p++) {
+        const int q = (p + 1) % 3;
+        if (n[p] != n[q] || !same((g.b[2 * p + 1] - g.b[2 * p]) / n[p], (g.b[2 * q + 1] - g.b[2 * q]) / n[q])) continue;
+        bool sym = true;
+        for (int x = 0; x < n[0] && sym; x++)
+            for (int y = 0; y < n[1] && sym; y++)
+                for (int z = 0; z < n[2] && sym; z++) {
+                    int d[3] = {x, y, z};
+                    std::swap(d[p], d[q]);
+                    sym = same(nb[at(x, y, z)], nb[at(d[0], d[1], d[2])]);
+                }
+        if (sym) return true;
+    }
+    return false;
 }
 
 int eigensolve(opsec_gpu* c, int ncells, const opsec_cell* cells, int M, bool want_modes) {
@@ -428,6 +560,9 @@ int eigensolve(opsec_gpu* c, int ncells, const opsec_cell* cells, int M, bool wa
         return M;
     }
     std::fill(c->eig_stats, c->eig_stats + 10, 0.0);
+    if (c->eig_solver == "auto" && c->az_own && N >= kOwnDenseMin && tridiag_chip_supported(N) && !exchange_symmetric(c, ncells, cells) &&
+        own_dense_eigensolve(c, N, M))
+        return M;
     c->W.alloc(N);
     c->info.alloc(1);
     // the 64-bit interface: the 32-bit one's workspace count overflows from N ~ 23,000 on

@@ -208,9 +208,11 @@ bool blockeig_supported(int n);
 // Householder tridiagonalisation (tridiag.cu) of nblk blocks of order n >= 3 (FP64, column-major,
 // lower triangle read): T = (dg, eg), the reflectors V[block][c][i] as (hi, lo) float pairs
 // (v[c+1] = 1) and tau, each [block][n].  work: tridiag_work_bytes() bytes.  *err (zeroed by the
-// caller) is set when a wait between CTAs ran out.
+// caller) is set when a wait between CTAs ran out.  chip: one block on the whole GPU instead of a
+// cluster (a cooperative launch; tridiag_chip_supported).
 size_t tridiag_work_bytes(int n, int nblk);
-void launch_tridiag(int n, int nblk, const double* A, double* V, double* tau, double* dg, double* eg, void* work,
+bool tridiag_chip_supported(int n);
+void launch_tridiag(int n, int nblk, bool chip, const double* A, double* V, double* tau, double* dg, double* eg, void* work,
                     int* err, long long wait_cycles, cudaStream_t s, long long* launches);
 void launch_blockeig_spectrum(int n, int nblk, const double* dg, const double* eg, double* w, double* scale,
                               cudaStream_t s, long long* launches);
@@ -229,11 +231,17 @@ struct BlockEigVectors {
     double* V;            // [nblk][n][n] reflectors, (hi, lo) float pairs
     const double* tau;    // [nblk][n]
     double* T;            // scratch, blockeig_compact_doubles()
+    double* R;            // scratch, blockeig_rows_doubles()
     double* out;          // [nblk][n][n] eigenvector columns, or with rows > 0 (one block) [rows][n], largest first
     int rows;
 };
 size_t blockeig_compact_doubles(int n, int nblk);
+size_t blockeig_rows_doubles(int n, int nblk);
 void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long* launches);
+// First-order correction X (I + E) of k approximate eigenvectors from G = X^T X and H = X^T S X
+// (k x k, lower triangles read): the k x m columns of E for the first m and their Rayleigh quotients.
+void launch_polish_coefficients(int k, int m, const double* G, const double* H, double tol, double* E, double* lam,
+                                cudaStream_t s, long long* launches);
 
 // The same for small surveys (blockeig_small.cu): A is overwritten.
 void launch_small_tridiag(int n, int nblk, double* A, double* V, double* tau, double* dg, double* eg, cudaStream_t s,

@@ -20,8 +20,10 @@
 //   * The pass runs on packed FP32 instructions (two columns an issue slot).
 // Bound by the FP32 pipe in the pass (44 % busy over all, with two warps a scheduler) and by the
 // step's chain of reductions (3.3 us of each step).  Against one triangle on clusters of four, with
-// partial sums and FP64 scalars: 34 blocks of 512^2 (the 32k-cell build) 8.19 -> 5.33 ms, 34 of
-// 1024^2 54.5 -> 36.4, 10 of 555^2 10.3 -> 4.87, 18 of 624^2 13.5 -> 7.24, 18 of 64^2 0.318 -> 0.226.
+// partial sums and FP64 scalars: 34 blocks of 512^2 (the 32k-cell build) 8.19 -> 5.18 ms, 34 of
+// 1024^2 54.5 -> 35.6, 10 of 555^2 10.3 -> 4.65, 18 of 624^2 13.5 -> 6.99, 18 of 64^2 0.318 -> 0.226.
+// One dense matrix on the chip: 990^2 5.5 ms, 1728^2 13.6, 2730^2 39.3 (8 us a step at 1728: the barrier
+// over 152 CTAs, the exchange through L2 and the reductions; 512 threads a CTA, spilling: 19.6).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -39,6 +41,8 @@ namespace {
 constexpr int kChunk = 64;   // columns of a pass step: two per lane
 constexpr int kDepth = 4;    // pass steps of a warp's rows under way from L2 (asynchronous copies)
 constexpr int kMaxC = 8;     // largest (portable) cluster
+constexpr int kElems = 4;    // vector entries of a thread in a cluster (n <= 4 x 256); 4, 8 or 16 on the chip
+constexpr int kChipT = 256;  // threads of a CTA on the chip
 
 // Vectors and matrix rows keep two neighbouring entries as (hi, hi, lo, lo): 16 bytes that load as
 // the operands of packed FP32 instructions (add/mul/fma .f32x2: two results an issue slot, each
@@ -317,7 +321,8 @@ __device__ __forceinline__ void pass_group(int j0, int ld, float* base, const in
     }
 }
 
-template <int T, int RG, bool CHIP>
+// n <= E T: a thread holds its entries of a step's vectors in registers.
+template <int T, int RG, int E, bool CHIP>
 __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
     constexpr int W = T / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -387,13 +392,11 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
             }
         }
         // the next pivot row, when it lives in shared memory, to where every CTA reads it
-        if (UPD && r0 % C == rank) {
-            const int lr = r0 / C, k = lr / W;
-            if (lr % W == warp && k >= a.kres) {
-                const float4* src = reinterpret_cast<const float4*>(rres + (size_t)(lr - W * a.kres) * 2 * ld);
-                float4* dst = reinterpret_cast<float4*>(D + (size_t)r0 * 2 * ld);
-                for (int j = (j0 >> 1) + lane; j < ld / 2; j += 32) __stcg(dst + j, src[j]);
-            }
+        if (UPD && r0 % C == rank && r0 / C / W >= a.kres) {
+            __syncthreads();
+            const float4* src = reinterpret_cast<const float4*>(rres + (size_t)(r0 / C - W * a.kres) * 2 * ld);
+            float4* dst = reinterpret_cast<float4*>(D + (size_t)r0 * 2 * ld);
+            for (int j = (j0 >> 1) + t; j < ld / 2; j += T) __stcg(dst + j, src[j]);
         }
     };
     using yes = std::true_type;
@@ -409,34 +412,41 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
     for (int i = t; i < 6 * ld; i += T) vcur[i] = 0.f;
     __syncthreads();
 
-    // reflector of the pivot column c1, whose entries from c1 on are in v (unscaled) and whose sum of
-    // squares below the first entry is this thread's share s; v becomes the reflector
+    // Reflector of the pivot column c1: x[q] is its entry c1 + t + T q (0 at c1), s this thread's share
+    // of the sum of squares below the first entry; the reflector goes to v.
     df tau{0.f, 0.f};
-    auto reflect = [&](int c1, df s, float* v) {
+    auto reflect = [&](int c1, df s, const df (&x)[E], float* v) {
         const df s2 = cta_sum<W>(s, red + 32);
         const Reflector h = reflector(df_unpack(x0s[1]), s2);
-        for (int i = c1 + 2 + t; i < n; i += T) put(v, i, df_mul(get(v, i), h.scal));
-        if (t == 0) {
-            put(v, c1 + 1, df{1.f, 0.f});
-            if (rank == 0) {
-                a.eg[(size_t)b * n + c1] = df_to(h.beta);
-                a.tau[(size_t)b * n + c1] = df_to(h.tau);
-            }
+#pragma unroll
+        for (int q = 0; q < E; q++) {
+            const int i = c1 + t + T * q;
+            if (c1 + T * q >= n) break;
+            if (i < n) put(v, i, i == c1 + 1 ? df{1.f, 0.f} : df_mul(x[q], h.scal));
+        }
+        if (t == 0 && rank == 0) {
+            a.eg[(size_t)b * n + c1] = df_to(h.beta);
+            a.tau[(size_t)b * n + c1] = df_to(h.tau);
         }
         tau = h.tau;
     };
 
     // column 0
     {
-        df s{0.f, 0.f};
-        for (int i = t; i < n; i += T) {
-            const df x = getcg(D, i);
-            put(vnxt, i, i == 0 ? df{0.f, 0.f} : x);
-            if (i == 0 && rank == 0) a.dg[(size_t)b * n] = df_to(x);
-            if (i == 1) x0s[1] = df_pack(x);
-            if (i >= 2) s = df_fma(s, x, x);
+        df s{0.f, 0.f}, x[E];
+#pragma unroll
+        for (int q = 0; q < E; q++) {
+            const int i = t + T * q;
+            if (T * q >= n) break;
+            x[q] = i < n ? getcg(D, i) : df{0.f, 0.f};
+            if (i == 0) {
+                if (rank == 0) a.dg[(size_t)b * n] = df_to(x[q]);
+                x[q] = df{0.f, 0.f};
+            }
+            if (i == 1) x0s[1] = df_pack(x[q]);
+            if (i >= 2) s = df_fma(s, x[q], x[q]);
         }
-        reflect(0, s, vnxt);
+        reflect(0, s, x, vnxt);
         __syncthreads();
         if (rank == 0)
             for (int i = 1 + t; i < n; i += T) V[i] = df_pack(get(vnxt, i));
@@ -448,43 +458,57 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
         float* sw = vcur;
         vcur = vnxt;
         vnxt = sw;
-        // p = A v from the CTAs, y = tau p, y.v
-        df part{0.f, 0.f};
+        // p = A v from the CTAs and the pivot row before this step's update; y = tau p, y.v
         const float* rowc = D + (size_t)c1 * 2 * ld;
-        for (int i = c1 + t; i < n; i += T) {
-            float2 p2;
-            if constexpr (CHIP)
-                p2 = __ldcg(a.pbuf + (size_t)par * n + i);
-            else
-                p2 = C > 1 ? cluster.map_shared_rank(pown, i % C)[par * nlmax + i / C] : pown[par * nlmax + i];
-            put(vnxt, i, getcg(rowc, i));  // the pivot row, before this step's update
-            const df y = df_mul(tau, df_unpack(p2));
-            put(w, i, y);
-            if (i == c1) x0s[0] = df_pack(y);
-            part = df_fma(part, y, get(vcur, i));
+        df y[E], x[E], v[E];
+        float2 p2[E];
+#pragma unroll
+        for (int q = 0; q < E; q++) {
+            const int i = c1 + t + T * q;
+            if (c1 + T * q >= n) break;
+            p2[q] = make_float2(0.f, 0.f);
+            x[q] = v[q] = df{0.f, 0.f};
+            if (i < n) {
+                if constexpr (CHIP)
+                    p2[q] = __ldcg(a.pbuf + (size_t)par * n + i);
+                else
+                    p2[q] = C > 1 ? cluster.map_shared_rank(pown, i % C)[par * nlmax + i / C] : pown[par * nlmax + i];
+                x[q] = getcg(rowc, i);
+                v[q] = get(vcur, i);
+            }
         }
-        if (t == 0) put(w, c, df{0.f, 0.f});
+        df part{0.f, 0.f};
+#pragma unroll
+        for (int q = 0; q < E; q++) {
+            if (c1 + T * q >= n) break;
+            y[q] = df_mul(tau, df_unpack(p2[q]));
+            part = df_fma(part, y[q], v[q]);
+        }
+        if (t == 0) {
+            x0s[0] = df_pack(y[0]);
+            put(w, c, df{0.f, 0.f});
+            put(vnxt, c, df{0.f, 0.f});
+        }
         const df yv = cta_sum<W>(part, red);
         // w = y - (tau/2)(y.v) v; pivot column c1 under the update (v[c1] = 1)
         const df alpha = df_mul(tau, df{0.5f * yv.h, 0.5f * yv.l});
         const df wc = df_add(df_unpack(x0s[0]), df{-alpha.h, -alpha.l});
         df s{0.f, 0.f};
-        for (int i = c1 + t; i < n; i += T) {
-            const df v = get(vcur, i);
-            const df wi = df_fms(get(w, i), alpha, v);
-            put(w, i, wi);
-            df x = df_fms(get(vnxt, i), v, wc);
-            x = df_add(x, df{-wi.h, -wi.l});
+#pragma unroll
+        for (int q = 0; q < E; q++) {
+            const int i = c1 + t + T * q;
+            if (c1 + T * q >= n) break;
+            const df wi = df_fms(y[q], alpha, v[q]);
+            if (i < n) put(w, i, wi);
+            x[q] = df_add(df_fms(x[q], v[q], wc), df{-wi.h, -wi.l});
             if (i == c1) {
-                if (rank == 0) a.dg[(size_t)b * n + c1] = df_to(x);
-                x = df{0.f, 0.f};
+                if (rank == 0) a.dg[(size_t)b * n + c1] = df_to(x[q]);
+                x[q] = df{0.f, 0.f};
             }
-            put(vnxt, i, x);
-            if (i == c1 + 1) x0s[1] = df_pack(x);
-            if (i > c1 + 1) s = df_fma(s, x, x);
+            if (i == c1 + 1) x0s[1] = df_pack(x[q]);
+            if (i > c1 + 1) s = df_fma(s, x[q], x[q]);
         }
-        if (t == 0) put(vnxt, c, df{0.f, 0.f});
-        reflect(c1, s, vnxt);
+        reflect(c1, s, x, vnxt);
         __syncthreads();
         if (rank == c1 % C)
             for (int i = (c1 & ~3) + 1 + t; i < n; i += T) V[(size_t)c1 * n + i] = df_pack(get(vnxt, i));
@@ -551,7 +575,7 @@ int max_clusters(int C) {
     OPSEC_CUDA(cudaGetDevice(&dev));
     int v = dev < 64 ? cache[dev][C].load() : 0;
     if (v <= 0) {
-        auto k = tridiag_kernel<T, RG, false>;
+        auto k = tridiag_kernel<T, RG, kElems, false>;
         const int cap = max_dynamic_smem((const void*)k);
         OPSEC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
         cudaLaunchAttribute at{};
@@ -576,7 +600,7 @@ int cluster_of(int n, int nblk) {
 template <int T, int RG>
 void launch_blocks(TridiagArgs a, int nblk, cudaStream_t s) {
     a.C = cluster_of<T, RG>(a.n, nblk);
-    auto k = tridiag_kernel<T, RG, false>;
+    auto k = tridiag_kernel<T, RG, kElems, false>;
     const size_t cap = (size_t)max_dynamic_smem((const void*)k), base = smem_base(a.n, a.C, T / 32, RG);
     if (base > cap) fail(OPSEC_ERR_CUDA, "tridiagonalisation: block too large for shared memory");
     residency(a, T / 32, RG, cap - base);
@@ -587,15 +611,32 @@ void launch_blocks(TridiagArgs a, int nblk, cudaStream_t s) {
     OPSEC_CUDA(cudaLaunchKernelEx(&cfg, k, a));
 }
 
+template <int E>
+void launch_chip(TridiagArgs a, cudaStream_t s) {
+    auto k = tridiag_kernel<kChipT, 2, E, true>;
+    a.C = std::min(sm_count(), a.n);
+    const size_t cap = (size_t)max_dynamic_smem((const void*)k), base = smem_base(a.n, a.C, kChipT / 32, 2);
+    if (base > cap) fail(OPSEC_ERR_CUDA, "tridiagonalisation: matrix too large for shared memory");
+    residency(a, kChipT / 32, 2, cap - base);
+    OPSEC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    OPSEC_CUDA(cudaMemsetAsync(a.count, 0, sizeof(unsigned), s));
+    void* args[] = {&a};
+    OPSEC_CUDA(cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)a.C), dim3(kChipT), args,
+                                           base + sizeof(float2) * (size_t)a.ld * a.nres, s));
+}
+
 }  // namespace
 
 size_t tridiag_work_bytes(int n, int nblk) {
     return sizeof(float2) * ((size_t)nblk * n * pad(n) + 2 * (size_t)n) + 64;
 }
 
-bool tridiag_dense_supported(int n) { return n >= 3 && smem_base(n, 152, 16, 2) <= (size_t)max_dynamic_smem((const void*)tridiag_kernel<512, 2, true>); }
+bool tridiag_chip_supported(int n) {
+    return n >= 3 && n <= 4 * kElems * kChipT &&
+           smem_base(n, 152, kChipT / 32, 2) <= (size_t)max_dynamic_smem((const void*)tridiag_kernel<kChipT, 2, 4 * kElems, true>);
+}
 
-void launch_tridiag(int n, int nblk, const double* A, double* V, double* tau, double* dg, double* eg, void* work,
+void launch_tridiag(int n, int nblk, bool chip, const double* A, double* V, double* tau, double* dg, double* eg, void* work,
                     int* err, long long wait_cycles, cudaStream_t s, long long* launches) {
     TridiagArgs a{};
     a.n = n;
@@ -612,17 +653,13 @@ void launch_tridiag(int n, int nblk, const double* A, double* V, double* tau, do
     pairs_kernel<<<dim3((n + 31) / 32, (n + 31) / 32, nblk), 256, 0, s>>>(n, a.ld, A, a.D);
     OPSEC_CUDA(cudaGetLastError());
     ++*launches;
-    if (nblk == 1 && n > 1024) {
-        auto k = tridiag_kernel<512, 2, true>;
-        a.C = std::min(sm_count(), n);
-        const size_t cap = (size_t)max_dynamic_smem((const void*)k), base = smem_base(n, a.C, 16, 2);
-        if (base > cap) fail(OPSEC_ERR_CUDA, "tridiagonalisation: matrix too large for shared memory");
-        residency(a, 512 / 32, 2, cap - base);
-        OPSEC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-        OPSEC_CUDA(cudaMemsetAsync(a.count, 0, sizeof(unsigned), s));
-        void* args[] = {&a};
-        OPSEC_CUDA(cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)a.C), dim3(512), args,
-                                               base + sizeof(float2) * (size_t)a.ld * a.nres, s));
+    if (chip && nblk == 1) {
+        if (n <= kElems * kChipT)
+            launch_chip<kElems>(a, s);
+        else if (n <= 2 * kElems * kChipT)
+            launch_chip<2 * kElems>(a, s);
+        else
+            launch_chip<4 * kElems>(a, s);
     } else {
         launch_blocks<256, 4>(a, nblk, s);
     }
