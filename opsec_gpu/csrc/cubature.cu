@@ -404,6 +404,7 @@ struct WinPlan {
     int flush;    // Cartesian window kernel: second-cell points per loop chunk (0: all)
     int dot64;    // compensated dot products for every key (1) or only where windows cancel strongly (0)
     float qinv;   // coarse fixed-point units per unit of pair weight (2^k / largest pair weight)
+    float nzero;  // -0
     float qfrac;  // fraction units per coarse unit (2^fbits)
     int fbits;
     float qfine;  // pair weight per unit of the 64-bit histogram (2^-fbits / qinv)
@@ -764,11 +765,11 @@ __global__ void __launch_bounds__(kPartThreads) part_scatter_kernel(long long nk
 // two native 32-bit integer shared-memory atomics; neither partial sum can
 // overflow within a pass, at whose end the dot products combine them into the
 // 64-bit value.  The sums are exact and independent of the order of the atomics.
-// Each warp keeps two copies of its histogram, one per half-warp, interleaved
-// (copy c of bin b at word 2b + c): the lanes' bins collide in shared-memory
-// banks, and the copies cut the wavefronts per atomic from 3.6 to 2.7 (a model
-// of the 32k-cell shell's bins; no extra memory: the 64-bit staging histogram
-// is gone).
+// A warp's lanes collide in the histogram's banks and, where windows are narrow, in its bins, so a
+// key's bins are kept in as many copies (2 to 32, a power of two) as its window leaves room for,
+// 2^lg of them, copy c of bin b at word (b << lg) + c, lane l adding to copy l >> (5 - lg).  By a
+// model of the bins, wavefronts of a key's atomics against two copies: 32k-cell shell (median
+// window 73 bins) 950 -> 760, mock surveys on the 512 + 256 table (14 bins) 2,300 -> 440.
 // (64-bit integer shared atomics instead: cubature 90 ms against 66 ms at 32k
 // cells.)
 // (FP32 shared-memory atomics were slower -- the counters showed them retried
@@ -798,37 +799,23 @@ __device__ __forceinline__ void add_fixed(int* hqa, int* hqb, int b, float x, fl
     atomicAdd(&hqb[b], __float_as_int(fmaf(f, frac, kMagic)) - kMagicBits);
 }
 
-// Table index (i, fr) of r^2 = r2 + r2l when r^2 >= r1^2 is known (every pair of a key whose
-// window starts above the linear section): index_r2's log branch with the same operations
-// and roundings, its exponent clamp and 2^-E folded into a table indexed by the biased
-// exponent, s_ce[eb] = (2^(127-eb), fraction of c_e, integer part of c_e - kMagicBits, 0),
-// the mantissa table split into (1/T_k, fraction of z_k) pairs and the integer parts of z_k
-// (8 + 2 bytes per entry instead of 16: the lanes' random entries cost fewer shared-memory
-// wavefronts), and floor(y) from an FP32 addition rounded down.
-__device__ __forceinline__ void index_log(const Lookup& lk, const float4* s_ce, const float2* s_kt2,
-                                          const unsigned short* s_kz, float r2, float r2l, int& i, float& fr) {
-    const unsigned u = __float_as_uint(r2) >> (23 - kLogBits);  // exponent and top mantissa bits
-    const float4 ce = s_ce[(u >> kLogBits) & 255];
-    const int k = u & (kLogN - 1);
-    const float2 kt = s_kt2[k];
-    const float Rk = __uint_as_float(u << (23 - kLogBits));
-    const float delta = ((r2 - Rk) + r2l) * (kt.x * ce.x);
-    const float ln1p = delta * fmaf(-delta, fmaf(-delta, fmaf(-delta, 0.25f, 1.f / 3.f), 0.5f), 1.f);
-    const float y = fmaf(ln1p, lk.cp, ce.y + kt.y);
-    const float s = __fadd_rd(y, kMagic);  // kMagic + floor(y), |y| < 2^22
-    i = __float_as_int(ce.z) + (int)s_kz[k] + __float_as_int(s);
-    fr = __fsub_rn(y, __fsub_rn(s, kMagic));
-    if (i > lk.imax) {
-        i = lk.imax;
-        fr = 1.0f;
-    }
+// log2 of a key's copies: one a lane where that fits, two for windows wider than kNarrow bins, where
+// summing more copies and shifting by a variable cost more than the atomics gain (one rule for all
+// windows: 32k-cell shell's build 60.5 ms, with two copies beyond 48 bins 57.3 ms; 16 mock surveys on
+// narrow windows 293 ms with two, 242 ms with up to 32)
+constexpr int kNarrow = 48;
+__device__ __forceinline__ int copies_log2(int Wkey, int n) {
+    int lg = 1;
+    while (n <= kNarrow && lg < 5 && (n << (lg + 1)) <= 2 * Wkey) ++lg;
+    return lg;
 }
 
-// Clear bins [0, n) of both copies.  Warp-wide.
-__device__ __forceinline__ void clear_fixed(int* hqa, int* hqb, int n, int lane) {
-    for (int j = lane; j < 2 * n; j += 32) {
-        hqa[j] = 0;
-        hqb[j] = 0;
+// Clear the copies of bins [0, n).  Rows are 16-byte aligned.  Warp-wide.
+__device__ __forceinline__ void clear_fixed(int* hqa, int* hqb, int n, int lg, int lane) {
+    const int4 zero = make_int4(0, 0, 0, 0);
+    for (int j = lane; 4 * j < n << lg; j += 32) {  // the last store may pass the last bin, not 2 Wkey
+        reinterpret_cast<int4*>(hqa)[j] = zero;
+        reinterpret_cast<int4*>(hqb)[j] = zero;
     }
     __syncwarp();
 }
@@ -847,18 +834,26 @@ constexpr int kDotChunk = 16;  // bins summed in FP32 per compensated addition i
 // values as FP32 high + low parts -- about FP64 accuracy.  The bin values replace the partial
 // sums in place: hp[b] is word b of hqa, hl[b] word b of hqb.  Warp-wide.
 __device__ __forceinline__ void window_dots(const CubatureArgs& a, const WinPlan& w, int* hqa, int* hqb, int key,
-                                            int wx, int s0, int segw, int pass, bool precise, int lane) {
+                                            int wx, int s0, int segw, int lg, int pass, bool precise, int lane) {
     const int ntab = a.ntab;
     float* hp = reinterpret_cast<float*>(hqa);
     float* hl = reinterpret_cast<float*>(hqb);
-    // bin b's two copies are words 2b, 2b+1, and its value goes to word b: the 32 bins of a
-    // sweep read words [64k, 64k + 64) and write [32k, 32k + 32), whose inputs earlier sweeps
-    // (or this one, before the barrier) have read
+    // bin b's copies are words (b << lg) .., and its value goes to word b: the 32 bins of sweep k read
+    // words [32k << lg, ..) and write [32k, 32k + 32), which earlier sweeps (or this one, before the
+    // barrier) have read.  The lanes start at different copies: same-numbered ones share banks.
+    const int nc = 1 << lg;
     for (int b0 = 0; b0 < segw; b0 += 32) {
         const int b = b0 + lane;
         long long v = 0;
-        if (b < segw)
-            v = (((long long)hqa[2 * b] + hqa[2 * b + 1]) << w.fbits) + (long long)hqb[2 * b] + hqb[2 * b + 1];
+        if (b < segw) {
+            int sa = 0, sb = 0;
+            for (int c = 0; c < nc; c++) {
+                const int o = (b << lg) + ((c + lane) & (nc - 1));
+                sa += hqa[o];
+                sb += hqb[o];
+            }
+            v = ((long long)sa << w.fbits) + sb;
+        }
         __syncwarp();
         if (b < segw) {
             if (precise) {
@@ -926,6 +921,118 @@ __device__ __forceinline__ void window_dots(const CubatureArgs& a, const WinPlan
 }
 
 
+// Packed FP32: two values an instruction, each rounded as the scalar instruction rounds.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void upk(f2 x, float* a, float* b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(x)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 add2_rd(f2 a, f2 b) {
+    f2 r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// The spherical kernel's log-section loop over a node pair's canonical phi-node pairs, two at a time
+// in packed FP32: the operations of the scalar statements beside them, with the same roundings
+// (signs are moved where the packed instructions have no negation).  SX: (x, x', y, y') of two
+// pairs' sin^2(theta/2) = x + y, SZ: their weights (0 for the one that evens out the count).
+// Products that an addition reads are written as fma(x, y, nz) with nz = -0 at run time: the same value,
+// and ptxas (13.0) joins a mul.rn.f32x2 and an addition into one fma.f32x2 although both are .rn.
+// What bounds it is issue: of its 93 instructions a pair the packed form takes about 30 away, and the
+// four shared atomics a pair come next (whole builds, scalar to packed: 32k-cell shell 57.3 -> 55.6 ms,
+// 65k 278 -> 270 ms, 16 mock surveys 242 -> 233 ms, a 2k-cell signal block 1.09 -> 1.07 ms).
+// NARROW: the histogram in 2^lg copies (else two).
+template <int NC2, bool NARROW>
+__device__ __forceinline__ int log_pairs(const ulonglong2* SX, const f2* SZ, const float4* s_ce, const float2* s_kt2,
+                                         const unsigned short* s_kz, float B4h, float B4l, float Dh, float Dl, float wpq,
+                                         float cp, float qinv, float qfrac, float nzero, int wx, int wl, int* hqa, int* hqb, int lg,
+                                         int cpy) {
+    const f2 kM = pk(kMagic, kMagic), nb4 = pk(-B4h, -B4h), b4 = pk(B4h, B4h), b4l = pk(B4l, B4l), dh = pk(Dh, Dh),
+             dl = pk(Dl, Dl), wp = pk(wpq, wpq), ncp = pk(-cp, -cp), q2 = pk(qinv, qinv), fr2 = pk(qfrac, qfrac),
+             nf2 = pk(-qfrac, -qfrac), nz = pk(nzero, nzero);
+    int bad = 0;
+#pragma unroll 1
+    for (int j = 0; j < NC2; j++) {
+        const ulonglong2 sp = SX[j];
+        const f2 sz = SZ[j];
+        const f2 nt = fma2(nb4, sp.x, nz);                                             // -t, t = B4h x
+        const f2 tl = add2(fma2(b4, sp.x, nt), fma2(b4, sp.y, mul2(b4l, sp.x)));
+        const f2 r2 = sub2(dh, nt);                                                  // two_sum(Dh, t, e)
+        const f2 bb = sub2(r2, dh);
+        const f2 e = sub2(sub2(dh, sub2(r2, bb)), add2(nt, bb));
+        const f2 r2l = add2(add2(e, dl), tl);
+        // table index: as index_r2 above the linear section, exponent and mantissa tables
+        float r0, r1;
+        upk(r2, &r0, &r1);
+        const unsigned u0 = __float_as_uint(r0) >> (23 - kLogBits), u1 = __float_as_uint(r1) >> (23 - kLogBits);
+        const float4 c0 = s_ce[(u0 >> kLogBits) & 255], c1 = s_ce[(u1 >> kLogBits) & 255];
+        const int k0 = u0 & (kLogN - 1), k1 = u1 & (kLogN - 1);
+        const float2 t0 = s_kt2[k0], t1 = s_kt2[k1];  // (-1/T_k, fraction of z_k)
+        const f2 Rk = pk(__uint_as_float(u0 << (23 - kLogBits)), __uint_as_float(u1 << (23 - kLogBits)));
+        const f2 nd = mul2(add2(sub2(r2, Rk), r2l), mul2(pk(t0.x, t1.x), pk(c0.x, c1.x)));  // -delta
+        const f2 p = fma2(nd, fma2(nd, fma2(nd, pk(0.25f, 0.25f), pk(1.f / 3.f, 1.f / 3.f)), pk(0.5f, 0.5f)), pk(1.f, 1.f));
+        const f2 y = fma2(mul2(nd, p), ncp, add2(pk(c0.y, c1.y), pk(t0.y, t1.y)));
+        const f2 sy = add2_rd(y, kM);            // kMagic + floor(y)
+        const f2 nfr = sub2(sub2(sy, kM), y);    // -fraction
+        float s0, s1;
+        upk(sy, &s0, &s1);
+        int i0 = __float_as_int(c0.z) + (int)s_kz[k0] + __float_as_int(s0) - wx;
+        int i1 = __float_as_int(c1.z) + (int)s_kz[k1] + __float_as_int(s1) - wx;
+        if (max((unsigned)i0, (unsigned)i1) > (unsigned)(wl - 2)) {  // outside the window: cannot happen for a sound window
+            bad += ((unsigned)i0 > (unsigned)(wl - 2)) + ((unsigned)i1 > (unsigned)(wl - 2));
+            i0 = min(max(i0, 0), wl - 2);
+            i1 = min(max(i1, 0), wl - 2);
+        }
+        const f2 wq = mul2(mul2(wp, sz), q2);
+        const f2 A = fma2(wq, nfr, wq), nB = fma2(wq, nfr, nz);  // wq (1 - fr), -wq fr
+        // add_fixed of A to bin i, of B to bin i + 1
+        const f2 as = add2(A, kM), af = fma2(sub2(A, sub2(as, kM)), fr2, kM);
+        const f2 bs = sub2(kM, nB), bf = fma2(add2(nB, sub2(bs, kM)), nf2, kM);
+        float a0, a1, f0, f1, b0, b1, g0, g1;
+        upk(as, &a0, &a1);
+        upk(af, &f0, &f1);
+        upk(bs, &b0, &b1);
+        upk(bf, &g0, &g1);
+        const int sh = NARROW ? lg : 1, st = NARROW ? 1 << lg : 2;
+        const int o0 = (i0 << sh) + cpy, o1 = (i1 << sh) + cpy;
+        atomicAdd(&hqa[o0], __float_as_int(a0) - kMagicBits);
+        atomicAdd(&hqb[o0], __float_as_int(f0) - kMagicBits);
+        atomicAdd(&hqa[o0 + st], __float_as_int(b0) - kMagicBits);
+        atomicAdd(&hqb[o0 + st], __float_as_int(g0) - kMagicBits);
+        atomicAdd(&hqa[o1], __float_as_int(a1) - kMagicBits);
+        atomicAdd(&hqb[o1], __float_as_int(f1) - kMagicBits);
+        atomicAdd(&hqa[o1 + st], __float_as_int(b1) - kMagicBits);
+        atomicAdd(&hqb[o1 + st], __float_as_int(g1) - kMagicBits);
+    }
+    return bad;
+}
+
+// float4s of a warp's phi-node pairs, two by two: x and y 16 bytes, weights 8
+__host__ __device__ constexpr int sph_pairs(int nc) { return (nc + 1) / 2 + ((nc + 1) / 2 + 1) / 2; }
+
 template <int NG>
 struct FarShape {
     static constexpr int NP = NG * NG * NG;
@@ -940,8 +1047,8 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
     constexpr int kWarps = FarShape<NG>::kWarps;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float4* pts = reinterpret_cast<float4*>(smem_raw);                  // [kWarps][2][NP]
-    int* pa = reinterpret_cast<int*>(pts + kWarps * 2 * NP);  // [kWarps][Wkey][2]: partial sums, integer part
-    int* pb = pa + 2 * kWarps * w.Wkey;                       // [kWarps][Wkey][2]: partial sums, fraction
+    int* pa = reinterpret_cast<int*>(pts + kWarps * 2 * NP);  // [kWarps][2 Wkey]: partial sums, integer part
+    int* pb = pa + 2 * kWarps * w.Wkey;                       // [kWarps][2 Wkey]: partial sums, fraction
     __shared__ int s_ci[kMaxExp];
     __shared__ float s_cf[kMaxExp];
     __shared__ float4 s_kt[kLogN];
@@ -957,7 +1064,6 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
     float4* P2l = P2 + NP;
     int* hqa = pa + 2 * warp * w.Wkey;
     int* hqb = pb + 2 * warp * w.Wkey;
-    const int cpy = lane >> 4;  // this lane's histogram copy
     const bool periodic = (a.coordsys == 1 && a.L > 0);
     const float Lh = (float)a.L, Ll = (float)(a.L - (double)Lh), hL = 0.5f * Lh;
     const int nfar = *w.nfar;
@@ -1009,7 +1115,8 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
                     f_hi = r * r;
                 }
             }
-            clear_fixed(hqa, hqb, segw, lane);
+            const int lg = copies_log2(w.Wkey, segw), cpy = lane >> (5 - lg);  // this lane's histogram copy
+            clear_fixed(hqa, hqb, segw, lg, lane);
             // Mirror symmetry of the innermost axis (phi on spherical grids, z on Cartesian
             // ones): the Gauss nodes are symmetric about each cell's centre, so the pair of
             // innermost nodes (l_p, l_q) and (NG-1-l_q, NG-1-l_p) have the same separation
@@ -1055,15 +1162,15 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
                                 bad += out;
                                 const float ww = (lsum < NG - 1 ? 2.f : 1.f) * Ah.w * B.w;
                                 const float wq = ww * w.qinv;  // fixed point: the largest pair weight -> 2^k units
-                                add_fixed(hqa, hqb, 2 * bi + cpy, fmaf(-wq, fr, wq), w.qfrac);
-                                add_fixed(hqa, hqb, 2 * bi + 2 + cpy, wq * fr, w.qfrac);
+                                add_fixed(hqa, hqb, (bi << lg) + cpy, fmaf(-wq, fr, wq), w.qfrac);
+                                add_fixed(hqa, hqb, ((bi + 1) << lg) + cpy, wq * fr, w.qfrac);
                             }
                         }
                     }
                 }
             }
             __syncwarp();
-            window_dots(a, w, hqa, hqb, key, wn.x, s0, segw, pass,
+            window_dots(a, w, hqa, hqb, key, wn.x, s0, segw, lg, pass,
                         w.dot64 || npass > 1 || wn.x < lk.n1, lane);
         }
         if (bad) atomicAdd(w.violations, bad);
@@ -1085,19 +1192,19 @@ template <int NG>
 __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
     cubature_far_sph_kernel(CubatureArgs a, Lookup lk, WinPlan w) {
     constexpr int NG2 = NG * NG;
-    constexpr int NC = NG * (NG + 1) / 2;
+    constexpr int NC = NG * (NG + 1) / 2, NC2 = (NC + 1) / 2;
     constexpr int kWarps = FarShape<NG>::kWarps;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4* sphw = reinterpret_cast<float4*>(smem_raw);        // [kWarps][NC]: the key's phi-node pairs
-    int* pa = reinterpret_cast<int*>(sphw + kWarps * NC);  // [kWarps][Wkey][2]: partial sums, integer part
+    float4* sphw = reinterpret_cast<float4*>(smem_raw);  // [kWarps][sph_pairs(NC)]: the key's phi-node pairs
+    int* pa = reinterpret_cast<int*>(sphw + kWarps * sph_pairs(NC));  // [kWarps][Wkey][2]: partial sums, integer part
     int* pb = pa + 2 * kWarps * w.Wkey;                    // [kWarps][Wkey][2]: partial sums, fraction
     __shared__ int s_ci[kMaxExp];
     __shared__ float s_cf[kMaxExp];
     __shared__ float4 s_kt[kLogN];
     __shared__ float s_wrm[NG2];
-    __shared__ float4 s_ce[256];  // index_log's exponent table
-    __shared__ float2 s_kt2[kLogN];          // index_log: 1/T_k, fraction of z_k
-    __shared__ unsigned short s_kz[kLogN];   // index_log: integer part of z_k
+    __shared__ float4 s_ce[256];  // log_pairs' exponent table
+    __shared__ float2 s_kt2[kLogN];          // log_pairs: -1/T_k, fraction of z_k
+    __shared__ unsigned short s_kz[kLogN];   // log_pairs: integer part of z_k
     for (int i = threadIdx.x; i < lk.ne; i += blockDim.x) {
         s_ci[i] = lk.ci[i];
         s_cf[i] = lk.cf[i];
@@ -1105,7 +1212,7 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
     for (int i = threadIdx.x; i < kLogN; i += blockDim.x) {
         const float4 kt = lk.kt[i];
         s_kt[i] = kt;
-        s_kt2[i] = make_float2(kt.x, kt.y);
+        s_kt2[i] = make_float2(-kt.x, kt.y);
         s_kz[i] = (unsigned short)__float_as_int(kt.z);  // < 2^16: checked on the host
     }
     for (int i = threadIdx.x; i < NG2; i += blockDim.x) s_wrm[i] = w.wrm[i];
@@ -1117,10 +1224,10 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
     __syncthreads();
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float4* SP = sphw + warp * NC;
+    ulonglong2* SX = reinterpret_cast<ulonglong2*>(sphw + warp * sph_pairs(NC));
+    f2* SZ = reinterpret_cast<f2*>(SX + NC2);
     int* hqa = pa + 2 * warp * w.Wkey;
     int* hqb = pb + 2 * warp * w.Wkey;
-    const int cpy = lane >> 4;  // this lane's histogram copy
     const int nfar = *w.nfar;
     for (int kk = blockIdx.x * kWarps + warp; kk < nfar; kk += gridDim.x * kWarps) {
         const int key = w.order[kk];
@@ -1129,7 +1236,13 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
         int c1[3], c2[3];
         decode_key(a.ks, key, c1, c2);
         const int ha = c1[0] * a.ks.N2 + c1[1], hb = c2[0] * a.ks.N2 + c2[1], df = c2[2];
-        for (int c = lane; c < NC; c += 32) SP[c] = w.sph[(size_t)df * NC + c];
+        for (int c = lane; c < 2 * NC2; c += 32) {
+            const float4 v = w.sph[(size_t)df * NC + min(c, NC - 1)];
+            float* x = reinterpret_cast<float*>(SX + (c >> 1)) + (c & 1);
+            x[0] = v.x;
+            x[2] = v.y;
+            reinterpret_cast<float*>(SZ)[c] = c < NC ? v.z : 0.f;
+        }
         const float4* AA = w.arc + (size_t)ha * NG2;
         const float4* AB = w.arc + (size_t)hb * NG2;
         __syncwarp();
@@ -1151,11 +1264,13 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
                     f_hi = r * r;
                 }
             }
-            clear_fixed(hqa, hqb, segw, lane);
+            const int lg = copies_log2(w.Wkey, segw), cpy = lane >> (5 - lg);  // this lane's histogram copy
+            clear_fixed(hqa, hqb, segw, lg, lane);
             // One pass whose window starts above the linear section of the table (most far
-            // keys): every pair has r^2 >= r1^2 and its bin is in the histogram, so the loop
-            // below needs neither the linear branch nor the pass filter.
-            const bool logkeys = w.logkeys && npass == 1 && wn.x > lk.n1;
+            // keys) and ends before the table does: every pair has r^2 >= r1^2 and its bin is in
+            // the histogram, so log_pairs needs neither the linear branch, the pass filter nor the
+            // clamp to the table's last bin.
+            const bool logkeys = w.logkeys && npass == 1 && wn.x > lk.n1 && wn.x + wl < a.xl.n();
             // lanes take the (P, Q) node pairs; every lane runs the same trip counts
             for (int c0 = 0; c0 < NG2 * NG2; c0 += 32) {
                 const int c = c0 + lane;
@@ -1175,32 +1290,16 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
                     const float B4l = 4.f * (fmaf(A.x, B.x, -t0) + fmaf(A.x, B.y, A.y * B.x));
                     const float wpq = s_wrm[P] * s_wrm[Q];
                     if (logkeys) {
-#pragma unroll 2
-                        for (int j = 0; j < NC; j++) {
-                            const float4 sp = SP[j];
-                            const float t = __fmul_rn(B4h, sp.x);
-                            const float tl = fmaf(B4h, sp.x, -t) + fmaf(B4h, sp.y, B4l * sp.x);
-                            float e;
-                            const float r2 = two_sum(Dh, t, &e);
-                            const float r2l = e + Dl + tl;
-                            int i;
-                            float fr;
-                            index_log(lk, s_ce, s_kt2, s_kz, r2, r2l, i, fr);
-                            int bi = i - wn.x;
-                            if ((unsigned)bi > (unsigned)(wl - 2)) {  // outside the window: cannot happen for a sound window
-                                ++bad;
-                                bi = min(max(bi, 0), wl - 2);
-                            }
-                            const float ww = wpq * sp.z;
-                            const float wq = ww * w.qinv;
-                            add_fixed(hqa, hqb, 2 * bi + cpy, fmaf(-wq, fr, wq), w.qfrac);
-                            add_fixed(hqa, hqb, 2 * bi + 2 + cpy, wq * fr, w.qfrac);
-                        }
+                        bad += lg > 1 ? log_pairs<NC2, true>(SX, SZ, s_ce, s_kt2, s_kz, B4h, B4l, Dh, Dl, wpq, lk.cp, w.qinv,
+                                                             w.qfrac, w.nzero, wn.x, wl, hqa, hqb, lg, cpy)
+                                      : log_pairs<NC2, false>(SX, SZ, s_ce, s_kt2, s_kz, B4h, B4l, Dh, Dl, wpq, lk.cp, w.qinv,
+                                                              w.qfrac, w.nzero, wn.x, wl, hqa, hqb, 1, cpy);
                         continue;
                     }
 #pragma unroll 2
                     for (int j = 0; j < NC; j++) {
-                        const float4 sp = SP[j];
+                        const float* sx = reinterpret_cast<const float*>(SX + (j >> 1)) + (j & 1);
+                        const float4 sp = make_float4(sx[0], sx[2], reinterpret_cast<const float*>(SZ)[j], 0.f);
                         if (filt) {
                             const float r2a = fmaf(B4h, sp.x, Dh);
                             if (r2a < f_lo || r2a >= f_hi) continue;
@@ -1220,14 +1319,14 @@ __global__ void __launch_bounds__(FarShape<NG>::kWarps * 32, 2)
                             bad += out;
                             const float ww = wpq * sp.z;
                             const float wq = ww * w.qinv;  // fixed point: the largest pair weight -> 2^k units
-                            add_fixed(hqa, hqb, 2 * bi + cpy, fmaf(-wq, fr, wq), w.qfrac);
-                            add_fixed(hqa, hqb, 2 * bi + 2 + cpy, wq * fr, w.qfrac);
+                            add_fixed(hqa, hqb, (bi << lg) + cpy, fmaf(-wq, fr, wq), w.qfrac);
+                            add_fixed(hqa, hqb, ((bi + 1) << lg) + cpy, wq * fr, w.qfrac);
                         }
                     }
                 }
             }
             __syncwarp();
-            window_dots(a, w, hqa, hqb, key, wn.x, s0, segw, pass,
+            window_dots(a, w, hqa, hqb, key, wn.x, s0, segw, lg, pass,
                         w.dot64 || npass > 1 || wn.x < lk.n1, lane);
         }
         if (bad) atomicAdd(w.violations, bad);
@@ -1343,7 +1442,7 @@ WinLayout win_layout(const KeySpace& ks, int nx, int ntab, int ng) {
 
 template <int NG>
 size_t far_smem(const WinPlan& w, bool sph) {
-    const size_t pts = sph ? sizeof(float4) * (NG * (NG + 1) / 2) : sizeof(float4) * 2 * FarShape<NG>::NP;
+    const size_t pts = sph ? sizeof(float4) * sph_pairs(NG * (NG + 1) / 2) : sizeof(float4) * 2 * FarShape<NG>::NP;
     return FarShape<NG>::kWarps * (pts + 4 * sizeof(int) * w.Wkey);
 }
 
@@ -1362,7 +1461,7 @@ bool run_window(const CubatureArgs& a, const Lookup& lk, cudaStream_t s, long lo
     w.dot64 = a.win_dot64;
     w.logkeys = a.win_logkeys;
     {
-        int zmax = 0;  // index_log keeps the integer parts of z_k in 16 bits
+        int zmax = 0;  // log_pairs keeps the integer parts of z_k in 16 bits
         for (int k = 0; k < kLogN; k++) {
             int zi = 0;
             std::memcpy(&zi, &lk.kt[k].z, sizeof zi);
@@ -1382,6 +1481,7 @@ bool run_window(const CubatureArgs& a, const Lookup& lk, cudaStream_t s, long lo
         const double pairs = sph ? (double)NG * NG * NG * NG * NC : (double)NP * NP;
         const int k = std::min(21, 30 - (int)std::ceil(std::log2(pairs)));
         const double wwmax = 2.0 * std::pow(a.wmax, 6) * (1.0 + 1e-6);
+        w.nzero = -0.0f;
         w.qinv = (float)(std::ldexp(1.0, k) / wwmax);
         w.fbits = k;
         w.qfrac = (float)std::ldexp(1.0, k);
