@@ -961,7 +961,7 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
 // pairs' sin^2(theta/2) = x + y, SZ: their weights (0 for the one that evens out the count).
 // Products that an addition reads are written as fma(x, y, nz) with nz = -0 at run time: the same value,
 // and ptxas (13.0) joins a mul.rn.f32x2 and an addition into one fma.f32x2 although both are .rn.
-// What bounds it is issue: of its 93 instructions a pair the packed form takes about 30 away, and the
+// What bounds it is issue, which the packed instructions relieve; the
 // four shared atomics a pair come next (whole builds, scalar to packed: 32k-cell shell 57.3 -> 55.6 ms,
 // 65k 278 -> 270 ms, 16 mock surveys 242 -> 233 ms, a 2k-cell signal block 1.09 -> 1.07 ms).
 // NARROW: the histogram in 2^lg copies (else two).
