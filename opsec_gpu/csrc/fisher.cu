@@ -325,76 +325,86 @@ __global__ void __launch_bounds__(kMaxThreads) fisher_kernel(Src src, int nb, co
     }
 }
 
-// fixed-order reduction of the per-CTA partials into F (full), f, q
+// Fixed-order reduction of the per-CTA partials into F (full), f, q: one warp an output, lanes over the
+// partials, then a shuffle tree (a thread an output chained 304 loads and additions: 127 us for 20 bands).
 __global__ void fisher_reduce_kernel(int nb, int nblocks, const double* partial, double* out) {
-    const int nout = nb * (nb + 1) / 2 + 2 * nb;
-    for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < nout; o += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < nblocks; b++) s += partial[(size_t)b * nout + o];
-        int p, q;
-        out_pair(o, nb, &p, &q);
-        if (q < nb) {
-            out[p * nb + q] = s;
-            out[q * nb + p] = s;
-        } else if (q == nb) {
-            out[nb * nb + p] = s;       // f
-        } else {
-            out[nb * nb + nb + p] = s;  // q
-        }
+    const int nout = nb * (nb + 1) / 2 + 2 * nb, lane = threadIdx.x & 31;
+    const int o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (o >= nout) return;
+    double s = 0.0;
+#pragma unroll 5
+    for (int b = lane; b < nblocks; b += 32) s += partial[(size_t)b * nout + o];
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) s += __shfl_xor_sync(0xffffffffu, s, w);
+    if (lane) return;
+    int p, q;
+    out_pair(o, nb, &p, &q);
+    if (q < nb) {
+        out[p * nb + q] = s;
+        out[q * nb + p] = s;
+    } else if (q == nb) {
+        out[nb * nb + p] = s;  // f
+    } else {
+        out[nb * nb + nb + p] = s;  // q
     }
 }
 
 // ---------------------------------------------------------------- epilogue
 // Gauss-Jordan inverse with partial pivoting of an n x n row-major matrix in
 // shared memory (A destroyed, X = A^-1).  Returns false if a pivot vanishes.
+// One block; FP64 issue and barriers bound it.  A step is three phases: one warp finds the pivot (the
+// largest bits of |A|, ties to the lower row; a NaN's are larger still and fail the test) and its
+// reciprocal, one thread a column swaps and scales the two rows, all eliminate the columns still to be
+// read: those of A beyond c, all of X.  (With the pivot sought by one thread and every column eliminated
+// the epilogue of 20 bands took 57 us.)
 __device__ bool gj_inverse(int n, double* A, double* X, int* piv_row) {
+    __shared__ int bad;
+    __shared__ double inv;
+    if (threadIdx.x == 0) bad = 0;
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) X[e] = (e / n == e % n) ? 1.0 : 0.0;
     __syncthreads();
-    __shared__ int bad;
-    if (threadIdx.x == 0) bad = 0;
-    __syncthreads();
     for (int c = 0; c < n; c++) {
-        if (threadIdx.x == 0) {
-            int best = c;
-            double bv = fabs(A[c * n + c]);
-            for (int r = c + 1; r < n; r++)
-                if (fabs(A[r * n + c]) > bv) {
-                    bv = fabs(A[r * n + c]);
+        if (threadIdx.x < 32) {
+            unsigned long long bv = 0;
+            int best = n;
+            for (int r = c + threadIdx.x; r < n; r += 32) {
+                const unsigned long long v = (unsigned long long)__double_as_longlong(A[r * n + c]) & ~(1ull << 63);
+                if (best == n || v > bv) {
+                    bv = v;
                     best = r;
                 }
-            *piv_row = best;
-            if (!(bv > 0.0) || !isfinite(bv)) bad = 1;
+            }
+            const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(bv >> 32));
+            if ((unsigned)(bv >> 32) != hi) best = n;
+            const unsigned lo = __reduce_max_sync(0xffffffffu, best < n ? (unsigned)bv : 0u);
+            if ((unsigned)bv != lo) best = n;
+            best = __reduce_min_sync(0xffffffffu, best);
+            if (threadIdx.x == 0) {
+                const double p = A[best * n + c];
+                *piv_row = best;
+                if (!(fabs(p) > 0.0) || !isfinite(p))
+                    bad = 1;
+                else
+                    inv = 1.0 / p;
+            }
         }
         __syncthreads();
         if (bad) return false;
-        const int pr = *piv_row;
-        if (pr != c)
-            for (int e = threadIdx.x; e < n; e += blockDim.x) {
-                double t = A[c * n + e];
-                A[c * n + e] = A[pr * n + e];
-                A[pr * n + e] = t;
-                t = X[c * n + e];
-                X[c * n + e] = X[pr * n + e];
-                X[pr * n + e] = t;
-            }
-        __syncthreads();
-        const double inv = 1.0 / A[c * n + c];
-        __syncthreads();
-        for (int e = threadIdx.x; e < n; e += blockDim.x) {
-            A[c * n + e] *= inv;
-            X[c * n + e] *= inv;
+        const int pr = *piv_row, na = n - 1 - c, wd = na + n;  // columns c + 1 .. of A, then X
+        const double iv = inv;
+        for (int e = threadIdx.x; e <= wd; e += blockDim.x) {  // the last one is column c of A
+            double* M = e < na ? A + c + 1 + e : e < wd ? X + e - na : A + c;
+            const double t = M[pr * n];
+            M[pr * n] = M[c * n];
+            M[c * n] = t * iv;
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-            int r = e / n, col = e % n;
+        for (int e = threadIdx.x; e < n * wd; e += blockDim.x) {
+            const int r = e / wd, j = e % wd;
             if (r == c) continue;
-            double f = A[r * n + c];
-            if (col != c) A[r * n + col] -= f * A[c * n + col];
-            X[r * n + col] -= f * X[c * n + col];
+            double* M = j < na ? A + c + 1 + j : X + j - na;
+            M[r * n] -= A[r * n + c] * M[c * n];
         }
-        __syncthreads();
-        for (int r = threadIdx.x; r < n; r += blockDim.x)
-            if (r != c) A[r * n + c] = 0.0;
         __syncthreads();
     }
     return true;
@@ -555,7 +565,7 @@ static void run_fisher(const FisherArgs& a, const Src& src, double K, double ele
     k<<<a.nblocks, tl.threads, tl.smem, s>>>(src, nb, a.evals, a.y, a.prior, a.partial);
     OPSEC_CUDA(cudaGetLastError());
     if (g_clock) g_clock->end(s);
-    fisher_reduce_kernel<<<(nout + 255) / 256, 256, 0, s>>>(nb, a.nblocks, a.partial, a.out);
+    fisher_reduce_kernel<<<(nout + 3) / 4, 128, 0, s>>>(nb, a.nblocks, a.partial, a.out);
     OPSEC_CUDA(cudaGetLastError());
     *launches += 2;
 }
@@ -658,6 +668,6 @@ extern "C" int opsec_gpu_fisher_noalloc(int nmodes, int nbands, const float* cov
     fisher_kernel<PackedSource<float>><<<nblocks, tl.threads, tl.smem, s>>>(src, nb, evals, y, prior,
                                                                             g_partial_addr[dev]);
     if (cudaGetLastError() != cudaSuccess) return OPSEC_ERR_CUDA;  // the reduction would read stale partials
-    fisher_reduce_kernel<<<(nout + 255) / 256, 256, 0, s>>>(nb, nblocks, g_partial_addr[dev], out);
+    fisher_reduce_kernel<<<(nout + 3) / 4, 128, 0, s>>>(nb, nblocks, g_partial_addr[dev], out);
     return cudaGetLastError() == cudaSuccess ? OPSEC_OK : OPSEC_ERR_CUDA;
 }
