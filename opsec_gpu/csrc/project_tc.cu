@@ -154,9 +154,11 @@ struct Step1Params {
     int N, Npad, Mpad;
     int n_at;                 // a-tiles (Npad / BM)
     const int4* ckey;         // per padded cell: key pieces; .w = 0 for padding
-    const uint32_t* Qhl;      // square key table of this band, scaled by 2^sQ, FP16 hi | lo << 16
-    float out_scale;          // 2^-(sQ + sB): T in its natural units
-    float* Tf;                // [Mpad][Npad] T^T, FP32
+    const uint32_t* Qhl;      // square key tables of the batch's bands, scaled by 2^sQ, FP16 hi | lo << 16
+    const unsigned* maxB;     // max |B'|, and of each band's keys (float bits): T is written in its
+    const unsigned* maxQ;     // natural units, 2^-(sQ + sB) times the accumulators
+    float* Tf;                // [bands][Mpad][Npad] T^T, FP32
+    unsigned* maxT;           // out: max |T| of each band
     int chunk;                // K-slices per accumulator chunk
     int* err;
     long long wait_cycles;  // bound of every mbarrier wait
@@ -186,6 +188,7 @@ __device__ __forceinline__ int pair_key(const KeySpace& ks, int4 a, int4 b) {
     return a.x * ks.H + b.x + df;  // a.x = h_a nf, b.x = h_b nf
 }
 
+// grid (tiles, bands of the batch)
 // warps: 0 TMA, 1 MMA, 2-9 gather producers, 10-11 idle, 12-15 drain + epilogue (lane quarters 0-3)
 // N3A: 0 for the key gather, else the phi cells per arc of the arc-run tables (p.arcs), a
 // compile-time constant so that the producers' row and column splits are shifts
@@ -201,7 +204,8 @@ __global__ void __launch_bounds__(512, 1)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int jt = blockIdx.x / p.n_at, at = blockIdx.x % p.n_at;
-    const int a0 = at * BM, j0 = jt * BN;
+    const int a0 = at * BM, j0 = jt * BN, band = blockIdx.y;
+    const uint32_t* Qhl = p.Qhl + (size_t)band * p.ks.nsquare;
     const int nk = p.Npad / BK;
     const int chunk = p.chunk > 0 ? p.chunk : 1;
     const int nchunks = (nk + chunk - 1) / chunk;
@@ -274,6 +278,9 @@ __global__ void __launch_bounds__(512, 1)
         const int q = warp & 3;
         const int a = a0 + 32 * q + lane;
         const uint32_t lane_base = (uint32_t)(32 * q) << 16;
+        const float out_scale = 1.0f / (pow2_scale(__uint_as_float(p.maxQ[band])) * pow2_scale(__uint_as_float(*p.maxB)));
+        float* Tf = p.Tf + (size_t)band * p.Mpad * p.Npad;
+        float mx = 0.f;
         bool ok = true;
         for (int c = 0; c < nchunks && ok; c++) {
             const bool last = (c == nchunks - 1);
@@ -295,8 +302,11 @@ __global__ void __launch_bounds__(512, 1)
                     }
                     if (last) {
 #pragma unroll
-                        for (int t = 0; t < 32; t++)
-                            p.Tf[(size_t)(j0 + 128 * h + 32 * cc + t) * p.Npad + a] = v[t] * p.out_scale;
+                        for (int t = 0; t < 32; t++) {
+                            const float x = v[t] * out_scale;
+                            Tf[(size_t)(j0 + 128 * h + 32 * cc + t) * p.Npad + a] = x;
+                            mx = fmaxf(mx, fabsf(x));
+                        }
                     } else {
                         tmem_st32(tmem + rcol + (uint32_t)(32 * cc), v);
                     }
@@ -307,6 +317,8 @@ __global__ void __launch_bounds__(512, 1)
                 if (lane == 0) mbar_arrive(smem_u32(&bar_drained[h]));
             }
         }
+        mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
+        if (lane == 0) atomicMax(p.maxT + band, __float_as_uint(mx));
     } else if (N3A > 0 && warp < 10) {
         // eight producers expanding arc-run tables: each warp loads slice k+1's table into
         // registers while it expands slice k from its own shared buffer.
@@ -332,7 +344,7 @@ __global__ void __launch_bounds__(512, 1)
         uint32_t nxt[kPer];
         auto load = [&](int k) {
             const int kb = (k * BK) / n3;
-            const uint32_t* base = p.Qhl + ((size_t)ha0 * H + kb) * nf;
+            const uint32_t* base = Qhl + ((size_t)ha0 * H + kb) * nf;
 #pragma unroll
             for (int q = 0; q < kPer; q++) {
                 const int pk = packed[q];
@@ -389,8 +401,8 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
             for (int i = 0; i < BM / 8; i++) {
                 const int4 ka = rowkey[pw + 8 * i];
-                x0[i] = (ka.w && kb0.w) ? __ldg(p.Qhl + pair_key(p.ks, ka, kb0)) : 0u;
-                x1[i] = (ka.w && kb1.w) ? __ldg(p.Qhl + pair_key(p.ks, ka, kb1)) : 0u;
+                x0[i] = (ka.w && kb0.w) ? __ldg(Qhl + pair_key(p.ks, ka, kb0)) : 0u;
+                x1[i] = (ka.w && kb1.w) ? __ldg(Qhl + pair_key(p.ks, ka, kb1)) : 0u;
             }
         };
         if (nk > 0) gather(0);
@@ -424,14 +436,16 @@ __global__ void __launch_bounds__(512, 1)
 struct Step2Params {
     int M, Npad;
     const int2* tiles;  // (i-tile, j-tile) pairs touching the upper triangle
-    float sB;           // scale of B'
-    const unsigned* maxT;  // max |T| of this band (float bits); T was scaled by pow2_scale(maxT)
-    float* Dp;          // packed output of this band
+    int Mpad;
+    const unsigned* maxB;  // max |B'| (float bits), which gave the scale of B'
+    const unsigned* maxT;  // max |T| of each of the batch's bands; T was scaled by pow2_scale(maxT)
+    float* Dp;          // packed output of the batch's bands
     int chunk;          // K-slices per accumulator chunk
     int* err;
     long long wait_cycles;  // bound of every mbarrier wait
 };
 
+// grid (tiles, bands of the batch); T's maps hold the bands one below the other
 __global__ void __launch_bounds__(256, 1)
     step2_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
                  const __grid_constant__ CUtensorMap mTh, const __grid_constant__ CUtensorMap mTl, Step2Params p) {
@@ -443,7 +457,7 @@ __global__ void __launch_bounds__(256, 1)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int2 tile = p.tiles[blockIdx.x];
-    const int i0 = tile.x * BM, j0 = tile.y * BN;
+    const int i0 = tile.x * BM, j0 = tile.y * BN, band = blockIdx.y;
     const int nk = p.Npad / BK;
     const int chunk = p.chunk > 0 ? p.chunk : 1;
     const int nchunks = (nk + chunk - 1) / chunk;
@@ -478,8 +492,8 @@ __global__ void __launch_bounds__(256, 1)
                 mbar_arrive_tx(fb, STAGE_BYTES);
                 tma_load_2d(smem_u32(A_hi(s)), &mAh, fb, k * BK, i0);
                 tma_load_2d(smem_u32(A_lo(s)), &mAl, fb, k * BK, i0);
-                tma_load_2d(smem_u32(B_hi(s)), &mTh, fb, k * BK, j0);
-                tma_load_2d(smem_u32(B_lo(s)), &mTl, fb, k * BK, j0);
+                tma_load_2d(smem_u32(B_hi(s)), &mTh, fb, k * BK, band * p.Mpad + j0);
+                tma_load_2d(smem_u32(B_lo(s)), &mTl, fb, k * BK, band * p.Mpad + j0);
             }
         }
     } else if (warp == 1) {
@@ -501,14 +515,15 @@ __global__ void __launch_bounds__(256, 1)
         }
     } else if (warp >= 4) {
         const int q = warp & 3;
-        const float out_scale = 1.0f / (p.sB * pow2_scale(__uint_as_float(*p.maxT)));
+        const float out_scale = 1.0f / (pow2_scale(__uint_as_float(*p.maxB)) * pow2_scale(__uint_as_float(p.maxT[band])));
+        float* Dp = p.Dp + (size_t)band * ((size_t)p.M * (p.M + 1) / 2);
         const int i = i0 + 32 * q + lane;
         drain_loop(tmem, q, lane, nchunks, ChunkBars{smem_u32(&bar_chunk), smem_u32(&bar_drained), p.wait_cycles}, &abort_flag,
                    p.err, [&](int cc, const float* v) {
 #pragma unroll
                        for (int t = 0; t < 32; t++) {
                            const int j = j0 + 32 * cc + t;
-                           if (i <= j && j < p.M) p.Dp[(size_t)j * (j + 1) / 2 + i] = v[t] * out_scale;
+                           if (i <= j && j < p.M) Dp[(size_t)j * (j + 1) / 2 + i] = v[t] * out_scale;
                        }
                    });
     }
@@ -557,26 +572,38 @@ __global__ void cell_keys_kernel(KeySpace ks, int N, int Npad, const int* h, con
     }
 }
 
+// largest of the block's values (>= 0) to *out, one atomic a block (one a warp serialised: 105 us for the
+// 20 tables of a 1,575-cell survey)
+__device__ __forceinline__ void block_max(float m, unsigned int* out) {
+    __shared__ unsigned s_m;
+    if (threadIdx.x == 0) s_m = 0;
+    __syncthreads();
+    const unsigned v = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_m, v);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(out, s_m);
+}
+
 __global__ void absmax_f64_kernel(size_t n, const double* x, unsigned int* out) {
     float m = 0.f;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
         m = fmaxf(m, (float)fabs(x[e]));
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+    block_max(m, out);
 }
 
-__global__ void absmax_f32_kernel(int ntab, size_t n, const float* x, unsigned int* out) {
+// grid (blocks, tables)
+__global__ void absmax_f32_kernel(size_t n, const float* x, unsigned int* out) {
     const int t = blockIdx.y;
     float m = 0.f;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
         m = fmaxf(m, fabsf(x[(size_t)t * n + e]));
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out + t, __float_as_uint(m));
+    block_max(m, out + t);
 }
 
-// B'[i][a] (FP64, M x N) * scale -> hi/lo FP16 [Mpad][Npad], zero padded
-__global__ void split_modes_kernel(int M, int N, int Mpad, int Npad, const double* Bs, float scale, __half* Bh,
+// B'[i][a] (FP64, M x N) * pow2_scale(max|B'|) -> hi/lo FP16 [Mpad][Npad], zero padded
+__global__ void split_modes_kernel(int M, int N, int Mpad, int Npad, const double* Bs, const unsigned* maxB, __half* Bh,
                                    __half* Bl) {
+    const float scale = pow2_scale(__uint_as_float(*maxB));
     const size_t total = (size_t)Mpad * Npad;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const int i = (int)(e / Npad), a = (int)(e % Npad);
@@ -589,23 +616,31 @@ __global__ void split_modes_kernel(int M, int N, int Mpad, int Npad, const doubl
     }
 }
 
-// Q table of one band * 2^sQ -> packed FP16 (hi | lo << 16)
-__global__ void split_q_kernel(size_t n, const float* Q, float scale, uint32_t* out) {
+// Q tables of the batch's bands * 2^sQ -> packed FP16 (hi | lo << 16); grid (blocks, bands)
+__global__ void split_q_kernel(size_t n, const float* Q, const unsigned* maxQ, uint32_t* out) {
+    const float scale = pow2_scale(__uint_as_float(maxQ[blockIdx.y]));
+    const size_t o = n * blockIdx.y;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
         __half h, l;
-        split_half(Q[e] * scale, h, l);
-        out[e] = (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
+        split_half(Q[o + e] * scale, h, l);
+        out[o + e] = (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
     }
 }
 
-// T^T (FP32) * pow2_scale(max|T|) -> hi/lo FP16
-__global__ void split_t_kernel(size_t n, const float* Tf, const unsigned* maxT, __half* Th, __half* Tl) {
-    const float sc = pow2_scale(__uint_as_float(*maxT));
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        __half h, l;
-        split_half(Tf[e] * sc, h, l);
-        Th[e] = h;
-        Tl[e] = l;
+// T^T (FP32, n4 groups of four a band) * pow2_scale(max|T|) -> hi/lo FP16; grid (blocks, bands)
+__global__ void split_t_kernel(size_t n4, const float4* Tf, const unsigned* maxT, uint2* Th, uint2* Tl) {
+    const float sc = pow2_scale(__uint_as_float(maxT[blockIdx.y]));
+    const size_t o = n4 * blockIdx.y;
+    auto two = [](__half a, __half b) { return (unsigned)__half_as_ushort(a) | ((unsigned)__half_as_ushort(b) << 16); };
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n4; e += (size_t)gridDim.x * blockDim.x) {
+        const float4 t = Tf[o + e];
+        __half h[4], l[4];
+        split_half(t.x * sc, h[0], l[0]);
+        split_half(t.y * sc, h[1], l[1]);
+        split_half(t.z * sc, h[2], l[2]);
+        split_half(t.w * sc, h[3], l[3]);
+        Th[o + e] = make_uint2(two(h[0], h[1]), two(h[2], h[3]));
+        Tl[o + e] = make_uint2(two(l[0], l[1]), two(l[2], l[3]));
     }
 }
 
@@ -625,7 +660,7 @@ CUtensorMap make_map(const __half* base, int rows, int cols, int box_rows) {
 }
 
 struct Layout {
-    int Npad, Mpad;
+    int Npad, Mpad, batch;
     size_t bh, bl, th, tl, tf, qhl, ckey, maxes, tiles, err, total;
 };
 
@@ -634,6 +669,18 @@ Layout layout_of(const ProjectArgs& a) {
     L.Npad = (a.ncells + BM - 1) / BM * BM;
     L.Mpad = (a.nmodes + BN - 1) / BN * BN;
     const size_t half_mat = (size_t)L.Mpad * L.Npad * sizeof(__half);
+    // Bands of one launch: a band is few tiles (step 1 26, step 2 5 at 1,575 cells and 588 modes, 101 and
+    // 65 us each whatever the number), so bands share launches until step 2, the smaller grid, has kWaves
+    // waves of one-CTA SMs, as far as kBatchBytes of T and tables go (a 1,575-cell comma over 20 bands
+    // 4.22 ms one at a time, 0.77 ms so; larger batches would fill no more SMs and leave L2 sooner).
+    constexpr size_t kBatchBytes = size_t(1) << 29;
+    constexpr int kSMs = 152, kWaves = 4;
+    const int tiles2 = std::max(1, (L.Mpad / BM) * (L.Mpad / BN) / 2);
+    const size_t per = 4 * half_mat + sizeof(uint32_t) * (size_t)a.ks.nsquare;
+    L.batch = (int)std::min<size_t>({(size_t)a.nbands, (size_t)((kWaves * kSMs + tiles2 - 1) / tiles2),
+                                     std::max<size_t>(1, kBatchBytes / per)});
+    const int launches = (a.nbands + L.batch - 1) / L.batch;
+    L.batch = (a.nbands + launches - 1) / launches;
     size_t o = 0;
     auto take = [&](size_t bytes) {
         size_t at = o;
@@ -642,10 +689,10 @@ Layout layout_of(const ProjectArgs& a) {
     };
     L.bh = take(half_mat);
     L.bl = take(half_mat);
-    L.th = take(half_mat);
-    L.tl = take(half_mat);
-    L.tf = take(2 * half_mat);
-    L.qhl = take(sizeof(uint32_t) * (size_t)a.ks.nsquare);
+    L.th = take(L.batch * half_mat);
+    L.tl = take(L.batch * half_mat);
+    L.tf = take(L.batch * 2 * half_mat);
+    L.qhl = take(L.batch * sizeof(uint32_t) * (size_t)a.ks.nsquare);
     L.ckey = take(sizeof(int4) * L.Npad);
     L.maxes = take(sizeof(unsigned) * (1 + 2 * a.nbands));
     const int nti = L.Mpad / BM, ntj = L.Mpad / BN;
@@ -688,24 +735,14 @@ void launch_project_tc(const ProjectArgs& a, cudaStream_t s, long long* launches
 
     OPSEC_CUDA(cudaMemsetAsync(maxes, 0, sizeof(unsigned) * (1 + 2 * nb), s));
     OPSEC_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+    auto blocks = [](size_t n, size_t per, size_t most) { return (unsigned)std::max<size_t>(1, std::min((n + per - 1) / per, most)); };
+    const size_t nsq = (size_t)a.ks.nsquare;
     cell_keys_kernel<<<(L.Npad + 255) / 256, 256, 0, s>>>(a.ks, N, L.Npad, a.cell_h, a.cell_f, a.cell_g, ckey);
-    absmax_f64_kernel<<<1024, 256, 0, s>>>((size_t)M * N, a.Bs, maxes);
-    absmax_f32_kernel<<<dim3(1024, nb), 256, 0, s>>>(nb, (size_t)a.ks.nsquare, a.Qsq + a.ks.nsquare, maxes + 1);
+    absmax_f64_kernel<<<blocks((size_t)M * N, 2048, 1024), 256, 0, s>>>((size_t)M * N, a.Bs, maxes);
+    absmax_f32_kernel<<<dim3(blocks(nsq, 2048, 256), nb), 256, 0, s>>>(nsq, a.Qsq + nsq, maxes + 1);
+    split_modes_kernel<<<2048, 256, 0, s>>>(M, N, L.Mpad, L.Npad, a.Bs, maxes, Bh, Bl);
     OPSEC_CUDA(cudaGetLastError());
-    *launches += 3;
-    std::vector<unsigned> hm(1 + nb);
-    OPSEC_CUDA(cudaMemcpyAsync(hm.data(), maxes, sizeof(unsigned) * (1 + nb), cudaMemcpyDeviceToHost, s));
-    OPSEC_CUDA(cudaStreamSynchronize(s));
-    auto asf = [](unsigned u) {
-        float f;
-        std::memcpy(&f, &u, sizeof f);
-        return f;
-    };
-    const float sB = pow2_scale(asf(hm[0]));
-
-    split_modes_kernel<<<2048, 256, 0, s>>>(M, N, L.Mpad, L.Npad, a.Bs, sB, Bh, Bl);
-    OPSEC_CUDA(cudaGetLastError());
-    ++*launches;
+    *launches += 4;
 
     // tiles (i-tile of 128, j-tile of 256) that hold an element with i <= j
     std::vector<int2> tl;
@@ -716,7 +753,7 @@ void launch_project_tc(const ProjectArgs& a, cudaStream_t s, long long* launches
 
     const CUtensorMap mBh256 = make_map(Bh, L.Mpad, L.Npad, BN), mBl256 = make_map(Bl, L.Mpad, L.Npad, BN);
     const CUtensorMap mBh128 = make_map(Bh, L.Mpad, L.Npad, BM), mBl128 = make_map(Bl, L.Mpad, L.Npad, BM);
-    const CUtensorMap mTh256 = make_map(Th, L.Mpad, L.Npad, BN), mTl256 = make_map(Tl, L.Mpad, L.Npad, BN);
+    const CUtensorMap mTh256 = make_map(Th, L.batch * L.Mpad, L.Npad, BN), mTl256 = make_map(Tl, L.batch * L.Mpad, L.Npad, BN);
 
     const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + sizeof(uint32_t) * 8 * 2 * kArcTab;
     OPSEC_CUDA(cudaFuncSetAttribute(step1_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -727,8 +764,8 @@ void launch_project_tc(const ProjectArgs& a, cudaStream_t s, long long* launches
 
     const int n_at = L.Npad / BM, n_jt = L.Mpad / BN;
     const size_t nT = (size_t)L.Mpad * L.Npad;
-    for (int p = 0; p < nb; p++) {
-        const float sQ = pow2_scale(asf(hm[1 + p]));
+    for (int p = 0; p < nb; p += L.batch) {
+        const int g = std::min(L.batch, nb - p);
         Step1Params p1;
         p1.ks = a.ks;
         p1.N = N;
@@ -736,17 +773,19 @@ void launch_project_tc(const ProjectArgs& a, cudaStream_t s, long long* launches
         p1.Mpad = L.Mpad;
         p1.n_at = n_at;
         p1.ckey = ckey;
-        split_q_kernel<<<2048, 256, 0, s>>>((size_t)a.ks.nsquare, a.Qsq + (size_t)(1 + p) * a.ks.nsquare, sQ, Qhl);
+        split_q_kernel<<<dim3(blocks(nsq, 1024, 2048), g), 256, 0, s>>>(nsq, a.Qsq + (size_t)(1 + p) * nsq, maxes + 1 + p, Qhl);
         OPSEC_CUDA(cudaGetLastError());
         p1.Qhl = Qhl;
-        p1.out_scale = 1.0f / (sQ * sB);
+        p1.maxB = maxes;
+        p1.maxQ = maxes + 1 + p;
         p1.Tf = Tf;
+        p1.maxT = maxT + p;
         p1.chunk = a.chunk;
         p1.err = err;
         p1.wait_cycles = a.wait_cycles;
         p1.arcs = a.arc_run;
-        if (g_clock) g_clock->begin("project_step1", s, 2.0 * N * (double)N * M);
-        const unsigned g1 = (unsigned)(n_at * n_jt);
+        if (g_clock) g_clock->begin("project_step1", s, 2.0 * N * (double)N * M * g);
+        const dim3 g1(n_at * n_jt, g);
         if (p1.arcs == 16)
             step1_kernel<16><<<g1, 512, smem, s>>>(mBh256, mBl256, p1);
         else if (p1.arcs == 32)
@@ -757,24 +796,25 @@ void launch_project_tc(const ProjectArgs& a, cudaStream_t s, long long* launches
             step1_kernel<0><<<g1, 512, smem, s>>>(mBh256, mBl256, p1);
         OPSEC_CUDA(cudaGetLastError());
         if (g_clock) g_clock->end(s);
-        absmax_f32_kernel<<<dim3(2048, 1), 256, 0, s>>>(1, nT, Tf, maxT + p);
-        split_t_kernel<<<4096, 256, 0, s>>>(nT, Tf, maxT + p, Th, Tl);
+        split_t_kernel<<<dim3(blocks(nT / 4, 1024, 2048), g), 256, 0, s>>>(nT / 4, reinterpret_cast<const float4*>(Tf), maxT + p,
+                                                                          reinterpret_cast<uint2*>(Th), reinterpret_cast<uint2*>(Tl));
         OPSEC_CUDA(cudaGetLastError());
         Step2Params p2;
         p2.M = M;
         p2.Npad = L.Npad;
+        p2.Mpad = L.Mpad;
         p2.tiles = tiles;
-        p2.sB = sB;
+        p2.maxB = maxes;
         p2.maxT = maxT + p;
         p2.chunk = a.chunk;
         p2.Dp = a.Dp + (size_t)p * ((size_t)M * (M + 1) / 2);
         p2.err = err;
         p2.wait_cycles = a.wait_cycles;
-        if (g_clock) g_clock->begin("project_step2", s, (double)N * M * (double)(M + 1));
-        step2_kernel<<<(unsigned)tl.size(), 256, smem, s>>>(mBh128, mBl128, mTh256, mTl256, p2);
+        if (g_clock) g_clock->begin("project_step2", s, (double)N * M * (double)(M + 1) * g);
+        step2_kernel<<<dim3((unsigned)tl.size(), g), 256, smem, s>>>(mBh128, mBl128, mTh256, mTl256, p2);
         OPSEC_CUDA(cudaGetLastError());
         if (g_clock) g_clock->end(s);
-        *launches += 5;
+        *launches += 4;
     }
     int herr = 0;
     OPSEC_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s));
