@@ -29,6 +29,7 @@
 
 #include "df64.h"
 #include "engine.h"
+#include "packed.h"
 
 namespace opsec {
 namespace {
@@ -766,14 +767,16 @@ __device__ __forceinline__ df df_mac(df acc, df x, df y) {
 }
 
 // T of every group of kR reflectors: one warp each.  Reflectors past the last (n - 3) become zero
-// rows.  V row c: zero from its group's first row + 1 to c (tridiag.cu), then v.
-__global__ void __launch_bounds__(128) compact_kernel(int n, int nblk, float2* __restrict__ Vall,
+// rows (the last group of a block may end at row n).  V row c: zero from its group's first row to c and
+// past n - 1 (tridiag.cu), then v.
+__global__ void __launch_bounds__(128) compact_kernel(int n, int nblk, float4* __restrict__ Vall,
                                                       const double* __restrict__ tau, float2* __restrict__ T) {
     const int ngrp = (n - 2 + kR - 1) / kR, lane = threadIdx.x & 31;
     const int w = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (w >= ngrp * nblk) return;
     const int b = w / ngrp, c0 = (w % ngrp) * kR;
-    float2* V = Vall + (size_t)b * n * n;
+    const int vs = (n + 1) / 2;
+    float4* V = Vall + (size_t)b * ((n + 3) & ~3) * vs;
     df tv[kR], g[kR][kR];
 #pragma unroll
     for (int q = 0; q < kR; q++) {
@@ -781,21 +784,22 @@ __global__ void __launch_bounds__(128) compact_kernel(int n, int nblk, float2* _
 #pragma unroll
         for (int p = 0; p < kR; p++) g[p][q] = df{0.f, 0.f};
     }
-    for (int i = c0 + 1 + lane; i < n; i += 32) {
-        df v[kR];
+    for (int i = c0 / 2 + lane; i < vs; i += 32) {
+        df v[kR][2];
 #pragma unroll
         for (int q = 0; q < kR; q++) {
-            if (c0 + q <= n - 3) {
-                v[q] = df_unpack(V[(size_t)(c0 + q) * n + i]);
-            } else {
-                v[q] = df{0.f, 0.f};
-                if (c0 + q < n) V[(size_t)(c0 + q) * n + i] = make_float2(0.f, 0.f);
-            }
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c0 + q <= n - 3)
+                x = V[(size_t)(c0 + q) * vs + i];
+            else
+                V[(size_t)(c0 + q) * vs + i] = x;
+            v[q][0] = df{x.x, x.z};
+            v[q][1] = df{x.y, x.w};
         }
 #pragma unroll
         for (int q = 1; q < kR; q++)
 #pragma unroll
-            for (int p = 0; p < q; p++) g[p][q] = df_mac(g[p][q], v[p], v[q]);
+            for (int p = 0; p < q; p++) g[p][q] = df_mac(df_mac(g[p][q], v[p][0], v[q][0]), v[p][1], v[q][1]);
     }
 #pragma unroll
     for (int q = 1; q < kR; q++)
@@ -833,45 +837,48 @@ __global__ void __launch_bounds__(128) compact_kernel(int n, int nblk, float2* _
 // block are neighbours, so that its reflectors stay in L2.  Writes candidate c in FP64: as column
 // n-1-c of the block (ascending order, column-major), or, with rows set, as row c of out while c <
 // rows.
-constexpr int kPipe = 8;
-constexpr int kRing = kPipe * kR * 32;  // pairs per warp
+constexpr int kPipe = 4;
+constexpr int kRing = kPipe * kR * 32;  // 16-byte pairs per warp
 template <int NV>
-__global__ void __launch_bounds__(128) backtransform_kernel(VecArgs a, const float2* __restrict__ Vall,
+__global__ void __launch_bounds__(128) backtransform_kernel(VecArgs a, const float4* __restrict__ Vall,
                                                             const float2* __restrict__ Tall, double* __restrict__ out,
                                                             int rows) {
-    extern __shared__ float2 zsm[];
-    const int b = blockIdx.y, n = a.n, kc = a.kc[b];
+    extern __shared__ float4 zsm[];
+    const int b = blockIdx.y, n = a.n, kc = a.kc[b], vs = (n + 1) / 2;
     const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c0 = (blockIdx.x * W + warp) * NV;
     if (c0 >= kc) return;
-    float2* ring = zsm + (size_t)warp * (kRing + NV * n) + lane;  // [kPipe][kR][32], this lane's slots
-    float2* z = zsm + (size_t)warp * (kRing + NV * n) + kRing;    // [NV][n]
+    float4* ring = zsm + (size_t)warp * (kRing + NV * vs) + lane;  // [kPipe][kR][32], this lane's slots
+    float4* z = zsm + (size_t)warp * (kRing + NV * vs) + kRing;    // [NV][vs], (hi, hi, lo, lo) of two rows
     const size_t K = (size_t)a.ktot;
     const int nv = min(NV, kc - c0);
-    for (int i = lane; i < n; i += 32) {
-        const double* src = a.Z + (size_t)i * K + a.koff[b] + c0;
+    for (int i = lane; i < vs; i += 32) {
+        const double* src = a.Z + (size_t)2 * i * K + a.koff[b] + c0;
 #pragma unroll
-        for (int v = 0; v < NV; v++) z[v * n + i] = df_pack(df_from(v < nv ? src[v] : 0.0));
+        for (int v = 0; v < NV; v++) {
+            const df x = df_from(v < nv ? src[v] : 0.0), y = df_from(v < nv && 2 * i + 1 < n ? src[K + v] : 0.0);
+            z[v * vs + i] = make_float4(x.h, y.h, x.l, y.l);
+        }
     }
     __syncwarp();
-    const float2* V = Vall + (size_t)b * n * n;
+    const float4* V = Vall + (size_t)b * ((n + 3) & ~3) * vs;
     const int ngrp = (n - 2 + kR - 1) / kR;
     constexpr int NS = NV * kR;  // sums a group: (vector, reflector)
-    // the stream: groups downwards, each twice, rows r0 + 1 + lane, + 32, ...
-    int sg = ngrp - 1, sp = 0, si = 0, slot = 0;  // next step to issue: group, pass, row offset
+    // the stream: groups downwards, each twice, row pairs r0 / 2 + lane, + 32, ...
+    int sg = ngrp - 1, sp = 0, si = 0, slot = 0;  // next step to issue: group, pass, offset
     auto issue = [&]() {
         if (sg >= 0) {
-            const int i = sg * kR + 1 + si + lane;
-            if (i < n) {
-                const float2* src = V + (size_t)(sg * kR) * n + i;
+            const int i = sg * (kR / 2) + si + lane;
+            if (i < vs) {
+                const float4* src = V + (size_t)(sg * kR) * vs + i;
 #pragma unroll
                 for (int q = 0; q < kR; q++) {
                     const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + (slot * kR + q) * 32);
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src + (size_t)q * n) : "memory");
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + (size_t)q * vs) : "memory");
                 }
             }
             si += 32;
-            if (sg * kR + 1 + si >= n) {
+            if (sg * (kR / 2) + si >= vs) {
                 si = 0;
                 sg -= sp;
                 sp ^= 1;
@@ -882,30 +889,44 @@ __global__ void __launch_bounds__(128) backtransform_kernel(VecArgs a, const flo
     };
     for (int k = 0; k < kPipe - 1; k++) issue();
     int rd = 0;
-    auto step = [&](df (&v)[kR]) {  // the next step's reflector entries
+    auto load = [](const float4* p) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p);
+        return df2{t.x, t.y};
+    };
+    auto step = [&](df2 (&v)[kR]) {  // the next step's reflector entries
         asm volatile("cp.async.wait_group %0;" ::"n"(kPipe - 2) : "memory");
 #pragma unroll
-        for (int q = 0; q < kR; q++) v[q] = df_unpack(ring[(rd * kR + q) * 32]);
+        for (int q = 0; q < kR; q++) v[q] = load(ring + (rd * kR + q) * 32);
         rd = rd + 1 == kPipe ? 0 : rd + 1;
         issue();
     };
+    const f2 minus = pk(-1.f, -1.f);
     for (int g = ngrp - 1; g >= 0; g--) {
-        const int r0 = g * kR;
-        df acc[NS];
+        const int r0 = g * (kR / 2);
+        df2 ac2[NS];
 #pragma unroll
-        for (int k = 0; k < NS; k++) acc[k] = df{0.f, 0.f};
-        for (int i0 = r0 + 1; i0 < n; i0 += 32) {
+        for (int k = 0; k < NS; k++) ac2[k] = df2{0, 0};
+        for (int i0 = r0; i0 < vs; i0 += 32) {
             const int i = i0 + lane;
-            df v[kR];
+            df2 v[kR];
             step(v);
-            if (i < n) {
+            if (i < vs) {
 #pragma unroll
                 for (int u = 0; u < NV; u++) {
-                    const df x = df_unpack(z[u * n + i]);
+                    const df2 x = load(z + u * vs + i);
+                    const f2 nx = mul2(x.h, minus);
 #pragma unroll
-                    for (int q = 0; q < kR; q++) acc[u * kR + q] = df_mac(acc[u * kR + q], v[q], x);
+                    for (int q = 0; q < kR; q++) ac2[u * kR + q] = df2_mac(ac2[u * kR + q], v[q], x.h, x.l, nx);
                 }
             }
+        }
+        df acc[NS];
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+            df x, y;
+            upk(ac2[k].h, &x.h, &y.h);
+            upk(ac2[k].l, &x.l, &y.l);
+            acc[k] = df_add(x, y);
         }
         // sum over the lanes, halving the sums held: lane l ends with sum l / (32 / NS)
         int o = 16;
@@ -930,23 +951,26 @@ __global__ void __launch_bounds__(128) backtransform_kernel(VecArgs a, const flo
             const df d = shfl_df(acc[0], (u0 * kR + q) * kL);
             if (q >= p0) f = df_fma(f, df_unpack(__ldg(Tg + q * (q + 1) / 2 + p0)), d);
         }
-        df fs[NS];
+        f2 fh[NS], fl[NS], nfh[NS];  // -f, and its high part's negative
 #pragma unroll
         for (int k = 0; k < NS; k++) {
             const df t = shfl_df(f, k * kL);
-            fs[k] = df{-t.h, -t.l};
+            fh[k] = pk(-t.h, -t.h);
+            fl[k] = pk(-t.l, -t.l);
+            nfh[k] = pk(t.h, t.h);
         }
-        for (int i0 = r0 + 1; i0 < n; i0 += 32) {
+        for (int i0 = r0; i0 < vs; i0 += 32) {
             const int i = i0 + lane;
-            df v[kR];
+            df2 v[kR];
             step(v);
-            if (i < n) {
+            if (i < vs) {
 #pragma unroll
                 for (int u = 0; u < NV; u++) {
-                    df x = df_unpack(z[u * n + i]);
+                    df2 x = load(z + u * vs + i);
 #pragma unroll
-                    for (int q = 0; q < kR; q++) x = df_mac(x, v[q], fs[u * kR + q]);
-                    z[u * n + i] = df_pack(fast_two_sum(x.h, x.l));
+                    for (int q = 0; q < kR; q++) x = df2_mac(x, v[q], fh[u * kR + q], fl[u * kR + q], nfh[u * kR + q]);
+                    const f2 h = add2(x.h, x.l);
+                    *reinterpret_cast<ulonglong2*>(z + u * vs + i) = make_ulonglong2(h, sub2(x.l, sub2(h, x.h)));
                 }
             }
         }
@@ -956,7 +980,11 @@ __global__ void __launch_bounds__(128) backtransform_kernel(VecArgs a, const flo
     for (int u = 0; u < nv; u++) {
         if (rows > 0 && c0 + u >= rows) break;
         double* o = rows > 0 ? out + (size_t)(c0 + u) * n : out + (size_t)b * n * n + (size_t)(n - 1 - (c0 + u)) * n;
-        for (int i = lane; i < n; i += 32) o[i] = df_to(df_unpack(z[u * n + i]));
+        for (int i = lane; i < vs; i += 32) {
+            const float4 x = z[u * vs + i];
+            o[2 * i] = (double)x.x + (double)x.z;
+            if (2 * i + 1 < n) o[2 * i + 1] = (double)x.y + (double)x.w;
+        }
     }
 }
 
@@ -985,10 +1013,10 @@ __global__ void polish_kernel(int k, int m, const double* __restrict__ G, const 
 template <int NV>
 void launch_back(const VecArgs& a, const BlockEigVectors& p, int warps, cudaStream_t s) {
     auto k = backtransform_kernel<NV>;
-    const size_t per = sizeof(float2) * (kRing + (size_t)NV * p.n);
+    const size_t per = sizeof(float4) * (kRing + (size_t)NV * ((p.n + 1) / 2));
     OPSEC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem((const void*)k)));
     k<<<dim3((p.kmax + warps * NV - 1) / (warps * NV), p.nblk), 32 * warps, per * warps, s>>>(
-        a, reinterpret_cast<const float2*>(p.V), reinterpret_cast<const float2*>(p.T), p.out, p.rows);
+        a, reinterpret_cast<const float4*>(p.V), reinterpret_cast<const float2*>(p.T), p.out, p.rows);
     OPSEC_CUDA(cudaGetLastError());
 }
 
@@ -1001,6 +1029,8 @@ void launch_polish_coefficients(int k, int m, const double* G, const double* H, 
     OPSEC_CUDA(cudaGetLastError());
     ++*launches;
 }
+
+size_t blockeig_reflector_doubles(int n) { return (size_t)((n + 3) & ~3) * ((n + 1) / 2) * 2; }  // whole groups of kR rows
 
 size_t blockeig_rows_doubles(int n, int nblk) { return (size_t)10 * ((n + kGrp64 - 1) / kGrp64 * kGrp64) * nblk; }
 
@@ -1043,7 +1073,7 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     OPSEC_CUDA(cudaGetLastError());
     if (g_clock) g_clock->begin("blockeig_back", s, 2.0 * p.n * (double)p.n * p.ktot);
     const int groups = (p.n - 2 + kR - 1) / kR * p.nblk;
-    compact_kernel<<<(groups + 3) / 4, 128, 0, s>>>(p.n, p.nblk, reinterpret_cast<float2*>(p.V), p.tau,
+    compact_kernel<<<(groups + 3) / 4, 128, 0, s>>>(p.n, p.nblk, reinterpret_cast<float4*>(p.V), p.tau,
                                                     reinterpret_cast<float2*>(p.T));
     OPSEC_CUDA(cudaGetLastError());
     // Vectors per warp.  One while the warps do not fill the chip four times over (10 blocks of 555^2,
@@ -1052,8 +1082,8 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     // reading the reflectors half as often counts (34 of 512^2, 4,351 vectors: 1.10 ms, two 1.43, one
     // 1.42; 66 of 256^2: two 0.35, four 0.41).
     const int cap = max_dynamic_smem((const void*)backtransform_kernel<4>);
-    const size_t vec = sizeof(float2) * (size_t)p.n;
-    auto warps_of = [&](int nv) { return (int)std::min<size_t>(4, (size_t)cap / (vec * nv + sizeof(float2) * kRing)); };
+    const size_t vec = sizeof(float4) * (size_t)((p.n + 1) / 2);
+    auto warps_of = [&](int nv) { return (int)std::min<size_t>(4, (size_t)cap / (vec * nv + sizeof(float4) * kRing)); };
     // On one dense matrix the reflectors leave L2 behind: two from 2,400 rows on (2730^2, 890 vectors: 14.3
     // ms, one 17.5, four 22.4; 1728^2, 530 vectors: one 3.6, two 5.8).
     int nv = p.n >= 2400 ? 2 : p.ktot < 16 * nsm ? 1 : p.ktot >= 24 * nsm && p.n > 384 && p.n <= 576 ? 4 : 2;

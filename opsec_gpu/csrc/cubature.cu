@@ -38,6 +38,7 @@
 #include <string>
 
 #include "engine.h"
+#include "packed.h"
 
 namespace opsec {
 namespace {
@@ -952,46 +953,11 @@ __device__ __forceinline__ void window_dots(const CubatureArgs& a, const WinPlan
 }
 
 
-// Packed FP32: two values an instruction, each rounded as the scalar instruction rounds.
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pk(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk(f2 x, float* a, float* b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(x)); }
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 add2_rd(f2 a, f2 b) {
-    f2 r;
-    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
-    f2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // The spherical kernel's log-section loop over a node pair's canonical phi-node pairs, two at a time
 // in packed FP32: the operations of the scalar statements beside them, with the same roundings
 // (signs are moved where the packed instructions have no negation).  SX: (x, x', y, y') of two
 // pairs' sin^2(theta/2) = x + y, SZ: their weights (0 for the one that evens out the count).
-// Products that an addition reads are written as fma(x, y, nz) with nz = -0 at run time: the same value,
-// and ptxas (13.0) joins a mul.rn.f32x2 and an addition into one fma.f32x2 although both are .rn.
+// Products that only additions read are written as fma2(x, y, nz), nz = -0 at run time (packed.h).
 // What bounds it is issue, which the packed instructions relieve; the
 // four shared atomics a pair come next (whole builds, scalar to packed: 32k-cell shell 57.3 -> 55.6 ms,
 // 65k 278 -> 270 ms, 16 mock surveys 242 -> 233 ms, a 2k-cell signal block 1.09 -> 1.07 ms).

@@ -70,7 +70,7 @@ bool small_survey(int npar, long long cells) { return cells < 1024 || (npar == 1
 // kernels failed; the caller then solves the rebuilt blocks with the library.
 bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int M, std::vector<int>& kc) {
     const size_t nn = (size_t)n * n;
-    c->bev_V.alloc((size_t)nblk * nn);
+    c->bev_V.alloc(nblk * blockeig_reflector_doubles(n));
     c->bev_T.alloc((size_t)nblk * (3 * n + 1));
     double* tau = c->bev_T.p;
     double* dg = tau + (size_t)nblk * n;
@@ -188,7 +188,7 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
 // c->evals (descending) and c->modes.  False when a check in the kernels failed.
 bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
     const size_t nn = (size_t)n * n;
-    c->bev_V.alloc(nn);
+    c->bev_V.alloc(blockeig_reflector_doubles(n));
     c->bev_T.alloc((size_t)3 * n + 1);
     double* tau = c->bev_T.p;
     double* dg = tau + n;

@@ -206,10 +206,12 @@ void launch_assemble_modes(int H, int Nphi, int Nmu, int npar, int nmodes, const
 // written as columns n-1-c of out (ascending order, as LAPACK's syevd).
 bool blockeig_supported(int n);
 // Householder tridiagonalisation (tridiag.cu) of nblk blocks of order n >= 3 (FP64, column-major,
-// lower triangle read): T = (dg, eg), the reflectors V[block][c][i] as (hi, lo) float pairs
-// (v[c+1] = 1) and tau, each [block][n].  work: tridiag_work_bytes() bytes.  *err (zeroed by the
+// lower triangle read): T = (dg, eg), the reflectors V[block][c][i/2] as (hi, hi, lo, lo) floats of
+// entries i and i + 1 (v[c+1] = 1) and tau, each [block][n].  work: tridiag_work_bytes() bytes.  *err (zeroed by the
 // caller) is set when a wait between CTAs ran out.  chip: one block on the whole GPU instead of a
 // cluster (a cooperative launch; tridiag_chip_supported).
+// doubles of one block's reflectors (the small surveys' [n][n] pairs fit as well)
+size_t blockeig_reflector_doubles(int n);
 size_t tridiag_work_bytes(int n, int nblk);
 bool tridiag_chip_supported(int n);
 void launch_tridiag(int n, int nblk, bool chip, const double* A, double* V, double* tau, double* dg, double* eg, void* work,
@@ -228,7 +230,7 @@ struct BlockEigVectors {
     double *Z, *X, *Y;    // [n][ktot] each: the vectors, and scratch
     int* K;               // scratch, 2 ceil(n/2) ktot
     int* status;          // [nblk], zeroed by the caller
-    double* V;            // [nblk][n][n] reflectors, (hi, lo) float pairs
+    double* V;            // [nblk] reflectors of launch_tridiag
     const double* tau;    // [nblk][n]
     double* T;            // scratch, blockeig_compact_doubles()
     double* R;            // scratch, blockeig_rows_doubles()

@@ -32,6 +32,7 @@
 
 #include "df64.h"
 #include "engine.h"
+#include "packed.h"
 
 namespace cg = cooperative_groups;
 
@@ -55,41 +56,6 @@ __device__ __forceinline__ void put(float* x, int i, df v) {
     x[at(i) + 2] = v.l;
 }
 
-using f2 = unsigned long long;  // two packed floats
-__device__ __forceinline__ f2 pk(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk(f2 x, float* a, float* b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(x)); }
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
-    f2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-struct df2 {  // two double-FP32 values
-    f2 h, l;
-};
-// error of the rounded difference s = a - q
-__device__ __forceinline__ f2 sub2_err(f2 a, f2 q, f2 s) {
-    const f2 bb = sub2(s, a);
-    return sub2(sub2(a, sub2(s, bb)), add2(q, bb));
-}
 // the factor of a rank-1 update that belongs to a row, twice each: x.h, -x.h, -x.l
 struct RowFactor {
     f2 h, nh, nl;
@@ -108,22 +74,14 @@ __device__ __forceinline__ df2 df2_rank2(df2 a, RowFactor x, f2 yh, f2 yl, RowFa
     const f2 r = add2(s2, l);
     return df2{r, sub2(l, sub2(r, s2))};
 }
-// acc + x y with ny = -y.h; the low parts are only added up (12 operations)
-__device__ __forceinline__ df2 df2_mac(df2 acc, df2 x, f2 yh, f2 yl, f2 ny) {
-    const f2 nq = mul2(x.h, ny);
-    f2 e = fma2(x.h, yl, fma2(x.h, yh, nq));
-    e = fma2(x.l, yh, e);
-    const f2 s = sub2(acc.h, nq);
-    return df2{s, add2(add2(acc.l, e), sub2_err(acc.h, nq, s))};
-}
-
 struct TridiagArgs {
     int n, ld;         // order, row stride of D (a multiple of kChunk)
     int C;             // CTAs per block
     int kres;          // a warp's rows k >= kres live in shared memory
     int nres;          // resident rows per CTA
     float* D;          // [block][n][2 ld] the matrix in double-FP32, both triangles, zero past column n
-    float2* V;         // [block][n][n] reflector c in row c (v[c+1] = 1), zeros from entry (c & ~3) + 1 on before it
+    float4* V;         // [block][n up to whole fours][ceil(n/2)] reflector c in row c (v[c+1] = 1), two entries as (hi, hi, lo, lo), zeros
+                       // from entry c & ~3 on before it and past entry n - 1
     double *tau, *dg, *eg;  // [block][n]
     // whole-chip form: exchange of p, and the barrier between CTAs
     float2* pbuf;      // [2][n]
@@ -330,7 +288,8 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
     const int rank = (int)(blockIdx.x % C), b = (int)(blockIdx.x / C);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     float* D = a.D + (size_t)b * n * 2 * ld;
-    float2* V = a.V + (size_t)b * n * n;
+    const int vs = (n + 1) / 2;
+    float4* V = a.V + (size_t)b * ((n + 3) & ~3) * vs;
     float* vcur = reinterpret_cast<float*>(smem_raw);  // v of the step being applied
     float* vnxt = vcur + 2 * ld;                       // the next reflector
     float* w = vnxt + 2 * ld;
@@ -449,7 +408,7 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
         reflect(0, s, x, vnxt);
         __syncthreads();
         if (rank == 0)
-            for (int i = 1 + t; i < n; i += T) V[i] = df_pack(get(vnxt, i));
+            for (int i = t; i < vs; i += T) V[i] = reinterpret_cast<const float4*>(vnxt)[i];
         pass(1, 0, no{}, yes{});
         if (!barrier()) return;
     }
@@ -511,7 +470,7 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
         reflect(c1, s, x, vnxt);
         __syncthreads();
         if (rank == c1 % C)
-            for (int i = (c1 & ~3) + 1 + t; i < n; i += T) V[(size_t)c1 * n + i] = df_pack(get(vnxt, i));
+            for (int i = (c1 & ~3) / 2 + t; i < vs; i += T) V[(size_t)c1 * vs + i] = reinterpret_cast<const float4*>(vnxt)[i];
         if (c < n - 3)
             pass(c + 2, par ^ 1, yes{}, yes{});
         else
@@ -642,7 +601,7 @@ void launch_tridiag(int n, int nblk, bool chip, const double* A, double* V, doub
     a.n = n;
     a.ld = pad(n);
     a.D = static_cast<float*>(work);
-    a.V = reinterpret_cast<float2*>(V);
+    a.V = reinterpret_cast<float4*>(V);
     a.tau = tau;
     a.dg = dg;
     a.eg = eg;
