@@ -34,7 +34,8 @@
 namespace opsec {
 namespace {
 
-constexpr int kMaxN = 1024;  // largest block of the batched form
+constexpr int kMaxN = 1024;     // largest block of the batched form
+constexpr int kMaxRows = 4096;  // largest matrix
 
 // Deterministic CTA-wide sum: the same inputs give the same bits in every CTA of the cluster.
 __device__ double cta_sum(double x, double* red) {
@@ -177,40 +178,48 @@ __device__ __forceinline__ double exp_scale(double x, int* e) {
 }
 __device__ __forceinline__ unsigned hi_xor(double a, double b) { return (unsigned)(__double2hiint(a) ^ __double2hiint(b)); }
 
-constexpr int kShifts = 2;  // Sturm counts at a time: independent recurrences under one row's latency
-
-// eigenvalues below each shift
-__device__ void sturm64(int np, const Rows64& t, const double (&s)[kShifts], int (&cnt)[kShifts]) {
-    double x[kShifts], xp[kShifts];
-    unsigned c[kShifts];
-#pragma unroll
-    for (int q = 0; q < kShifts; q++) {
-        x[q] = 1.0;
-        xp[q] = 0.0;
-        c[q] = 0;
+// The lanes that share a candidate: 2 to 32 neighbouring ones, which take the same decisions.
+struct Team {
+    unsigned mask;
+    int size, sub, base;  // lanes, this lane's place among them, the first one
+    template <class X>
+    __device__ __forceinline__ X from(X v, int q) const {
+        return __shfl_sync(mask, v, base + q);
     }
+    __device__ __forceinline__ double sum(double v) const {
+        for (int o = size / 2; o; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+    // the largest v's smallest r
+    __device__ __forceinline__ void best(int* v, int* r) const {
+        for (int o = size / 2; o; o >>= 1) {
+            const int vo = __shfl_xor_sync(mask, *v, o), ro = __shfl_xor_sync(mask, *r, o);
+            if (vo > *v || (vo == *v && ro < *r)) {
+                *v = vo;
+                *r = ro;
+            }
+        }
+    }
+};
+
+// eigenvalues below the shift
+__device__ int sturm64(int np, const Rows64& t, double s) {
+    double x = 1.0, xp = 0.0;
+    unsigned c = 0;
     for (int i = 0; i < np; i += kGrp64) {
 #pragma unroll
         for (int k = 0; k < kGrp64; k++) {
-            const double f = t.ff[i + k], g = t.fi[i + k], b = t.fb[i + k];
-#pragma unroll
-            for (int q = 0; q < kShifts; q++) {
-                const double y = fma(fma(-s[q], g, f), x[q], b * xp[q]);
-                c[q] += hi_xor(y, x[q]) >> 31;
-                xp[q] = x[q];
-                x[q] = y;
-            }
+            const double y = fma(fma(-s, t.fi[i + k], t.ff[i + k]), x, t.fb[i + k] * xp);
+            c += hi_xor(y, x) >> 31;
+            xp = x;
+            x = y;
         }
-#pragma unroll
-        for (int q = 0; q < kShifts; q++) {
-            int e;
-            const double sc = exp_scale(fmax(fabs(x[q]), fabs(xp[q])), &e);
-            x[q] *= sc;
-            xp[q] *= sc;
-        }
+        int e;
+        const double sc = exp_scale(fmax(fabs(x), fabs(xp)), &e);
+        x *= sc;
+        xp *= sc;
     }
-#pragma unroll
-    for (int q = 0; q < kShifts; q++) cnt[q] = (int)c[q];
+    return (int)c;
 }
 
 // The same counts in double-FP32 (47 bits; rescaled every row, FP32's exponent range being short):
@@ -218,66 +227,46 @@ __device__ void sturm64(int np, const Rows64& t, const double (&s)[kShifts], int
 struct RowsDf {
     const float2 *f, *g, *b;  // d/|e_i|, 1/|e_i|, -|e_{i-1}|/|e_i| as (hi, lo) pairs
 };
-__device__ void sturm_df(int np, const RowsDf& t, const double (&s)[kShifts], int (&cnt)[kShifts]) {
-    df x[kShifts], xp[kShifts], ms[kShifts];
-    unsigned c[kShifts];
-#pragma unroll
-    for (int q = 0; q < kShifts; q++) {
-        x[q] = df{1.f, 0.f};
-        xp[q] = df{0.f, 0.f};
-        ms[q] = df_from(-s[q]);
-        c[q] = 0;
-    }
-#pragma unroll 2
+__device__ int sturm_df(int np, const RowsDf& t, double s) {
+    df x{1.f, 0.f}, xp{0.f, 0.f};
+    const df ms = df_from(-s);
+    unsigned c = 0;
+#pragma unroll 4
     for (int i = 0; i < np; i++) {
         const df f = df_unpack(t.f[i]), g = df_unpack(t.g[i]), b = df_unpack(t.b[i]);
-#pragma unroll
-        for (int q = 0; q < kShifts; q++) {
-            const df y = df_fma(df_mul(b, xp[q]), df_fma(f, ms[q], g), x[q]);
-            c[q] += (__float_as_uint(y.h) ^ __float_as_uint(x[q].h)) >> 31;
-            const unsigned e = __float_as_uint(fmaxf(fabsf(y.h), fabsf(x[q].h))) & 0x7f800000u;
-            const float sc = __uint_as_float(0x7f000000u - e);  // 2^-exponent
-            xp[q] = df{x[q].h * sc, x[q].l * sc};
-            x[q] = df{y.h * sc, y.l * sc};
-        }
+        const df y = df_fma(df_mul(b, xp), df_fma(f, ms, g), x);
+        c += (__float_as_uint(y.h) ^ __float_as_uint(x.h)) >> 31;
+        const unsigned e = __float_as_uint(fmaxf(fabsf(y.h), fabsf(x.h))) & 0x7f800000u;
+        const float sc = __uint_as_float(0x7f000000u - e);  // 2^-exponent
+        xp = df{x.h * sc, x.l * sc};
+        x = df{y.h * sc, y.l * sc};
     }
-#pragma unroll
-    for (int q = 0; q < kShifts; q++) cnt[q] = (int)c[q];
+    return (int)c;
 }
 
 // One step of the search for eigenvalue j in (lo, hi), which hold clo and chi eigenvalues below
-// them: the bracket's interior shifts, evenly spaced.  False when they no longer separate.
+// them: the bracket's interior shifts, evenly spaced, one a lane of the team (two where more no longer
+// separate).  False when two do not.
 template <class Count>
-__device__ bool narrow(Count count, int j, double* lo, double* hi, int* clo, int* chi) {
-    double s[kShifts];
-    int c[kShifts];
-    bool apart = true;
-#pragma unroll
-    for (int q = 0; q < kShifts; q++) {
-        s[q] = *lo + (*hi - *lo) * ((q + 1) / (double)(kShifts + 1));
-        apart = apart && s[q] > (q ? s[q - 1] : *lo);
+__device__ bool narrow(const Team& tm, Count count, int j, double* lo, double* hi, int* clo, int* chi) {
+    for (int ns = tm.size;; ns = 2) {
+        auto shift = [&](int q) { return q < 0 ? *lo : q >= ns ? *hi : *lo + (*hi - *lo) * ((q + 1) / (double)(ns + 1)); };
+        const int q = min(tm.sub, ns - 1);
+        const double s = shift(q);
+        if (__all_sync(tm.mask, s > shift(q - 1) && s < shift(q + 1))) {
+            const int c = count(s);
+            const unsigned above = (__ballot_sync(tm.mask, c > j) >> tm.base) & (ns == 32 ? ~0u : (1u << ns) - 1);
+            const int h = above ? __ffs((int)above) - 1 : ns;  // the first shift above eigenvalue j
+            const double l = shift(h - 1), u = shift(h);
+            const int cl = tm.from(c, max(h - 1, 0)), cu = tm.from(c, min(h, ns - 1));
+            if (h > 0) *clo = cl;
+            if (h < ns) *chi = cu;
+            *lo = l;
+            *hi = u;
+            return true;
+        }
+        if (ns == 2) return false;
     }
-    if (!apart || !(s[kShifts - 1] < *hi)) return false;
-    count(s, c);
-    double l = *lo, h = *hi;
-    int cl = *clo, ch = *chi;
-#pragma unroll
-    for (int q = kShifts - 1; q >= 0; q--)
-        if (c[q] > j) {
-            h = s[q];
-            ch = c[q];
-        }
-#pragma unroll
-    for (int q = 0; q < kShifts; q++)
-        if (c[q] <= j && s[q] < h) {
-            l = s[q];
-            cl = c[q];
-        }
-    *lo = l;
-    *hi = h;
-    *clo = cl;
-    *chi = ch;
-    return true;
 }
 
 // 2^k, zero far below the smallest normal
@@ -288,97 +277,103 @@ __device__ __forceinline__ double pow2i(int k) { return k < -1000 ? 0.0 : __hilo
 // Wronskian, so that is where the residual gamma_r of z = (x_i / x_r above, 1, y_i / y_r below) is
 // least.  Entries carry the exponent of their group of kGrp64 rows.  Returns the
 // Rayleigh-quotient correction gamma_r / |z|^2; |z|^2 in *nz_out.
-__device__ double rq_step(int n, const Rows64& t, const double* __restrict__ d, const double* __restrict__ e, double inv,
-                          double s, const VecArgs& a, int col, int* r_out, double* nz_out) {
+// Even lanes of the team take the solution from the top, odd ones that from the bottom; the scans are dealt
+// over all of them.
+__device__ double rq_step(const Team& tm, int n, const Rows64& t, const double* __restrict__ d,
+                          const double* __restrict__ e, double inv, double s, const VecArgs& a, int col, int* r_out,
+                          double* nz_out) {
     const size_t K = (size_t)a.ktot;
     double* X = a.X + col;
     double* Y = a.Y + col;
     const int ngrp = (n + kGrp64 - 1) / kGrp64;
     int* KX = a.KX + col;
     int* KY = KX + (size_t)ngrp * K;
-    double x = 1.0, xp = 0.0, y = 1.0, yp = 0.0;
-    int kx = 0, ky = 0;
-    for (int g = 0; g < ngrp; g++) {
-        // from the top rows of group g, from the bottom rows of group ngrp-1-g (rows past n keep y = 1)
-        KX[g * K] = kx;
-        KY[(ngrp - 1 - g) * K] = ky;
+    __syncwarp(tm.mask);  // the last step's solutions have been read
+    {
+        const bool up = tm.sub & 1, own = tm.sub < 2;
+        const double *pf = up ? t.bf : t.ff, *pb = up ? t.bb : t.fb;
+        double* P = up ? Y : X;
+        int* KP = up ? KY : KX;
+        double x = 1.0, xp = 0.0;
+        int kx = 0;
+        for (int g = 0; g < ngrp; g++) {
+            // rows of group g from the top, of group ngrp-1-g from the bottom (rows past n keep x)
+            const int gi = up ? ngrp - 1 - g : g;
+            if (own) KP[gi * K] = kx;
 #pragma unroll
-        for (int k = 0; k < kGrp64; k++) {
-            const int i = g * kGrp64 + k, j = (ngrp - g) * kGrp64 - 1 - k;
-            if (i < n) X[i * K] = x;
-            if (j < n) Y[j * K] = y;
-            const double xn = fma(fma(-s, t.fi[i], t.ff[i]), x, t.fb[i] * xp);
-            const double yn = fma(fma(-s, t.fi[max(j - 1, 0)], t.bf[j]), y, t.bb[j] * yp);
-            xp = x;
-            x = xn;
-            yp = y;
-            y = j < n ? yn : y;
+            for (int k = 0; k < kGrp64; k++) {
+                const int i = gi * kGrp64 + (up ? kGrp64 - 1 - k : k);
+                if (own && i < n) P[i * K] = x;
+                const double xn = fma(fma(-s, t.fi[up ? max(i - 1, 0) : i], pf[i]), x, pb[i] * xp);
+                xp = x;
+                x = i < n ? xn : x;
+            }
+            int ex;
+            const double sx = exp_scale(fmax(fabs(x), fabs(xp)), &ex);
+            x *= sx;
+            xp *= sx;
+            kx += ex;
         }
-        int ex, ey;
-        const double sx = exp_scale(fmax(fabs(x), fabs(xp)), &ex), sy = exp_scale(fmax(fabs(y), fabs(yp)), &ey);
-        x *= sx;
-        xp *= sx;
-        y *= sy;
-        yp *= sy;
-        kx += ex;
-        ky += ey;
     }
-    // the twist: log2 |x_r y_r| to 0.1 from the high words; kB rows' loads at a time, without branches
-    constexpr int kB = 4 * kGrp64;
+    __syncwarp(tm.mask);
+    // the twist: log2 |x_r y_r| to 0.1 from the high words; kB groups' loads at a time, without branches
+    constexpr int kB = 4;
     int r = 0, best = INT_MIN;
-    for (int i0 = 0; i0 < n; i0 += kB) {
-        int l[kB], kg[kB / kGrp64];
+    for (int g0 = tm.sub; g0 < ngrp; g0 += kB * tm.size) {
+        int l[kB * kGrp64], kg[kB];
 #pragma unroll
-        for (int u = 0; u < kB / kGrp64; u++) {
-            const int g = min(i0 / kGrp64 + u, ngrp - 1);
+        for (int u = 0; u < kB; u++) {
+            const int g = min(g0 + u * tm.size, ngrp - 1);
             kg[u] = (KX[g * K] + KY[g * K]) << 10;
         }
 #pragma unroll
-        for (int k = 0; k < kB; k++) {
-            const size_t o = (size_t)min(i0 + k, n - 1) * K;
+        for (int k = 0; k < kB * kGrp64; k++) {
+            const size_t o = (size_t)min((g0 + k / kGrp64 * tm.size) * kGrp64 + k % kGrp64, n - 1) * K;
             l[k] = ((__double2hiint(X[o]) & 0x7fffffff) >> 10) + ((__double2hiint(Y[o]) & 0x7fffffff) >> 10);
         }
 #pragma unroll
-        for (int k = 0; k < kB; k++) {
-            const int v = l[k] + kg[k / kGrp64];
-            if (i0 + k < n && v > best) {
+        for (int k = 0; k < kB * kGrp64; k++) {
+            const int v = l[k] + kg[k / kGrp64], i = (g0 + k / kGrp64 * tm.size) * kGrp64 + k % kGrp64;
+            if (i < n && v > best) {
                 best = v;
-                r = i0 + k;
+                r = i;
             }
         }
     }
+    tm.best(&best, &r);
     // entries above and below r relative to it
     const double xr = 1.0 / X[r * K], yr = 1.0 / Y[r * K];
     const int kxr = KX[(r / kGrp64) * K], kyr = KY[(r / kGrp64) * K];
     double gamma = d[r] * inv - s;
     if (r > 0) gamma -= fabs(e[r - 1]) * inv * (X[(r - 1) * K] * xr * pow2i(KX[((r - 1) / kGrp64) * K] - kxr));
     if (r + 1 < n) gamma -= fabs(e[r]) * inv * (Y[(r + 1) * K] * yr * pow2i(KY[((r + 1) / kGrp64) * K] - kyr));
-    double nz = 1.0;
-    for (int i0 = 0; i0 < n; i0 += kB) {
-        double v[kB], fx[kB / kGrp64], fy[kB / kGrp64];
+    double nz = 0.0;
+    for (int g0 = tm.sub; g0 < ngrp; g0 += kB * tm.size) {
+        double v[kB * kGrp64], fx[kB], fy[kB];
 #pragma unroll
-        for (int u = 0; u < kB / kGrp64; u++) {
-            const int g = min(i0 / kGrp64 + u, ngrp - 1);
+        for (int u = 0; u < kB; u++) {
+            const int g = min(g0 + u * tm.size, ngrp - 1);
             fx[u] = pow2i(KX[g * K] - kxr);
             fy[u] = pow2i(KY[g * K] - kyr);
         }
 #pragma unroll
-        for (int k = 0; k < kB; k++) {
-            const int i = min(i0 + k, n - 1);
+        for (int k = 0; k < kB * kGrp64; k++) {
+            const int i = min((g0 + k / kGrp64 * tm.size) * kGrp64 + k % kGrp64, n - 1);
             v[k] = (i < r ? X : Y)[(size_t)i * K];
         }
 #pragma unroll
-        for (int u = 0; u < kB / kGrp64; u++) {
+        for (int u = 0; u < kB; u++) {
             fx[u] *= xr;
             fy[u] *= yr;
         }
 #pragma unroll
-        for (int k = 0; k < kB; k++) {
-            const int i = i0 + k;
+        for (int k = 0; k < kB * kGrp64; k++) {
+            const int i = (g0 + k / kGrp64 * tm.size) * kGrp64 + k % kGrp64;
             const double zi = v[k] * (i < r ? fx[k / kGrp64] : fy[k / kGrp64]);
             nz = fma(zi, i < n && i != r ? zi : 0.0, nz);
         }
     }
+    nz = 1.0 + tm.sum(nz);
     *r_out = r;
     *nz_out = nz;
     return gamma / nz;
@@ -405,7 +400,7 @@ __device__ __forceinline__ double gamma_of(int n, const double* d, const double*
     if (r + 1 < n) g -= fabs(e[r]) * inv * ty;
     return g;
 }
-__device__ double rq_first(int n, const RowsDf& t, const RowsDfB& tb, const double* __restrict__ d,
+__device__ double rq_first(const Team& tm, int n, const RowsDf& t, const RowsDfB& tb, const double* __restrict__ d,
                            const double* __restrict__ e, double inv, double s, const VecArgs& a, int col, int* r_out,
                            double* nz_out) {
     const size_t K = (size_t)a.ktot;
@@ -414,107 +409,106 @@ __device__ double rq_first(int n, const RowsDf& t, const RowsDfB& tb, const doub
     const int ngrp = (n + kGrpDf - 1) / kGrpDf;
     int* KX = a.KX + col;
     int* KY = KX + (size_t)ngrp * K;
-    const df ms = df_from(-s);
-    df x{1.f, 0.f}, xp{0.f, 0.f}, y{1.f, 0.f}, yp{0.f, 0.f};
-    int kx = 0, ky = 0;
-    for (int g = 0; g < ngrp; g++) {
-        KX[g * K] = kx;
-        KY[(ngrp - 1 - g) * K] = ky;
+    {
+        const bool up = tm.sub & 1, own = tm.sub < 2;
+        const float2 *pf = up ? tb.f : t.f, *pb = up ? tb.b : t.b;
+        float2* P = up ? Y : X;
+        int* KP = up ? KY : KX;
+        const df ms = df_from(-s);
+        df x{1.f, 0.f}, xp{0.f, 0.f};
+        int kx = 0;
+#pragma unroll 2
+        for (int g = 0; g < ngrp; g++) {
+            const int gi = up ? ngrp - 1 - g : g;
+            if (own) KP[gi * K] = kx;
 #pragma unroll
-        for (int k = 0; k < kGrpDf; k++) {
-            const int i = g * kGrpDf + k, j = (ngrp - g) * kGrpDf - 1 - k;
-            if (i < n) X[i * K] = df_pack(x);
-            if (j < n) Y[j * K] = df_pack(y);
-            const df xn = df_fma(df_mul(df_unpack(t.b[i]), xp), df_fma(df_unpack(t.f[i]), ms, df_unpack(t.g[i])), x);
-            const df yn = df_fma(df_mul(df_unpack(tb.b[j]), yp),
-                                 df_fma(df_unpack(tb.f[j]), ms, df_unpack(t.g[max(j - 1, 0)])), y);
-            xp = x;
-            x = xn;
-            yp = y;
-            if (j < n) y = yn;
+            for (int k = 0; k < kGrpDf; k++) {
+                const int i = gi * kGrpDf + (up ? kGrpDf - 1 - k : k);
+                if (own && i < n) P[i * K] = df_pack(x);
+                const df xn = df_fma(df_mul(df_unpack(pb[i]), xp),
+                                     df_fma(df_unpack(pf[i]), ms, df_unpack(t.g[up ? max(i - 1, 0) : i])), x);
+                xp = x;
+                if (i < n) x = xn;
+            }
+            int ex;
+            const float sx = exp_scale(x, xp, &ex);
+            x = rescaled(x, sx);
+            xp = rescaled(xp, sx);
+            kx += ex;
         }
-        int ex, ey;
-        const float sx = exp_scale(x, xp, &ex), sy = exp_scale(y, yp, &ey);
-        x = rescaled(x, sx);
-        xp = rescaled(xp, sx);
-        y = rescaled(y, sy);
-        yp = rescaled(yp, sy);
-        kx += ex;
-        ky += ey;
     }
+    __syncwarp(tm.mask);
     constexpr int kB = 32;  // rows' loads at a time, without branches
     int r = 0, best = INT_MIN;
-    for (int i0 = 0; i0 < n; i0 += kB) {
+    for (int i0 = tm.sub; i0 < n; i0 += kB * tm.size) {
         int l[kB];
 #pragma unroll
         for (int k = 0; k < kB; k++) {
-            const int i = min(i0 + k, n - 1);
+            const int i = min(i0 + k * tm.size, n - 1);
             const size_t o = (size_t)i * K, og = (size_t)(i / kGrpDf) * K;
             l[k] = ((KX[og] + KY[og]) << 10) + ((__float_as_int(X[o].x) & 0x7fffffff) >> 13) +
                    ((__float_as_int(Y[o].x) & 0x7fffffff) >> 13);
         }
 #pragma unroll
         for (int k = 0; k < kB; k++)
-            if (i0 + k < n && l[k] > best) {
+            if (i0 + k * tm.size < n && l[k] > best) {
                 best = l[k];
-                r = i0 + k;
+                r = i0 + k * tm.size;
             }
     }
+    tm.best(&best, &r);
     auto pow2f = [](int k) { return k < -126 ? 0.f : __int_as_float((min(k, 126) + 127) << 23); };
     const int kxr = KX[(r / kGrpDf) * K], kyr = KY[(r / kGrpDf) * K];
     const float xr = 1.0f / X[r * K].x, yr = 1.0f / Y[r * K].x;
-    float nz = 1.f;
-    for (int i0 = 0; i0 < n; i0 += kB) {
+    float nz = 0.f;
+    for (int i0 = tm.sub; i0 < n; i0 += kB * tm.size) {
         float v[kB], f[kB];
 #pragma unroll
         for (int k = 0; k < kB; k++) {
-            const int i = min(i0 + k, n - 1);
+            const int i = min(i0 + k * tm.size, n - 1);
             const bool top = i < r;
             v[k] = (top ? X : Y)[(size_t)i * K].x;
             f[k] = pow2f((top ? KX : KY)[(size_t)(i / kGrpDf) * K] - (top ? kxr : kyr));
         }
 #pragma unroll
         for (int k = 0; k < kB; k++) {
-            const int i = i0 + k;
+            const int i = i0 + k * tm.size;
             const float zi = v[k] * (i < r ? xr : yr) * f[k];
             if (i < n && i != r) nz = fmaf(zi, zi, nz);
         }
     }
+    const double nzs = 1.0 + tm.sum((double)nz);
     double tx = 0.0, ty = 0.0;
     if (r > 0)
         tx = df_to(df_unpack(X[(r - 1) * K])) / df_to(df_unpack(X[r * K])) * pow2i(KX[((r - 1) / kGrpDf) * K] - kxr);
     if (r + 1 < n)
         ty = df_to(df_unpack(Y[(r + 1) * K])) / df_to(df_unpack(Y[r * K])) * pow2i(KY[((r + 1) / kGrpDf) * K] - kyr);
     *r_out = r;
-    *nz_out = (double)nz;
-    return gamma_of(n, d, e, inv, s, r, tx, ty) / (double)nz;
+    *nz_out = nzs;
+    return gamma_of(n, d, e, inv, s, r, tx, ty) / nzs;
 }
 
-// gamma_r at s for a given twist row: the solution from the top down to r, then the one from the
-// bottom up to r, in double-FP32; nothing is stored.
-__device__ double gamma_df(int n, const RowsDf& t, const RowsDfB& tb, const double* __restrict__ d,
+// gamma_r at s for a given twist row: even lanes the solution from the top down to r, odd lanes the
+// one from the bottom up to r, in double-FP32; nothing is stored.
+__device__ double gamma_df(const Team& tm, int n, const RowsDf& t, const RowsDfB& tb, const double* __restrict__ d,
                            const double* __restrict__ e, double inv, double s, int r) {
+    const bool up = tm.sub & 1;
+    const float2 *pf = up ? tb.f : t.f, *pb = up ? tb.b : t.b, *pg = up ? t.g - 1 : t.g;
+    const int i0 = up ? n - 1 : 0, di = up ? -1 : 1, steps = up ? n - 1 - r : r;
     const df ms = df_from(-s);
     df x{1.f, 0.f}, xp{0.f, 0.f};
-    double tx = 0.0;
-    for (int q = 0; q < n - 1; q++) {
-        const bool top = q < r;
-        if (q == r) {  // x holds row r of the solution from the top
-            tx = r > 0 ? df_to(xp) / df_to(x) : 0.0;
-            x = df{1.f, 0.f};
-            xp = df{0.f, 0.f};
-        }
-        const int i = top ? q : n - 1 - (q - r);
-        const df f = df_unpack((top ? t.f : tb.f)[i]), b = df_unpack((top ? t.b : tb.b)[i]);
-        const df g = df_unpack(t.g[top ? i : i - 1]);
-        const df y = df_fma(df_mul(b, xp), df_fma(f, ms, g), x);
+#pragma unroll 4
+    for (int q = 0; q < steps; q++) {
+        const int i = i0 + di * q;
+        const df y = df_fma(df_mul(df_unpack(pb[i]), xp), df_fma(df_unpack(pf[i]), ms, df_unpack(pg[i])), x);
         int ex;
         const float sc = exp_scale(y, x, &ex);
         xp = rescaled(x, sc);
         x = rescaled(y, sc);
     }
-    const double ratio = df_to(xp) / df_to(x);
-    return gamma_of(n, d, e, inv, s, r, r == n - 1 ? ratio : tx, r == n - 1 ? 0.0 : ratio);
+    __syncwarp(tm.mask);
+    const double ratio = steps > 0 ? df_to(xp) / df_to(x) : 0.0;
+    return gamma_of(n, d, e, inv, s, r, tm.from(ratio, 0), tm.from(ratio, 1));
 }
 
 // The rows of the recurrences of every block, five FP64 arrays and their double-FP32 pairs, each of
@@ -551,9 +545,10 @@ __global__ void rows_kernel(int n, int nblk, const double* __restrict__ dg, cons
     }
 }
 
-// grid (nblk, parts of kc), 4 warps of `per` candidates each, one per thread: candidate c (0 =
-// largest) of block b.  An FP64 instruction takes a warp 64 cycles of its scheduler's pipe however
-// many of its lanes work, so the candidates are dealt over all schedulers of the chip.
+// grid (nblk, parts of kc), 4 warps of `per` candidates each, a team of lanes per candidate: candidate c
+// (0 = largest) of block b.  An FP64 instruction takes a warp 64 cycles of its scheduler's pipe however
+// many of its lanes work, so the candidates are dealt over all schedulers of the chip, and the lanes left
+// over share a candidate: two directions of a solution, a shift of a Sturm count each, rows of the scans.
 // The FP32 estimate's bracket is confirmed by FP64 Sturm counts.  An eigenvalue alone in
 // its bracket is refined by Rayleigh-quotient iteration on twisted factorisations (cubic
 // convergence; the iterate must stay in the bracket); an eigenvalue sharing its bracket is
@@ -563,8 +558,10 @@ __global__ void rows_kernel(int n, int nblk, const double* __restrict__ dg, cons
 // every row; 34 of 1024^2 25.5 -> 3.77, 10 of 555^2 12.5 -> 2.01, 18 of 64^2 0.406 -> 0.092.
 // LOCAL: the block's rows in shared memory; otherwise (orders whose rows do not fit) read through L1.
 template <bool LOCAL>
-__global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* __restrict__ R, int per) {
+__global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* __restrict__ R, int per, int team) {
     extern __shared__ double rows64[];
+    __shared__ unsigned flips[kMaxRows / 32];           // row i: whether entries i and i + 1 change sign by T's e_i
+    __shared__ unsigned char before[kMaxRows / 32];  // parity of the words before
     const int b = blockIdx.x, n = a.n, np = round_up(n, kGrp64);
     const int kc = a.kc[b];
     if ((int)blockIdx.y * 4 * per >= kc) return;
@@ -581,21 +578,35 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
     const float2* rowsf = reinterpret_cast<const float2*>(rows + 5 * np);
     const RowsDf tf{rowsf, rowsf + np, rowsf + 2 * np};
     const RowsDfB tfb{rowsf + 3 * np, rowsf + 4 * np};
-    const int lane = threadIdx.x & 31, c = (blockIdx.y * 4 + (threadIdx.x >> 5)) * per + lane;
-    if (lane >= per || c >= kc) return;
+    const int lane = threadIdx.x & 31;
+    for (int w = threadIdx.x >> 5; 32 * w < n; w += 4) {
+        const int i = 32 * w + lane;
+        const unsigned m = __ballot_sync(0xffffffffu, i + 1 < n && !(egb[i] < 0.0));
+        if (lane == 0) flips[w] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 0, p = 0; 32 * w < n; w++) {
+            before[w] = (unsigned char)p;
+            p ^= __popc(flips[w]) & 1;
+        }
+    __syncthreads();
+    const int c = (blockIdx.y * 4 + (threadIdx.x >> 5)) * per + lane / team;
+    if (lane / team >= per || c >= kc) return;
+    const int tb0 = lane / team * team;
+    const Team tm{(team == 32 ? ~0u : (1u << team) - 1) << tb0, team, lane - tb0, tb0};
     const int j = n - 1 - c;  // ascending index
     const int col = a.koff[b] + c;
     const size_t K = (size_t)a.ktot;
     const double x = a.w[(size_t)b * n + j] * inv;
-    auto count_df = [&](const double (&sh)[kShifts], int (&cn)[kShifts]) { sturm_df(np, tf, sh, cn); };
-    auto count64 = [&](const double (&sh)[kShifts], int (&cn)[kShifts]) { sturm64(np, t, sh, cn); };
+    auto count_df = [&](double sh) { return sturm_df(np, tf, sh); };
+    auto count64 = [&](double sh) { return sturm64(np, t, sh); };
     // the FP32 estimate's bracket, confirmed
     double del = 8.0 * FLT_EPSILON, lo = -1.0, hi = 1.0;  // the scaled spectrum lies inside (-1, 1)
     int clo = 0, chi = n;
     for (int k = 0; k < 8 && (lo == -1.0 || hi == 1.0); k++, del *= 8.0) {
-        const double sh[kShifts] = {x - del, x + del};
-        int cn[kShifts];
-        count_df(sh, cn);
+        const double sh[2] = {x - del, x + del};
+        const int own = count_df(sh[tm.sub & 1]), cn[2] = {tm.from(own, 0), tm.from(own, 1)};
         if (cn[0] <= j && sh[0] > lo) {
             lo = sh[0];
             clo = cn[0];
@@ -612,17 +623,15 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
     // a bracket holding several eigenvalues is narrowed until it holds this one alone: in double-FP32
     // down to well above its rounding, then in FP64
     for (int it = 0; it < 40 && chi - clo > 1 && hi - lo > 1e-12; it++)
-        if (!narrow(count_df, j, &lo, &hi, &clo, &chi)) break;
+        if (!narrow(tm, count_df, j, &lo, &hi, &clo, &chi)) break;
     if (chi - clo > 1) {
         lo -= 1e-13;  // a double-FP32 count may be off this close to an eigenvalue
         hi += 1e-13;
-        const double sh[kShifts] = {lo, hi};
-        int cn[kShifts];
-        count64(sh, cn);
-        clo = cn[0];
-        chi = cn[1];
+        const int own = count64(tm.sub & 1 ? hi : lo);
+        clo = tm.from(own, 0);
+        chi = tm.from(own, 1);
         for (int it = 0; it < 40 && chi - clo > 1 && hi - lo > 4.0 * DBL_EPSILON; it++)
-            if (!narrow(count64, j, &lo, &hi, &clo, &chi)) break;
+            if (!narrow(tm, count64, j, &lo, &hi, &clo, &chi)) break;
     }
     if (chi - clo == 1) {
         // converged when the correction is below 1e-14 of the block scale (T is scaled to norm
@@ -630,14 +639,14 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
         double s = fmin(fmax(x, lo), hi), prev = 1.0;
         {
             // most of the way in double-FP32, at one twist row: an FP64 step costs four times as much
-            double s1 = s, dl = rq_first(n, tf, tfb, dgb, egb, inv, s, a, col, &r, &nz), pl = 1.0;
+            double s1 = s, dl = rq_first(tm, n, tf, tfb, dgb, egb, inv, s, a, col, &r, &nz), pl = 1.0;
             for (int it = 0;; it++) {
                 s1 += dl;
                 if (!(s1 > lo && s1 < hi) || it == 4 || !(fabs(dl) < pl)) break;
                 s = s1;
                 if (fabs(dl) <= 1e-13) break;
                 pl = fabs(dl);
-                dl = gamma_df(n, tf, tfb, dgb, egb, inv, s, r) / nz;
+                dl = gamma_df(tm, n, tf, tfb, dgb, egb, inv, s, r) / nz;
             }
         }
         // FP64 from there; an iterate that left the bracket starts again from the bracket narrowed to
@@ -645,14 +654,14 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
         for (int att = 0; att < 2 && !done; att++) {
             if (att) {
                 for (int it = 0; it < 40 && hi - lo > 1e-12; it++)
-                    if (!narrow(count_df, j, &lo, &hi, &clo, &chi)) break;
+                    if (!narrow(tm, count_df, j, &lo, &hi, &clo, &chi)) break;
                 lo -= 1e-13;
                 hi += 1e-13;
                 s = 0.5 * (lo + hi);
                 prev = 1.0;
             }
             for (int it = 0; it < 8; it++) {
-                const double dl = rq_step(n, t, dgb, egb, inv, s, a, col, &r, &nz);
+                const double dl = rq_step(tm, n, t, dgb, egb, inv, s, a, col, &r, &nz);
                 const double s1 = s + dl;
                 if (!(s1 > lo && s1 < hi)) break;  // left the bracket
                 if (fabs(dl) <= 1e-14 || (fabs(dl) <= 1e-10 && fabs(dl) > 0.25 * prev)) {
@@ -667,11 +676,11 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
     }
     if (!done) {
         for (int it = 0; it < 48 && hi - lo > 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + 1e-300; it++)
-            if (!narrow(count64, j, &lo, &hi, &clo, &chi)) break;
+            if (!narrow(tm, count64, j, &lo, &hi, &clo, &chi)) break;
         lam = 0.5 * (lo + hi);
-        rq_step(n, t, dgb, egb, inv, lam, a, col, &r, &nz);
+        rq_step(tm, n, t, dgb, egb, inv, lam, a, col, &r, &nz);
     }
-    a.w[(size_t)b * n + j] = lam * sc;
+    if (tm.sub == 0) a.w[(size_t)b * n + j] = lam * sc;
     const double s = 1.0 / sqrt(nz);
     if (!isfinite(s) || !(s > 0.0)) atomicMax(&a.status[b], 3);
     // the vector, normalised, with the signs of T's own off-diagonals (entry r positive)
@@ -682,29 +691,29 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
     const double* Y = a.Y + col;
     const double xr = s / X[r * K], yr = s / Y[r * K];
     const int kxr = KX[(r / kGrp64) * K], kyr = KY[(r / kGrp64) * K];
-    int neg = 0;  // parity of the sign flips between row i and row r
-    for (int i = 0; i < r; i++) neg ^= !(egb[i] < 0.0);
+    // parity of the sign flips above row i
+    auto parity = [&](int i) { return before[i >> 5] ^ (__popc(flips[i >> 5] & ((1u << (i & 31)) - 1)) & 1); };
+    const int pr = parity(r);
     constexpr int kU = 4;  // groups loaded at a time
-    for (int g0 = 0; g0 < ngrp; g0 += kU) {
+    for (int g0 = tm.sub; g0 < ngrp; g0 += kU * team) {
         double v[kU * kGrp64], fx[kU], fy[kU];
 #pragma unroll
         for (int u = 0; u < kU; u++) {
-            const int g = min(g0 + u, ngrp - 1);
+            const int g = min(g0 + u * team, ngrp - 1);
             fx[u] = xr * pow2i(KX[g * K] - kxr);
             fy[u] = yr * pow2i(KY[g * K] - kyr);
         }
 #pragma unroll
         for (int k = 0; k < kU * kGrp64; k++) {
-            const int i = g0 * kGrp64 + k;
+            const int i = (g0 + k / kGrp64 * team) * kGrp64 + k % kGrp64;
             v[k] = i < n ? (i < r ? X : Y)[i * K] : 0.0;
         }
 #pragma unroll
         for (int k = 0; k < kU * kGrp64; k++) {
-            const int i = g0 * kGrp64 + k;
+            const int i = (g0 + k / kGrp64 * team) * kGrp64 + k % kGrp64;
             if (i < n) {
                 const double zi = v[k] * (i < r ? fx[k / kGrp64] : fy[k / kGrp64]);
-                a.Z[i * K + col] = neg ? -zi : zi;
-                if (i + 1 < n) neg ^= !(egb[i] < 0.0);
+                a.Z[i * K + col] = parity(i) != pr ? -zi : zi;
             }
         }
     }
@@ -1053,7 +1062,9 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     int dev = 0, nsm = 0;
     OPSEC_CUDA(cudaGetDevice(&dev));
     OPSEC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const int per = std::min(32, std::max(1, (p.ktot + 4 * nsm - 1) / (4 * nsm)));
+    const int per = std::min(16, std::max(1, (p.ktot + 4 * nsm - 1) / (4 * nsm)));
+    int team = 32;  // lanes a candidate
+    while (team * per > 32) team /= 2;
     const dim3 grid(p.nblk, (p.kmax + 4 * per - 1) / (4 * per));
     if (g_clock) g_clock->begin("blockeig_pairs", s);
     const int np = (p.n + kGrp64 - 1) / kGrp64 * kGrp64;
@@ -1063,9 +1074,9 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     const size_t room = (size_t)max_dynamic_smem((const void*)vectors_kernel<true>);
     if (rows <= room) {
         OPSEC_CUDA(cudaFuncSetAttribute(vectors_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
-        vectors_kernel<true><<<grid, 128, rows, s>>>(a, p.R, per);
+        vectors_kernel<true><<<grid, 128, rows, s>>>(a, p.R, per, team);
     } else {
-        vectors_kernel<false><<<grid, 128, 0, s>>>(a, p.R, per);
+        vectors_kernel<false><<<grid, 128, 0, s>>>(a, p.R, per, team);
     }
     OPSEC_CUDA(cudaGetLastError());
     if (g_clock) g_clock->end(s);
