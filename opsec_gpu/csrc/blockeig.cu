@@ -114,7 +114,10 @@ __device__ double block_scale(int n, const double* d, const double* e, double* r
     return ldexp(1.0, ex);  // 2^ex > g
 }
 
-// Every eigenvalue j (ascending) of block b to ~1e-6 of its scale; grid (nblk, ceil(n/256)).
+// Every eigenvalue j (ascending) of block b to ~1e-6 of its scale; grid (nblk, ceil(n SECT / 256)).
+// SECT lanes an eigenvalue, SECT - 1 of which count below one shift each: the bracket shrinks SECT-fold a
+// count.  With two (bisection, one lane) the chip idles behind each count's chain of n rows.
+template <int SECT>
 __global__ void __launch_bounds__(256) spectrum_kernel(int n, const double* __restrict__ dg,
                                                        const double* __restrict__ eg, double* __restrict__ w,
                                                        double* __restrict__ scale_out) {
@@ -137,13 +140,27 @@ __global__ void __launch_bounds__(256) spectrum_kernel(int n, const double* __re
     }
     __syncthreads();
     if (blockIdx.y == 0 && threadIdx.x == 0) scale_out[b] = sc;
-    const int j = blockIdx.y * blockDim.x + threadIdx.x;
-    if (j >= n) return;
+    constexpr int kLanes = SECT > 2 ? SECT : 1;
+    const int t = blockIdx.y * blockDim.x + threadIdx.x, j = t / kLanes, q = t % kLanes;
     float lo = -1.0f, hi = 1.0f;  // the scaled spectrum lies in (-1, 1)
-    for (int it = 0; it < 40 && hi - lo > 2.5e-7f; it++) {
-        const float mid = 0.5f * (lo + hi);
-        if (sturm32(np, rows32, mid) > j) hi = mid;
-        else lo = mid;
+    if constexpr (SECT > 2) {
+        const int base = threadIdx.x & 31 & ~(SECT - 1);
+        for (int it = 0; it < 40 && hi - lo > 2.5e-7f; it++) {  // the same steps for every eigenvalue
+            const float d = (hi - lo) * (1.f / SECT);
+            const bool above = q + 1 == SECT || sturm32(np, rows32, fmaf((float)(q + 1), d, lo)) > j;
+            const int h = __ffs((int)((__ballot_sync(0xffffffffu, above) >> base) & ((1u << SECT) - 1)));  // 1 .. SECT
+            const float l = fmaf((float)(h - 1), d, lo);
+            if (h < SECT) hi = fmaf((float)h, d, lo);
+            lo = l;
+        }
+        if (j >= n || q) return;
+    } else {
+        if (j >= n) return;
+        for (int it = 0; it < 40 && hi - lo > 2.5e-7f; it++) {
+            const float mid = 0.5f * (lo + hi);
+            if (sturm32(np, rows32, mid) > j) hi = mid;
+            else lo = mid;
+        }
     }
     w[(size_t)b * n + j] = 0.5 * ((double)lo + (double)hi) * sc;
 }
@@ -555,7 +572,8 @@ __global__ void rows_kernel(int n, int nblk, const double* __restrict__ dg, cons
 // narrowed down first.  The last twisted factorisation gives the vector.
 // Bound by the FP64 pipe (64 cycles an instruction, measured, with nothing to overlap) and by loads of the stored solutions (32 rows at a time: row by row their latency was half the kernel).
 // Candidates of 34 blocks of 512^2 (4,351): 4.51 -> 1.15 ms against FP64 pivots with a division in
-// every row; 34 of 1024^2 25.5 -> 3.77, 10 of 555^2 12.5 -> 2.01, 18 of 64^2 0.406 -> 0.092.
+// every row; 34 of 1024^2 25.5 -> 3.77, 10 of 555^2 12.5 -> 2.01, 18 of 64^2 0.406 -> 0.092; with the lanes in teams
+// 34 of 512^2 0.90 -> 0.45, 10 of 555^2 0.98 -> 0.46, one of 1728^2 5.11 -> 1.61, of 3150^2 6.05 -> 2.69.
 // LOCAL: the block's rows in shared memory; otherwise (orders whose rows do not fit) read through L1.
 template <bool LOCAL>
 __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* __restrict__ R, int per, int team) {
@@ -1050,9 +1068,17 @@ bool blockeig_supported(int n) { return n >= 3 && n <= kMaxN; }
 void launch_blockeig_spectrum(int n, int nblk, const double* dg, const double* eg, double* w, double* scale,
                               cudaStream_t s, long long* launches) {
     const size_t smem = sizeof(float4) * (size_t)((n + kGrp32 - 1) / kGrp32 * kGrp32);
-    OPSEC_CUDA(cudaFuncSetAttribute(spectrum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    max_dynamic_smem((const void*)spectrum_kernel)));
-    spectrum_kernel<<<dim3(nblk, (n + 255) / 256), 256, smem, s>>>(n, dg, eg, w, scale);
+    auto run = [&](auto k, int lanes) {
+        OPSEC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem((const void*)k)));
+        k<<<dim3(nblk, (n * lanes + 255) / 256), 256, smem, s>>>(n, dg, eg, w, scale);
+    };
+    // Eight lanes an eigenvalue do 2.8 times the work in a third of the steps: while the chip is not full
+    // (18 blocks of 64^2 25 -> 14 us, 10 of 555^2 193 -> 102, one of 1728^2 585 -> 193, of 3150^2 1062 -> 350;
+    // 34 of 512^2 178 and 176).
+    if ((long long)n * nblk <= 16000)
+        run(spectrum_kernel<8>, 8);
+    else
+        run(spectrum_kernel<2>, 1);
     OPSEC_CUDA(cudaGetLastError());
     ++*launches;
 }
@@ -1087,7 +1113,9 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     compact_kernel<<<(groups + 3) / 4, 128, 0, s>>>(p.n, p.nblk, reinterpret_cast<float4*>(p.V), p.tau,
                                                     reinterpret_cast<float2*>(p.T));
     OPSEC_CUDA(cudaGetLastError());
-    // Vectors per warp.  One while the warps do not fill the chip four times over (10 blocks of 555^2,
+    // Vectors per warp (times before the packed arithmetic; since, the ones taken: 10 blocks of 555^2 0.53,
+    // 34 of 512^2 0.92, one of 1728^2 2.6, of 3150^2 11.7 ms, and the order of the choices is the same).
+    // One while the warps do not fill the chip four times over (10 blocks of 555^2,
     // 1,390 vectors: 0.68 ms, two 0.84, four 1.07); two beyond (34 of 1024^2: 10.2 ms, four 13.4: a
     // warp's 40 KB leave five warps an SM); four where their rows still leave nine warps an SM and
     // reading the reflectors half as often counts (34 of 512^2, 4,351 vectors: 1.10 ms, two 1.43, one
