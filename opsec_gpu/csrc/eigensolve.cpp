@@ -341,7 +341,7 @@ int eigensolve(opsec_gpu* c, int ncells, const opsec_cell* cells, int M, bool wa
         d_nba.alloc(H);
         OPSEC_CUDA(cudaMemcpyAsync(d_nba.p, nba.data(), sizeof(double) * H, cudaMemcpyHostToDevice, c->stream));
         c->S.alloc((size_t)nblk * Hb * Hb);
-        launch_azimuthal_blocks(ks, c->Q.p, d_nba.p, nm, npar, c->S.p, c->stream, &c->launches);
+        launch_azimuthal_blocks(ks, c->Q.p, d_nba.p, nm, npar, 1, c->S.p, c->stream, &c->launches);
         c->W.alloc((size_t)nblk * Hb);
         c->info.alloc(nblk);
         std::vector<int> own_kc;
@@ -349,7 +349,7 @@ int eigensolve(opsec_gpu* c, int ncells, const opsec_cell* cells, int M, bool wa
         const bool own_done = own_try && own_block_eigensolve(c, Hb, nblk, npar, Nphi, M, own_kc);
         if (!own_done) {
             if (own_try)  // the reduction overwrote the blocks: rebuild them for the library solver
-                launch_azimuthal_blocks(ks, c->Q.p, d_nba.p, nm, npar, c->S.p, c->stream, &c->launches);
+                launch_azimuthal_blocks(ks, c->Q.p, d_nba.p, nm, npar, 1, c->S.p, c->stream, &c->launches);
             int lwork = 0;
             solver_check(cusolverDnDsyevd_bufferSize(c->solver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, Hb,
                                                      c->S.p, Hb, c->W.p, &lwork),
@@ -444,7 +444,7 @@ int eigensolve(opsec_gpu* c, int ncells, const opsec_cell* cells, int M, bool wa
                 cusolverDnDestroyParams(prm);
                 batched_done = st == CUSOLVER_STATUS_SUCCESS;
                 if (!batched_done)  // the blocks may have been partly overwritten: rebuild them
-                    launch_azimuthal_blocks(ks, c->Q.p, d_nba.p, nm, npar, c->S.p, c->stream, &c->launches);
+                    launch_azimuthal_blocks(ks, c->Q.p, d_nba.p, nm, npar, 1, c->S.p, c->stream, &c->launches);
             }
             // the block eigenproblems are independent: spread them over side streams
             const int ns = batched_done ? 0 : std::min(nblk, c->az_streams);

@@ -169,11 +169,12 @@ void launch_signal_block(const KeySpace& ks, const CellKeyInfo& ci, const double
                          int ncols, const int* cols, double* s, int lld, cudaStream_t st, long long* launches);
 
 // Azimuthal blocks of a full-sky S: Sm[m][ha][hb] = D_ha D_hb sum_df Q(ha,hb,df) cos(2 pi m df/Nphi)
-// npar = 2 splits each order into its mu-even and mu-odd blocks (half size); block b = m npar + parity
+// npar = 2 splits each order into its mu-even and mu-odd blocks (half size); block b = m npar + parity.
+// nbands consecutive tables of Qtab, their blocks one band after the other.
 void launch_azimuthal_blocks(const KeySpace& ks, const double* Qtab, const double* nbar_arc, int nm, int npar,
-                             double* Sm, cudaStream_t st, long long* launches);
+                             int nbands, double* Sm, cudaStream_t st, long long* launches);
 void launch_azimuthal_blocks(const KeySpace& ks, const double* Qtab, const double* nbar_arc, int nm, int npar,
-                             float* Sm, cudaStream_t st, long long* launches, bool tiled = true);
+                             int nbands, float* Sm, cudaStream_t st, long long* launches, bool tiled = true);
 // Block eigenvector columns (m, idx) gathered into Ucat[col][h]
 void launch_gather_block_vectors(int H, int ncol, const int* col_m, const int* col_idx, const double* U, double* Ucat,
                                  cudaStream_t st, long long* launches);

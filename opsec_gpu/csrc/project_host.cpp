@@ -89,14 +89,14 @@ T* az_blocks(opsec_gpu* c, const AzPlan& a) {
             OPSEC_CUDA(cudaStreamWaitEvent(c->stream, c->band_ev[1], 0));
             c->band_pending = false;
         }
-        for (int p = (pre && p0 == 0) ? p0 + np : p0; p < p0 + np; p++) {
-            if (g_clock) g_clock->begin("azimuthal_transform", c->stream, 2.0 * nblk * (double)H * H * c->ks.nf);
+        if (!(pre && p0 == 0)) {
+            const double* Qp = c->Q.p + (size_t)(1 + p0) * c->ks.nkeys;
+            if (g_clock) g_clock->begin("azimuthal_transform", c->stream, 2.0 * nblk * (double)H * H * c->ks.nf * np);
             if constexpr (std::is_same<T, float>::value)
-                launch_azimuthal_blocks(c->ks, c->Q.p + (size_t)(1 + p) * c->ks.nkeys, a.nbar_arc, a.nm, a.npar,
-                                        Sb + (size_t)(p - p0) * nS, c->stream, &c->launches, c->az_tiled != 0);
+                launch_azimuthal_blocks(c->ks, Qp, a.nbar_arc, a.nm, a.npar, np, Sb, c->stream, &c->launches,
+                                        c->az_tiled != 0);
             else
-                launch_azimuthal_blocks(c->ks, c->Q.p + (size_t)(1 + p) * c->ks.nkeys, a.nbar_arc, a.nm, a.npar,
-                                        Sb + (size_t)(p - p0) * nS, c->stream, &c->launches);
+                launch_azimuthal_blocks(c->ks, Qp, a.nbar_arc, a.nm, a.npar, np, Sb, c->stream, &c->launches);
             if (g_clock) g_clock->end(c->stream);
         }
         if (g_clock) g_clock->begin("azimuthal_gemm", c->stream, a.flops * np);
@@ -293,12 +293,10 @@ void prefetch_band_blocks(opsec_gpu* c, int ncells, const opsec_cell* cells) {
     OPSEC_CUDA(cudaEventRecord(c->band_ev[0], c->stream));
     OPSEC_CUDA(cudaStreamWaitEvent(c->band_stream, c->band_ev[0], 0));
     float* Sb = reinterpret_cast<float*>(c->azSb.p);
-    for (int p = 0; p < np; p++) {
-        if (g_clock) g_clock->begin("azimuthal_transform", c->band_stream, 2.0 * nblk * (double)H * H * ks.nf);
-        launch_azimuthal_blocks(ks, c->Q.p + (size_t)(1 + p) * ks.nkeys, c->nba_band.p, nm, npar, Sb + (size_t)p * nS,
-                                c->band_stream, &c->launches, c->az_tiled != 0);
-        if (g_clock) g_clock->end(c->band_stream);
-    }
+    if (g_clock) g_clock->begin("azimuthal_transform", c->band_stream, 2.0 * nblk * (double)H * H * ks.nf * np);
+    launch_azimuthal_blocks(ks, c->Q.p + (size_t)ks.nkeys, c->nba_band.p, nm, npar, np, Sb, c->band_stream, &c->launches,
+                            c->az_tiled != 0);
+    if (g_clock) g_clock->end(c->band_stream);
     OPSEC_CUDA(cudaEventRecord(c->band_ev[1], c->band_stream));
     c->band_pending = true;
     c->band_batch = np;

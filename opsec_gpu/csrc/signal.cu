@@ -346,6 +346,8 @@ template <int NFM>
 __global__ void azimuthal_blocks_f32_kernel(KeySpace ks, const double* Q, const double* nbar_arc, int nm, int npar,
                                             float* Sm) {
     extern __shared__ float cwf[];  // [nm][NFM], zero past nf
+    Q += blockIdx.z * (size_t)ks.nkeys;
+    Sm += blockIdx.z * ((size_t)nm * npar * (ks.H / npar) * (ks.H / npar));
     const int H = ks.H, Nphi = ks.N3, nf = ks.nf, Nmu = ks.N2;
     for (int t = threadIdx.x; t < nm * NFM; t += blockDim.x) {
         const int m = t / NFM, df = t % NFM;
@@ -400,7 +402,9 @@ template <int NFM>
 __global__ void __launch_bounds__(256) azimuthal_blocks_tiled_kernel(KeySpace ks, const double* Q,
                                                                      const double* nbar_arc, int nm, int npar,
                                                                      float* Sm) {
-    // tile (blockIdx.x, blockIdx.y); tiles entirely below the diagonal have nothing to do
+    // tile (blockIdx.x, blockIdx.y) of band blockIdx.z; tiles entirely below the diagonal have nothing to do
+    Q += blockIdx.z * (size_t)ks.nkeys;
+    Sm += blockIdx.z * ((size_t)nm * npar * (ks.H / npar) * (ks.H / npar));
     const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY;
     if (y0 + kTY - 1 < x0) return;
     extern __shared__ __align__(16) float tsm[];
@@ -497,42 +501,47 @@ __global__ void __launch_bounds__(256) azimuthal_blocks_tiled_kernel(KeySpace ks
     }
 }
 
+// Bands share launches up to kBandCtas CTAs: a small survey's band is a few CTAs (8 at 2,048 cells, 22 us a
+// launch, 20 of them longer than the eigensolve beside which they run).  Larger launches would hold the SMs
+// that the eigensolve's clusters wait for.
+constexpr int kBandCtas = 304;
 template <int NFM>
-void launch_azimuthal_f32(const KeySpace& ks, const double* Q, const double* nbar_arc, int nm, int npar, float* Sm,
-                          cudaStream_t st, bool tiled) {
+void launch_azimuthal_f32(const KeySpace& ks, const double* Q, const double* nbar_arc, int nm, int npar, int nbands,
+                          float* Sm, cudaStream_t st, bool tiled, long long* l) {
     const int Hb = ks.H / npar;
-    if (tiled) {
-        const size_t smem = sizeof(float) * ((size_t)nm * NFM + 2 * (size_t)kTX * kTY * NFM + 2 * kTY * (kTX + 1));
-        OPSEC_CUDA(cudaFuncSetAttribute(azimuthal_blocks_tiled_kernel<NFM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
-        const dim3 grid((unsigned)((Hb + kTX - 1) / kTX), (unsigned)((Hb + kTY - 1) / kTY));
-        azimuthal_blocks_tiled_kernel<NFM><<<grid, 256, smem, st>>>(ks, Q, nbar_arc, nm, npar, Sm);
-        return;
-    }
-    const size_t smem = sizeof(float) * (size_t)nm * NFM;
-    OPSEC_CUDA(cudaFuncSetAttribute(azimuthal_blocks_f32_kernel<NFM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    max_dynamic_smem((const void*)azimuthal_blocks_f32_kernel<NFM>)));
     const long long HH = (long long)Hb * Hb;
-    long long gx = (HH + 255) / 256;
-    if (gx > 65535) gx = 65535;
-    azimuthal_blocks_f32_kernel<NFM><<<(unsigned)gx, 256, smem, st>>>(ks, Q, nbar_arc, nm, npar, Sm);
+    const size_t nS = (size_t)nm * npar * HH;
+    size_t smem = sizeof(float) * (size_t)nm * NFM;
+    dim3 grid((unsigned)std::min<long long>((HH + 255) / 256, 65535));
+    auto k = azimuthal_blocks_f32_kernel<NFM>;
+    if (tiled) {
+        smem += sizeof(float) * (2 * (size_t)kTX * kTY * NFM + 2 * kTY * (kTX + 1));
+        grid = dim3((unsigned)((Hb + kTX - 1) / kTX), (unsigned)((Hb + kTY - 1) / kTY));
+        k = azimuthal_blocks_tiled_kernel<NFM>;
+    }
+    OPSEC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem((const void*)k)));
+    const int per = std::max(1, (int)(kBandCtas / ((long long)grid.x * grid.y)));
+    for (int p = 0; p < nbands; p += per) {
+        grid.z = (unsigned)std::min(per, nbands - p);
+        k<<<grid, 256, smem, st>>>(ks, Q + (size_t)p * ks.nkeys, nbar_arc, nm, npar, Sm + (size_t)p * nS);
+        OPSEC_CUDA(cudaGetLastError());
+        ++*l;
+    }
 }
 
 template <typename T>
-void launch_azimuthal_blocks_t(const KeySpace& ks, const double* Q, const double* nbar_arc, int nm, int npar, T* Sm,
-                               cudaStream_t st, long long* l, bool tiled = false) {
+void launch_azimuthal_blocks_t(const KeySpace& ks, const double* Q, const double* nbar_arc, int nm, int npar, int nbands,
+                               T* Sm, cudaStream_t st, long long* l, bool tiled = false) {
     if (npar != 1 && !(npar == 2 && ks.N2 % 2 == 0)) fail(OPSEC_ERR_ARG, "parity split needs an even mu grid");
     if (!ks.fold) fail(OPSEC_ERR_CONFIG, "azimuthal blocks need a full-sky grid");
     if constexpr (std::is_same<T, float>::value) {
         if (ks.nf <= 33) {
             if (ks.nf <= 9)
-                launch_azimuthal_f32<9>(ks, Q, nbar_arc, nm, npar, Sm, st, tiled);
+                launch_azimuthal_f32<9>(ks, Q, nbar_arc, nm, npar, nbands, Sm, st, tiled, l);
             else if (ks.nf <= 17)
-                launch_azimuthal_f32<17>(ks, Q, nbar_arc, nm, npar, Sm, st, tiled);
+                launch_azimuthal_f32<17>(ks, Q, nbar_arc, nm, npar, nbands, Sm, st, tiled, l);
             else
-                launch_azimuthal_f32<33>(ks, Q, nbar_arc, nm, npar, Sm, st, tiled);
-            OPSEC_CUDA(cudaGetLastError());
-            ++*l;
+                launch_azimuthal_f32<33>(ks, Q, nbar_arc, nm, npar, nbands, Sm, st, tiled, l);
             return;
         }
     }
@@ -543,19 +552,24 @@ void launch_azimuthal_blocks_t(const KeySpace& ks, const double* Q, const double
     const int gy = nm < 8 ? nm : 8;
     long long gx = (HH + 255) / 256;
     if (gx > 4096) gx = 4096;
-    azimuthal_blocks_kernel<T><<<dim3((unsigned)gx, gy), 256, smem, st>>>(ks, Q, nbar_arc, nm, npar, Sm);
-    OPSEC_CUDA(cudaGetLastError());
-    ++*l;
+    for (int p = 0; p < nbands; p++) {
+        azimuthal_blocks_kernel<T><<<dim3((unsigned)gx, gy), 256, smem, st>>>(
+            ks, Q + (size_t)p * ks.nkeys, nbar_arc, nm, npar, Sm + (size_t)p * nm * npar * HH);
+        OPSEC_CUDA(cudaGetLastError());
+        ++*l;
+    }
 }
 
-void launch_azimuthal_blocks(const KeySpace& ks, const double* Q, const double* nbar_arc, int nm, int npar, double* Sm,
+void launch_azimuthal_blocks(const KeySpace& ks, const double* Q, const double* nbar_arc, int nm, int npar, int nbands,
+                             double* Sm,
                              cudaStream_t st, long long* l) {
-    launch_azimuthal_blocks_t(ks, Q, nbar_arc, nm, npar, Sm, st, l);
+    launch_azimuthal_blocks_t(ks, Q, nbar_arc, nm, npar, nbands, Sm, st, l);
 }
 
-void launch_azimuthal_blocks(const KeySpace& ks, const double* Q, const double* nbar_arc, int nm, int npar, float* Sm,
+void launch_azimuthal_blocks(const KeySpace& ks, const double* Q, const double* nbar_arc, int nm, int npar, int nbands,
+                             float* Sm,
                              cudaStream_t st, long long* l, bool tiled) {
-    launch_azimuthal_blocks_t(ks, Q, nbar_arc, nm, npar, Sm, st, l, tiled);
+    launch_azimuthal_blocks_t(ks, Q, nbar_arc, nm, npar, nbands, Sm, st, l, tiled);
 }
 
 template <typename T>
