@@ -220,14 +220,14 @@ def tensor_roofline(s1, bf16, peak_kind):
 # Lane instructions the spherical far-key window kernel executes per algorithmic point pair (the
 # 4096 Gauss-point pairs of a key; the phi-node mirror symmetry evaluates 10 of every 16),
 # everything included (pair loop, histograms, dot products, key decode), from one ncu capture on
-# the inner half of the 32k-cell shell (profiles/cubature_far_sph_c2inner.md: 1.0759e10 warp
+# the inner half of the 32k-cell shell (profiles/cubature_far_sph_c2inner.md: 9.5003e9 warp
 # instructions x 32 lanes over 1,118,464 keys x 4096 pairs).
-FAR_OPS_PER_PAIR = 1.0758645e10 * 32 / (1118464 * 4096)
+FAR_OPS_PER_PAIR = 9.500310713e9 * 32 / (1118464 * 4096)
 
 # DRAM bytes (read + written) per canonical key of the spherical window kernel, from the same
-# capture (101.5 MB + 376.8 MB over 1,118,464 keys); the kernel's traffic grows with the keys it
+# capture (104.5 MB + 380.1 MB over 1,118,464 keys); the kernel's traffic grows with the keys it
 # integrates (Q written per key and table), so a launch's traffic is this x its keys.
-FAR_TRAFFIC_PER_KEY = (101.491968e6 + 376.818944e6) / 1118464
+FAR_TRAFFIC_PER_KEY = (104.501504e6 + 380.082432e6) / 1118464
 
 
 def roofline(stats, clk, hbm, bf16, peak_kind, ntab):
@@ -259,7 +259,7 @@ def roofline(stats, clk, hbm, bf16, peak_kind, ntab):
                 "achieved": iach, "peak": ipeak, "unit": "G point pairs/s", "frac": iach / ipeak,
                 "peak_kind": f"derived, not measured: 128 lane instructions/clk/SM x {nsm} SMs x {mhz:.0f} MHz "
                              f"(sampled median) / {FAR_OPS_PER_PAIR:.1f} lane instructions per point pair (ncu "
-                             f"instruction count of this kernel); ncu measured issue active 81 % of peak on the "
+                             f"instruction count of this kernel); ncu measured issue active 74 % of peak on the "
                              f"16x32x32 inner shell",
                 "algorithmic_unit": "one Gauss-point pair (all xi tables at once)",
                 "traffic": FAR_TRAFFIC_PER_KEY * keys,
