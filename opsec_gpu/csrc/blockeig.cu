@@ -20,7 +20,7 @@
 //      block norm, where separately computed vectors need not be orthogonal.
 //   6. backtransform_kernel: x = Q z by the stored reflectors, four at a time (double-FP32), written
 //      as the block's eigenvector column (ascending eigenvalue order, the layout of LAPACK's syevd):
-//      34 blocks of 512^2 1.85 -> 1.10 ms, 34 of 1024^2 16.2 -> 10.2, 10 of 555^2 1.40 -> 0.68 against
+//      34 blocks of 512^2 1.85 -> 0.92 ms, 10 of 555^2 1.40 -> 0.53 against
 //      one reflector at a time by CTAs of 16 vectors.
 #include <algorithm>
 #include <cfloat>

@@ -517,7 +517,7 @@ __global__ void transpose_tables_kernel(const float* tab32, int ntab, int nx, fl
 // four cells: lanes over the points, except for the sums of the coordinates, which keep the points' order:
 // twelve lanes, one a cell and axis.  FP64 issue bounds it (66 cycles an instruction and warp, however many
 // lanes run), so the square root is taken once a cell, of the largest square.  (One thread a cell, a square
-// root a point: 171 us whether 2,048 or 32,768 cells.)
+// root a point: 171 us whether 2,048 or 32,768 cells; now 19 us at 2,048.)
 constexpr int kSphCells = 4, kSphThreads = 64;
 __global__ void __launch_bounds__(kSphThreads) cell_sphere_kernel(const float4* pts, int np, long long ncell, float4* cen) {
     __shared__ double s_p[kSphThreads / 32][3 * kSphCells][33];
@@ -800,8 +800,9 @@ __global__ void __launch_bounds__(kPartThreads) part_scatter_kernel(long long nk
 // A warp's lanes collide in the histogram's banks and, where windows are narrow, in its bins, so a
 // key's bins are kept in as many copies (2 to 32, a power of two) as its window leaves room for,
 // 2^lg of them, copy c of bin b at word (b << lg) + c, lane l adding to copy l >> (5 - lg).  By a
-// model of the bins, wavefronts of a key's atomics against two copies: 32k-cell shell (median
-// window 73 bins) 950 -> 760, mock surveys on the 512 + 256 table (14 bins) 2,300 -> 440.
+// model of the bins, wavefronts of a key's atomics with two copies and with as many as fit: mock
+// surveys on the 512 + 256 table (median window 14 bins) 2,300 and 440, 32k-cell shell (73 bins) 950
+// and 760; copies_log2 takes more than two where that wins.
 // (64-bit integer shared atomics instead: cubature 90 ms against 66 ms at 32k
 // cells.)
 // (FP32 shared-memory atomics were slower -- the counters showed them retried
@@ -834,7 +835,8 @@ __device__ __forceinline__ void add_fixed(int* hqa, int* hqb, int b, float x, fl
 // log2 of a key's copies: one a lane where that fits, two for windows wider than kNarrow bins, where
 // summing more copies and shifting by a variable cost more than the atomics gain (one rule for all
 // windows: 32k-cell shell's build 60.5 ms, with two copies beyond 48 bins 57.3 ms; 16 mock surveys on
-// narrow windows 293 ms with two, 242 ms with up to 32)
+// narrow windows 293 ms with two, 242 ms with up to 32; four for up to 192 bins, as a constant of the
+// packed loop: cubature at 32k cells 41.9 -> 42.6 ms, 65k 182 -> 185)
 constexpr int kNarrow = 48;
 __device__ __forceinline__ int copies_log2(int Wkey, int n) {
     int lg = 1;

@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kMaxThreads) fisher_kernel(Src src, int nb, co
 }
 
 // Fixed-order reduction of the per-CTA partials into F (full), f, q: one warp an output, lanes over the
-// partials, then a shuffle tree (a thread an output chained 304 loads and additions: 127 us for 20 bands).
+// partials, then a shuffle tree (a thread an output chained 304 loads and additions: 127 us for 20 bands, now 7).
 __global__ void fisher_reduce_kernel(int nb, int nblocks, const double* partial, double* out) {
     const int nout = nb * (nb + 1) / 2 + 2 * nb, lane = threadIdx.x & 31;
     const int o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -356,7 +356,7 @@ __global__ void fisher_reduce_kernel(int nb, int nblocks, const double* partial,
 // largest bits of |A|, ties to the lower row; a NaN's are larger still and fail the test) and its
 // reciprocal, one thread a column swaps and scales the two rows, all eliminate the columns still to be
 // read: those of A beyond c, all of X.  (With the pivot sought by one thread and every column eliminated
-// the epilogue of 20 bands took 57 us.)
+// the epilogue of 20 bands took 57 us, now 43: what is left is FP64 issue on one SM.)
 __device__ bool gj_inverse(int n, double* A, double* X, int* piv_row) {
     __shared__ int bad;
     __shared__ double inv;
