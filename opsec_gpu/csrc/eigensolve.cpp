@@ -178,7 +178,7 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
         if (st[b]) {
             c->warning = "block eigensolver check " + std::to_string(st[b]) + " failed on block " +
                          std::to_string(b) + "; solved by cuSOLVER instead";
-            c->eig_stats[1] = 0.0;
+            c->eig_stats[1] = c->eig_stats[4] = 0.0;
             return false;
         }
     return true;
@@ -216,7 +216,6 @@ bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
     int kc = M;
     while (kc < n && w[n - 1 - kc] >= cut) kc++;
     kc = std::min(n, std::max(kc, M + std::max(32, M / 8)));  // a margin below the cut for the polish
-    c->eig_stats[4] = kc;
     const int hi[3] = {kc, 0, 0};
     c->bev_i.alloc(3);
     OPSEC_CUDA(cudaMemcpyAsync(c->bev_i.p, hi, sizeof hi, cudaMemcpyHostToDevice, c->stream));
@@ -275,6 +274,7 @@ bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
         c->warning = "dense eigensolver check " + std::to_string(st) + " failed; solved by cuSOLVER instead";
         return false;
     }
+    c->eig_stats[4] = kc;  // only now: the library's solve leaves it 0
     std::stable_sort(ev.begin(), ev.end(), std::greater<double>());  // refined one by one: equal to rounding
     OPSEC_CUDA(cudaMemcpyAsync(c->evals.p, ev.data(), sizeof(double) * M, cudaMemcpyHostToDevice, c->stream));
     sync(c);
