@@ -1,6 +1,7 @@
 // eigensolve.cpp -- the KL eigensolve (klt.cpp:173-248): azimuthal blocks by the hand-written
 // block eigensolver or cuSOLVER, dense cuSOLVER syevdx, or the iterative solver.
 #include "context.h"
+#include "symmetry.h"
 
 bool azimuthal_ok(opsec_gpu* c, int ncells, const opsec_cell* cells) {
     const Geometry& g = c->geo;
@@ -56,7 +57,8 @@ void drop_eig_graph(opsec_gpu* c) {
 // kernels, open box with all else equal, top 29 %: 512 cells 14.9 -> 4.3 ms, 990 31.5 -> 10.4, 1,728
 // 67.7 -> 30.4, 2,730 156.6 -> 85.  Smaller ones gain as much (294 cells 9.0 -> 2.3 ms) but stay with
 // cuSOLVER: their C_p, rounded to FP32 in few modes, moves q by up to 1e-9 with any other rounding
-// of the vectors.  So do exactly degenerate S (exchange_symmetric), whose basis rounding picks.
+// of the vectors.  So do exactly degenerate S (symmetry.h), whose basis rounding picks and two of whose
+// separately computed vectors may come out parallel.
 constexpr int kOwnDenseMin = 512;
 
 // Surveys whose Fisher matrix moves by over 1e-9 with the eigensolver's rounding (blockeig_small.cu):
@@ -290,32 +292,6 @@ void forget_device_state(opsec_gpu* c) {
     if (!c->xi64.p || !c->xi32.p) c->tables_ok = false;
     c->az_valid = false;
     drop_eig_graph(c);
-}
-
-// True when a Cartesian survey looks the same with two of its axes exchanged (equal cell counts and
-// sizes, and Nbar): S then has exactly degenerate eigenvalues.  Only a full grid can.
-bool exchange_symmetric(const opsec_gpu* c, int ncells, const opsec_cell* cells) {
-    const Geometry& g = c->geo;
-    const int* n = g.n;
-    if (g.coordsys != 1 || (long long)ncells != (long long)n[0] * n[1] * n[2]) return false;
-    std::vector<double> nb(ncells, -1.0);
-    auto at = [&](int x, int y, int z) { return ((size_t)x * n[1] + y) * n[2] + z; };
-    for (int a = 0; a < ncells; a++) nb[at(cells[a].d1, cells[a].d2, cells[a].d3)] = cells[a].Nbar;
-    auto same = [](double x, double y) { return std::fabs(x - y) <= 1e-9 * std::max(std::fabs(x), std::fabs(y)); };
-    for (int p = 0; p < 3; p++) {
-        const int q = (p + 1) % 3;
-        if (n[p] != n[q] || !same((g.b[2 * p + 1] - g.b[2 * p]) / n[p], (g.b[2 * q + 1] - g.b[2 * q]) / n[q])) continue;
-        bool sym = true;
-        for (int x = 0; x < n[0] && sym; x++)
-            for (int y = 0; y < n[1] && sym; y++)
-                for (int z = 0; z < n[2] && sym; z++) {
-                    int d[3] = {x, y, z};
-                    std::swap(d[p], d[q]);
-                    sym = same(nb[at(x, y, z)], nb[at(d[0], d[1], d[2])]);
-                }
-        if (sym) return true;
-    }
-    return false;
 }
 
 int eigensolve(opsec_gpu* c, int ncells, const opsec_cell* cells, int M, bool want_modes) {
@@ -560,9 +536,11 @@ int eigensolve(opsec_gpu* c, int ncells, const opsec_cell* cells, int M, bool wa
         return M;
     }
     std::fill(c->eig_stats, c->eig_stats + 10, 0.0);
-    if (c->eig_solver == "auto" && c->az_own && N >= kOwnDenseMin && tridiag_chip_supported(N) && !exchange_symmetric(c, ncells, cells) &&
-        own_dense_eigensolve(c, N, M))
-        return M;
+    if (c->eig_solver == "auto" && c->az_own && N >= kOwnDenseMin && tridiag_chip_supported(N)) {
+        const Geometry& g = c->geo;
+        if (!Symmetry(g.coordsys, g.b, g.n, g.L, g.full_sky(), ncells, cells).forces_degeneracy() && own_dense_eigensolve(c, N, M))
+            return M;
+    }
     c->W.alloc(N);
     c->info.alloc(1);
     // the 64-bit interface: the 32-bit one's workspace count overflows from N ~ 23,000 on
