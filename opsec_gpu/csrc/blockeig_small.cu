@@ -73,15 +73,24 @@ __device__ df cta_sum_df(df x, float2* red) {
 // with v[c+1] = 1 maps col[c+1..n) onto beta e_{c+1}.  The sum of squares and v in double-FP32,
 // the scalars in FP64 by warp 0 alone (the FP64 pipe issues at 1/64 of the FP32 rate: once per
 // CTA, not in every warp).  sc: tau, beta (FP64); sc2: tau, 1/(x0 - beta) as (hi, lo) pairs.
-// Every CTA of the cluster computes it from the same data and gets the same bits.
-__device__ void householder_df(int n, int c, const float2* col, float2* v, double* sc, float2* sc2, float2* red) {
+// Every CTA of the cluster computes it from the same data and gets the same bits.  A column whose squares
+// would underflow FP32 is taken times 2^80 (in place), as in tridiag.cu.
+__device__ void householder_df(int n, int c, float2* col, float2* v, double* sc, float2* sc2, float2* red) {
     const int t = threadIdx.x;
-    df s{0.f, 0.f};
-    for (int i = c + 2 + t; i < n; i += blockDim.x) {
-        const df x = df_unpack(col[i]);
-        s = df_fma(s, x, x);
+    df s2;
+    int k = 0;
+    for (;; k++) {
+        df s{0.f, 0.f};
+        for (int i = c + 2 + t; i < n; i += blockDim.x) {
+            const df x = df_unpack(col[i]);
+            s = df_fma(s, x, x);
+        }
+        s2 = cta_sum_df(s, red);
+        if (k == 2 || !(fmaf(col[c + 1].x, col[c + 1].x, s2.h) < 0x1p-80f)) break;
+        __syncthreads();  // every thread has read col[c + 1]
+        for (int i = c + 1 + t; i < n; i += blockDim.x) col[i] = make_float2(col[i].x * 0x1p80f, col[i].y * 0x1p80f);
+        __syncthreads();
     }
-    const df s2 = cta_sum_df(s, red);
     if (t < 32) {
         const double x0 = df_to(df_unpack(col[c + 1])), s2d = df_to(s2);
         double tau = 0.0, beta = x0, scal = 0.0;
@@ -93,7 +102,7 @@ __device__ void householder_df(int n, int c, const float2* col, float2* v, doubl
         }
         if (t == 0) {
             sc[0] = tau;
-            sc[1] = beta;
+            sc[1] = k ? ldexp(beta, -80 * k) : beta;
             sc2[0] = df_pack(df_from(tau));
             sc2[1] = df_pack(df_from(scal));
         }
@@ -107,10 +116,11 @@ __device__ void householder_df(int n, int c, const float2* col, float2* v, doubl
 // One fused pass over the columns j in [j0, n) of the lower triangle, in double-FP32 (the
 // FP64 pipe is the bound otherwise): a -= v_i w_j + w_i v_j (when upd), then the partial
 // products p += A vn into this warp's row of pw (when sym).  conv: the column still holds FP64
-// values (the first pass), which are read as doubles and written back as (hi, lo) pairs in the
-// same 8 bytes.
+// values (the first pass), which are read as doubles and written back, times the block's unit, as
+// (hi, lo) pairs in the same 8 bytes.
 __device__ void fused_pass(int n, int j0, double* __restrict__ A, const float2* vk, const float2* wk,
-                           const float2* vn, float2* pw, bool upd, bool sym, bool conv, int gwarp, int nwarps) {
+                           const float2* vn, float2* pw, bool upd, bool sym, bool conv, double unit, int gwarp,
+                           int nwarps) {
     const int lane = threadIdx.x & 31;
     const int L = n - j0;
     float2* A2 = reinterpret_cast<float2*>(A);
@@ -125,7 +135,7 @@ __device__ void fused_pass(int n, int j0, double* __restrict__ A, const float2* 
         const df vnj = sym ? df_unpack(vn[j]) : df{0.f, 0.f};
         df cacc{0.f, 0.f};
         for (int i = j + lane; i < n; i += 32) {
-            df a = conv ? df_from(A[cj + i]) : df_unpack(A2[cj + i]);
+            df a = conv ? df_from(A[cj + i] * unit) : df_unpack(A2[cj + i]);
             if (upd) {
                 a = df_fms(a, df_unpack(vk[i]), wkj);
                 a = df_fms(a, df_unpack(wk[i]), vkj);
@@ -162,7 +172,7 @@ __device__ void reduce_warp_rows(int n, int i0, const float2* pw, float2* out) {
 // (FP64, one warp): the O(n^2) fused pass and the O(n) work of each step (p = A v from the
 // cluster, w, the pivot column, v).
 __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kTT, 1)
-tridiag_kernel(int n, double* __restrict__ Aall, double* __restrict__ Vall, double* __restrict__ tau,
+tridiag_kernel(int n, double* __restrict__ Aall, const double2* __restrict__ unit, double* __restrict__ Vall, double* __restrict__ tau,
                double* __restrict__ dg, double* __restrict__ eg) {
     extern __shared__ double sm[];
     cg::cluster_group cluster = cg::this_cluster();
@@ -185,7 +195,7 @@ tridiag_kernel(int n, double* __restrict__ Aall, double* __restrict__ Vall, doub
     const float2* A2 = reinterpret_cast<const float2*>(A);
 
     // pivot column 0 and the first reflector
-    for (int i = t; i < n; i += kTT) col2[i] = df_pack(df_from(A[i]));
+    for (int i = t; i < n; i += kTT) col2[i] = df_pack(df_from(A[i] * unit[b].x));
     __syncthreads();
     householder_df(n, 0, col2, vn2, sc, sc2, red);
     __syncthreads();
@@ -199,7 +209,7 @@ tridiag_kernel(int n, double* __restrict__ Aall, double* __restrict__ Vall, doub
     }
     for (int i = 1 + (t & 31); i < n; i += 32) pw_mine[i] = make_float2(0.f, 0.f);
     __syncthreads();
-    fused_pass(n, 1, A, vk2, wk2, vn2, pw_mine, false, true, true, gwarp, nwarps);
+    fused_pass(n, 1, A, vk2, wk2, vn2, pw_mine, false, true, true, unit[b].x, gwarp, nwarps);
     __syncthreads();
     reduce_warp_rows(n, 1, pw, buf);  // parity 0
     cluster.sync();
@@ -251,7 +261,7 @@ tridiag_kernel(int n, double* __restrict__ Aall, double* __restrict__ Vall, doub
         if (sym)
             for (int i = c1 + 1 + (t & 31); i < n; i += 32) pw_mine[i] = make_float2(0.f, 0.f);
         __syncthreads();
-        fused_pass(n, c1 + 1, A, vk2, wk2, vn2, pw_mine, true, sym, false, gwarp, nwarps);
+        fused_pass(n, c1 + 1, A, vk2, wk2, vn2, pw_mine, true, sym, false, 1.0, gwarp, nwarps);
         __syncthreads();
         if (sym) reduce_warp_rows(n, c1 + 1, pw, buf + (size_t)(c1 & 1) * n);
         cluster.sync();
@@ -260,6 +270,13 @@ tridiag_kernel(int n, double* __restrict__ Aall, double* __restrict__ Vall, doub
         dg[(size_t)b * n + n - 1] = df_to(df_unpack(A2[(size_t)(n - 1) * n + n - 1]));
         eg[(size_t)b * n + n - 1] = 0.0;
         tau[(size_t)b * n + n - 1] = 0.0;
+    }
+    if (rank == 0) {  // T back in A's own units
+        __syncthreads();
+        for (int i = t; i < n; i += kTT) {
+            dg[(size_t)b * n + i] *= unit[b].y;
+            eg[(size_t)b * n + i] *= unit[b].y;
+        }
     }
 }
 
@@ -637,12 +654,12 @@ __global__ void __launch_bounds__(kBT) backtransform_kernel(VecArgs a, const dou
 
 static size_t small_tridiag_smem(int n) { return sizeof(double) * ((size_t)(6 + kTW) * n + 48); }
 
-void launch_small_tridiag(int n, int nblk, double* A, double* V, double* tau, double* dg, double* eg,
+void launch_small_tridiag(int n, int nblk, double* A, const double* unit, double* V, double* tau, double* dg, double* eg,
                              cudaStream_t s, long long* launches) {
     const size_t smem = small_tridiag_smem(n);
     OPSEC_CUDA(cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     max_dynamic_smem((const void*)tridiag_kernel)));
-    tridiag_kernel<<<nblk * kCl, kTT, smem, s>>>(n, A, V, tau, dg, eg);
+    tridiag_kernel<<<nblk * kCl, kTT, smem, s>>>(n, A, reinterpret_cast<const double2*>(unit), V, tau, dg, eg);
     OPSEC_CUDA(cudaGetLastError());
     ++*launches;
 }

@@ -73,8 +73,9 @@ bool small_survey(int npar, long long cells) { return cells < 1024 || (npar == 1
 bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int M, std::vector<int>& kc) {
     const size_t nn = (size_t)n * n;
     c->bev_V.alloc(nblk * blockeig_reflector_doubles(n));
-    c->bev_T.alloc((size_t)nblk * (3 * n + 1));
-    double* tau = c->bev_T.p;
+    c->bev_T.alloc((size_t)nblk * (3 * n + 3));
+    double* unit = c->bev_T.p;  // pairs: 16-byte aligned
+    double* tau = unit + (size_t)2 * nblk;
     double* dg = tau + (size_t)nblk * n;
     double* eg = dg + (size_t)nblk * n;
     double* scale = eg + (size_t)nblk * n;
@@ -82,12 +83,13 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     c->bev_err.alloc(1);
     OPSEC_CUDA(cudaMemsetAsync(c->bev_err.p, 0, sizeof(int), c->stream));
     if (!small) c->bev_D.alloc(tridiag_work_bytes(n, nblk));
+    launch_block_unit(n, nblk, c->S.p, unit, c->stream, &c->launches);
     if (g_clock) g_clock->begin("blockeig_tridiag", c->stream, 4.0 / 3.0 * n * nn * nblk);
     if (small)
-        launch_small_tridiag(n, nblk, c->S.p, c->bev_V.p, tau, dg, eg, c->stream, &c->launches);
+        launch_small_tridiag(n, nblk, c->S.p, unit, c->bev_V.p, tau, dg, eg, c->stream, &c->launches);
     else
-        launch_tridiag(n, nblk, false, c->S.p, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
-                       &c->launches);
+        launch_tridiag(n, nblk, false, c->S.p, unit, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait,
+                       c->stream, &c->launches);
     if (g_clock) g_clock->end(c->stream);
     if (small)
         launch_small_spectrum(n, nblk, dg, eg, c->W.p, scale, c->stream, &c->launches);
@@ -191,8 +193,9 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
 bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
     const size_t nn = (size_t)n * n;
     c->bev_V.alloc(blockeig_reflector_doubles(n));
-    c->bev_T.alloc((size_t)3 * n + 1);
-    double* tau = c->bev_T.p;
+    c->bev_T.alloc((size_t)3 * n + 3);
+    double* unit = c->bev_T.p;  // a pair: 16-byte aligned
+    double* tau = unit + 2;
     double* dg = tau + n;
     double* eg = dg + n;
     double* scale = eg + n;
@@ -200,8 +203,9 @@ bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
     c->bev_D.alloc(tridiag_work_bytes(n, 1));
     c->bev_err.alloc(1);
     OPSEC_CUDA(cudaMemsetAsync(c->bev_err.p, 0, sizeof(int), c->stream));
+    launch_block_unit(n, 1, c->S.p, unit, c->stream, &c->launches);
     if (g_clock) g_clock->begin("blockeig_tridiag", c->stream, 4.0 / 3.0 * n * nn);
-    launch_tridiag(n, 1, true, c->S.p, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
+    launch_tridiag(n, 1, true, c->S.p, unit, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
                    &c->launches);
     if (g_clock) g_clock->end(c->stream);
     launch_blockeig_spectrum(n, 1, dg, eg, c->W.p, scale, c->stream, &c->launches);

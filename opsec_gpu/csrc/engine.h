@@ -215,8 +215,10 @@ bool blockeig_supported(int n);
 size_t blockeig_reflector_doubles(int n);
 size_t tridiag_work_bytes(int n, int nblk);
 bool tridiag_chip_supported(int n);
-void launch_tridiag(int n, int nblk, bool chip, const double* A, double* V, double* tau, double* dg, double* eg, void* work,
-                    int* err, long long wait_cycles, cudaStream_t s, long long* launches);
+// unit: [block] (power of two, its inverse) by which the reduction scales A, from launch_block_unit
+void launch_block_unit(int n, int nblk, const double* A, double* unit, cudaStream_t s, long long* launches);
+void launch_tridiag(int n, int nblk, bool chip, const double* A, const double* unit, double* V, double* tau, double* dg,
+                    double* eg, void* work, int* err, long long wait_cycles, cudaStream_t s, long long* launches);
 void launch_blockeig_spectrum(int n, int nblk, const double* dg, const double* eg, double* w, double* scale,
                               cudaStream_t s, long long* launches);
 struct BlockEigVectors {
@@ -247,7 +249,7 @@ void launch_polish_coefficients(int k, int m, const double* G, const double* H, 
                                 cudaStream_t s, long long* launches);
 
 // The same for small surveys (blockeig_small.cu): A is overwritten.
-void launch_small_tridiag(int n, int nblk, double* A, double* V, double* tau, double* dg, double* eg, cudaStream_t s,
+void launch_small_tridiag(int n, int nblk, double* A, const double* unit, double* V, double* tau, double* dg, double* eg, cudaStream_t s,
                           long long* launches);
 void launch_small_spectrum(int n, int nblk, const double* dg, const double* eg, double* w, double* scale,
                            cudaStream_t s, long long* launches);

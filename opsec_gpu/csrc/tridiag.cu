@@ -18,6 +18,9 @@
 //   * The reflector's square root and reciprocals are double-FP32 Newton steps from the FP32
 //     hardware estimates: in FP64, at 1/64 of the FP32 rate, they were a long chain of each step.
 //   * The pass runs on packed FP32 instructions (two columns an issue slot).
+// Pairs of floats have FP32's exponent range, so a block is reduced times a power of two that brings its
+// largest diagonal entry (S is a covariance: its largest entry) to [1/2, 1), and the reflector of a column
+// whose squares would underflow is formed from the column times 2^80.
 // Bound by the FP32 pipe in the pass (44 % busy over all, with two warps a scheduler) and by the
 // step's chain of reductions (3.3 us of each step).  Against one triangle on clusters of four, with
 // partial sums and FP64 scalars: 34 blocks of 512^2 (the 32k-cell build) 8.19 -> 5.18 ms, 34 of
@@ -83,6 +86,7 @@ struct TridiagArgs {
     float4* V;         // [block][n up to whole fours][ceil(n/2)] reflector c in row c (v[c+1] = 1), two entries as (hi, hi, lo, lo), zeros
                        // from entry c & ~3 on before it and past entry n - 1
     double *tau, *dg, *eg;  // [block][n]
+    const double2* unit;    // [block] the power of two, and its inverse
     // whole-chip form: exchange of p, and the barrier between CTAs
     float2* pbuf;      // [2][n]
     unsigned* count;   // arrivals
@@ -90,20 +94,39 @@ struct TridiagArgs {
     long long wait_cycles;
 };
 
-// lower triangle of the FP64 blocks -> both triangles in double-FP32, rows padded with zeros
+// (2^-e, 2^e) of each block, 2^e > its largest |diagonal entry| >= 2^(e-1): one CTA a block
+__global__ void __launch_bounds__(256) unit_kernel(int n, const double* __restrict__ A, double2* __restrict__ unit) {
+    __shared__ double red[8];
+    const double* Ab = A + (size_t)blockIdx.x * n * n;
+    double m = 0.0;
+    for (int i = threadIdx.x; i < n; i += 256) m = fmax(m, fabs(Ab[(size_t)i * n + i]));
+#pragma unroll
+    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int w = 1; w < 8; w++) m = fmax(m, red[w]);
+    int e = 0;
+    if (m > 0.0 && isfinite(m)) frexp(m, &e);
+    e = max(-1000, min(1000, e));  // both powers are normal numbers
+    unit[blockIdx.x] = make_double2(ldexp(1.0, -e), ldexp(1.0, e));
+}
+
+// lower triangle of the FP64 blocks, times their unit -> both triangles in double-FP32, rows padded with zeros
 __global__ void __launch_bounds__(256) pairs_kernel(int n, int ld, const double* __restrict__ A,
-                                                    float* __restrict__ D) {
+                                                    const double2* __restrict__ unit, float* __restrict__ D) {
     __shared__ float2 tile[32][33];
     const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;  // rows i (the contiguous index of A), columns j
     if (i0 + 31 < j0) return;  // above the diagonal: written with its mirror image
     const double* Ab = A + (size_t)blockIdx.z * n * n;
     float* Db = D + (size_t)blockIdx.z * n * 2 * ld;
+    const double u = unit[blockIdx.z].x;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int y = ty; y < 32; y += 8) {
         const int i = i0 + tx, j = j0 + y;
         float2 v = make_float2(0.f, 0.f);
         if (i < n && j < n && i >= j) {
-            v = df_pack(df_from(Ab[(size_t)j * n + i]));
+            v = df_pack(df_from(Ab[(size_t)j * n + i] * u));
             put(Db + (size_t)j * 2 * ld, i, df_unpack(v));  // row j, column i
         }
         tile[y][tx] = v;
@@ -372,11 +395,27 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
     __syncthreads();
 
     // Reflector of the pivot column c1: x[q] is its entry c1 + t + T q (0 at c1), s this thread's share
-    // of the sum of squares below the first entry; the reflector goes to v.
+    // of the sum of squares below the first entry; the reflector goes to v.  Where the column is below
+    // 2^-40 of the block (its squares below 2^-80, whose pairs underflow) it is formed anew times 2^80,
+    // twice if need be: the reflector does not depend on the column's scale, beta does.
     df tau{0.f, 0.f};
-    auto reflect = [&](int c1, df s, const df (&x)[E], float* v) {
-        const df s2 = cta_sum<W>(s, red + 32);
-        const Reflector h = reflector(df_unpack(x0s[1]), s2);
+    auto reflect = [&](int c1, df s, df (&x)[E], float* v) {
+        df s2 = cta_sum<W>(s, red + 32), x0 = df_unpack(x0s[1]);
+        int k = 0;
+        for (; k < 2 && fmaf(x0.h, x0.h, s2.h) < 0x1p-80f; k++) {
+            __syncthreads();  // every thread has read red
+            s = df{0.f, 0.f};
+#pragma unroll
+            for (int q = 0; q < E; q++) {
+                const int i = c1 + t + T * q;
+                if (c1 + T * q >= n) break;
+                x[q] = df{x[q].h * 0x1p80f, x[q].l * 0x1p80f};
+                if (i > c1 + 1) s = df_fma(s, x[q], x[q]);
+            }
+            x0 = df{x0.h * 0x1p80f, x0.l * 0x1p80f};
+            s2 = cta_sum<W>(s, red + 32);
+        }
+        const Reflector h = reflector(x0, s2);
 #pragma unroll
         for (int q = 0; q < E; q++) {
             const int i = c1 + t + T * q;
@@ -384,7 +423,7 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
             if (i < n) put(v, i, i == c1 + 1 ? df{1.f, 0.f} : df_mul(x[q], h.scal));
         }
         if (t == 0 && rank == 0) {
-            a.eg[(size_t)b * n + c1] = df_to(h.beta);
+            a.eg[(size_t)b * n + c1] = k ? ldexp(df_to(h.beta), -80 * k) : df_to(h.beta);
             a.tau[(size_t)b * n + c1] = df_to(h.tau);
         }
         tau = h.tau;
@@ -477,9 +516,17 @@ __global__ void __launch_bounds__(T, 1) tridiag_kernel(TridiagArgs a) {
             pass(c + 2, par ^ 1, yes{}, no{});
         if (!barrier()) return;
     }
+    // T back in A's own units: not step by step, where its FP64 products (64 cycles each) are in every
+    // step's chain (2 % of a 1,728-cell box)
+    const double back = a.unit[b].y;
+    if (rank == 0)  // which wrote all but the last row
+        for (int i = t; i < n - 1; i += T) {
+            a.dg[(size_t)b * n + i] *= back;
+            a.eg[(size_t)b * n + i] *= back;
+        }
     if (rank == (n - 1) % C && t == 0) {
         // the last row is its own next pivot row: its final value is in D whichever way it lived
-        a.dg[(size_t)b * n + n - 1] = df_to(getcg(D + (size_t)(n - 1) * 2 * ld, n - 1));
+        a.dg[(size_t)b * n + n - 1] = df_to(getcg(D + (size_t)(n - 1) * 2 * ld, n - 1)) * back;
         a.eg[(size_t)b * n + n - 1] = 0.0;
         a.tau[(size_t)b * n + n - 1] = 0.0;
     }
@@ -595,8 +642,14 @@ bool tridiag_chip_supported(int n) {
            smem_base(n, 152, kChipT / 32, 2) <= (size_t)max_dynamic_smem((const void*)tridiag_kernel<kChipT, 2, 4 * kElems, true>);
 }
 
-void launch_tridiag(int n, int nblk, bool chip, const double* A, double* V, double* tau, double* dg, double* eg, void* work,
-                    int* err, long long wait_cycles, cudaStream_t s, long long* launches) {
+void launch_block_unit(int n, int nblk, const double* A, double* unit, cudaStream_t s, long long* launches) {
+    unit_kernel<<<nblk, 256, 0, s>>>(n, A, reinterpret_cast<double2*>(unit));
+    OPSEC_CUDA(cudaGetLastError());
+    ++*launches;
+}
+
+void launch_tridiag(int n, int nblk, bool chip, const double* A, const double* unit, double* V, double* tau, double* dg,
+                    double* eg, void* work, int* err, long long wait_cycles, cudaStream_t s, long long* launches) {
     TridiagArgs a{};
     a.n = n;
     a.ld = pad(n);
@@ -605,11 +658,12 @@ void launch_tridiag(int n, int nblk, bool chip, const double* A, double* V, doub
     a.tau = tau;
     a.dg = dg;
     a.eg = eg;
+    a.unit = reinterpret_cast<const double2*>(unit);
     a.pbuf = reinterpret_cast<float2*>(a.D + (size_t)nblk * n * 2 * a.ld);
     a.count = reinterpret_cast<unsigned*>(a.pbuf + 2 * (size_t)n);
     a.err = err;
     a.wait_cycles = wait_cycles;
-    pairs_kernel<<<dim3((n + 31) / 32, (n + 31) / 32, nblk), 256, 0, s>>>(n, a.ld, A, a.D);
+    pairs_kernel<<<dim3((n + 31) / 32, (n + 31) / 32, nblk), 256, 0, s>>>(n, a.ld, A, a.unit, a.D);
     OPSEC_CUDA(cudaGetLastError());
     ++*launches;
     if (chip && nblk == 1) {
