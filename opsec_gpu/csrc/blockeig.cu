@@ -178,6 +178,7 @@ struct VecArgs {
     int* KX;             // scratch: exponents of groups of rows of X, then of Y ([ceil(n/2)][ktot] each)
     double* X;           // [n][ktot] scratch: the solution from the top
     double* Y;           // [n][ktot] scratch: the solution from the bottom
+    bool polished;       // a correction of the vectors follows
     int* status;         // [nblk]: 0, or 1 when a bracket could not be confirmed, 2 when a cluster degenerated
 };
 
@@ -530,9 +531,10 @@ __device__ double gamma_df(const Team& tm, int n, const RowsDf& t, const RowsDfB
 
 // The rows of the recurrences of every block, five FP64 arrays and their double-FP32 pairs, each of
 // np = n rounded up to kGrp64 entries: Rows64's ff, fi, fb, bf, bb, then RowsDf's and RowsDfB's f, g,
-// b, f, b.
+// b, f, b; last, the distance of each approximate eigenvalue to its nearer neighbour.
+constexpr int kRowArrays = 11;
 __global__ void rows_kernel(int n, int nblk, const double* __restrict__ dg, const double* __restrict__ eg,
-                            const double* __restrict__ scale, double* __restrict__ R) {
+                            const double* __restrict__ scale, const double* __restrict__ w, double* __restrict__ R) {
     const int np = round_up(n, kGrp64);
     constexpr double kMinE = 8.673617379884035e-19;  // 2^-60
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < np * nblk; t += gridDim.x * blockDim.x) {
@@ -540,7 +542,7 @@ __global__ void rows_kernel(int n, int nblk, const double* __restrict__ dg, cons
         const double inv = 1.0 / scale[b];
         const double* dgb = dg + (size_t)b * n;
         const double* egb = eg + (size_t)b * n;
-        double* r = R + (size_t)b * 10 * np;
+        double* r = R + (size_t)b * kRowArrays * np;
         double v[5] = {1.0, 0.0, 0.0, 0.0, 0.0};  // rows past the end keep x
         if (i < n) {
             const double d = dgb[i] * inv;
@@ -551,6 +553,11 @@ __global__ void rows_kernel(int n, int nblk, const double* __restrict__ dg, cons
             v[2] = i > 0 ? -ep * v[1] : 0.0;
             v[3] = d / ep;
             v[4] = i + 1 < n ? -e / ep : 0.0;
+        }
+        if (i < n) {
+            const double* wb = w + (size_t)b * n;
+            const double down = i > 0 ? fabs(wb[i] - wb[i - 1]) : HUGE_VAL, up = i + 1 < n ? fabs(wb[i + 1] - wb[i]) : HUGE_VAL;
+            r[10 * np + i] = fmin(down, up) * inv;
         }
         float2* f = reinterpret_cast<float2*>(r + 5 * np);
         for (int q = 0; q < 5; q++) r[q * np + i] = v[q];
@@ -566,7 +573,7 @@ __global__ void rows_kernel(int n, int nblk, const double* __restrict__ dg, cons
 // (0 = largest) of block b.  An FP64 instruction takes a warp 64 cycles of its scheduler's pipe however
 // many of its lanes work, so the candidates are dealt over all schedulers of the chip, and the lanes left
 // over share a candidate: two directions of a solution, a shift of a Sturm count each, rows of the scans.
-// The FP32 estimate's bracket is confirmed by FP64 Sturm counts.  An eigenvalue alone in
+// The FP32 estimate's bracket is confirmed by double-FP32 Sturm counts.  An eigenvalue alone in
 // its bracket is refined by Rayleigh-quotient iteration on twisted factorisations (cubic
 // convergence; the iterate must stay in the bracket); an eigenvalue sharing its bracket is
 // narrowed down first.  The last twisted factorisation gives the vector.
@@ -586,7 +593,8 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
     const double sc = a.scale[b], inv = 1.0 / sc;
     const double* dgb = a.dg + (size_t)b * n;
     const double* egb = a.eg + (size_t)b * n;
-    const double* rows = R + (size_t)b * 10 * np;
+    const double* rows = R + (size_t)b * kRowArrays * np;
+    const double* gaps = rows + 10 * np;
     if (LOCAL) {
         for (int i = threadIdx.x; i < 10 * np; i += 128) rows64[i] = rows[i];
         rows = rows64;
@@ -652,8 +660,12 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
             if (!narrow(tm, count64, j, &lo, &hi, &clo, &chi)) break;
     }
     if (chi - clo == 1) {
-        // converged when the correction is below 1e-14 of the block scale (T is scaled to norm
-        // < 1), or when it stops shrinking at a level below 1e-10 (the rounding floor of gamma)
+        // Converged when the correction is below 1e-14 of the block scale (T is scaled to norm < 1) and
+        // 1e-10 of the distance to the next eigenvalue: the vector is that of the shift before the
+        // correction, off by their quotient (left to the polish where there is one: 0.12 ms at 1,728
+        // rows); or when it stops shrinking at a level below 1e-10 (the
+        // rounding floor of gamma)
+        const double tol = a.polished ? 1e-14 : fmin(1e-14, fmax(0.5 * DBL_EPSILON, 1e-10 * gaps[j]));
         double s = fmin(fmax(x, lo), hi), prev = 1.0;
         {
             // most of the way in double-FP32, at one twist row: an FP64 step costs four times as much
@@ -682,7 +694,7 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
                 const double dl = rq_step(tm, n, t, dgb, egb, inv, s, a, col, &r, &nz);
                 const double s1 = s + dl;
                 if (!(s1 > lo && s1 < hi)) break;  // left the bracket
-                if (fabs(dl) <= 1e-14 || (fabs(dl) <= 1e-10 && fabs(dl) > 0.25 * prev)) {
+                if (fabs(dl) <= tol || (fabs(dl) <= 1e-10 && fabs(dl) > 0.25 * prev)) {
                     lam = s1;
                     done = true;  // the stored solutions belong to s
                     break;
@@ -1059,7 +1071,7 @@ void launch_polish_coefficients(int k, int m, const double* G, const double* H, 
 
 size_t blockeig_reflector_doubles(int n) { return (size_t)((n + 3) & ~3) * ((n + 1) / 2) * 2; }  // whole groups of kR rows
 
-size_t blockeig_rows_doubles(int n, int nblk) { return (size_t)10 * ((n + kGrp64 - 1) / kGrp64 * kGrp64) * nblk; }
+size_t blockeig_rows_doubles(int n, int nblk) { return (size_t)kRowArrays * ((n + kGrp64 - 1) / kGrp64 * kGrp64) * nblk; }
 
 size_t blockeig_compact_doubles(int n, int nblk) { return (size_t)((n - 2 + kR - 1) / kR) * nblk * kT; }
 
@@ -1084,7 +1096,7 @@ void launch_blockeig_spectrum(int n, int nblk, const double* dg, const double* e
 }
 
 void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long* launches) {
-    VecArgs a{p.n, p.nblk, p.ktot, p.kc, p.koff, p.dg, p.eg, p.scale, p.w, p.Z, p.K, p.X, p.Y, p.status};
+    VecArgs a{p.n, p.nblk, p.ktot, p.kc, p.koff, p.dg, p.eg, p.scale, p.w, p.Z, p.K, p.X, p.Y, p.rows > 0, p.status};
     int dev = 0, nsm = 0;
     OPSEC_CUDA(cudaGetDevice(&dev));
     OPSEC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1094,7 +1106,7 @@ void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long
     const dim3 grid(p.nblk, (p.kmax + 4 * per - 1) / (4 * per));
     if (g_clock) g_clock->begin("blockeig_pairs", s);
     const int np = (p.n + kGrp64 - 1) / kGrp64 * kGrp64;
-    rows_kernel<<<(np * p.nblk + 127) / 128, 128, 0, s>>>(p.n, p.nblk, p.dg, p.eg, p.scale, p.R);
+    rows_kernel<<<(np * p.nblk + 127) / 128, 128, 0, s>>>(p.n, p.nblk, p.dg, p.eg, p.scale, p.w, p.R);
     OPSEC_CUDA(cudaGetLastError());
     const size_t rows = sizeof(double) * 10 * (size_t)np;
     const size_t room = (size_t)max_dynamic_smem((const void*)vectors_kernel<true>);

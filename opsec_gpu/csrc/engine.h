@@ -237,7 +237,7 @@ struct BlockEigVectors {
     const double* tau;    // [nblk][n]
     double* T;            // scratch, blockeig_compact_doubles()
     double* R;            // scratch, blockeig_rows_doubles()
-    double* out;          // [nblk][n][n] eigenvector columns, or with rows > 0 (one block) [rows][n], largest first
+    double* out;          // [nblk][n][n] eigenvector columns, or with rows > 0 (one block, a polish to follow) [rows][n], largest first
     int rows;
 };
 size_t blockeig_compact_doubles(int n, int nblk);
