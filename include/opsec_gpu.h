@@ -122,7 +122,8 @@ int opsec_gpu_stage_times(const opsec_gpu* ctx, double* times);
 /* How the last eigensolve ran: stats[0] the solver (0 dense, 1 azimuthal
  * blocks, 2 Chebyshev-filtered subspace iteration -- klt.solver).  For 0 and 1, [4] is the
  * number of eigenvectors that the engine's own kernels computed, 0 when the library solved
- * (for 1 [1] is then 0, else 1).  For 2:
+ * (for 1 [1] is then 0, else 1); for 0, [8] counts the vectors whose eigenvalues lay
+ * so close that groups of them were diagonalised on the host.  For 2:
  * [1] filter iterations, [2] final Chebyshev degree, [3] N x N x B GEMMs, [4] block
  * size B, [5] [6] the spectrum bounds used, [7] the largest relative residual
  * |S x - lambda x| / lambda of the returned modes (FP64), [8] FP64 Rayleigh-Ritz

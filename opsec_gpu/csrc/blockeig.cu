@@ -30,6 +30,7 @@
 #include "df64.h"
 #include "engine.h"
 #include "packed.h"
+#include "polish.h"
 
 namespace opsec {
 namespace {
@@ -1029,23 +1030,48 @@ __global__ void __launch_bounds__(128) backtransform_kernel(VecArgs a, const flo
 
 // ---------------------------------------------------------------- polish of a dense solve
 // E of X <- X (I + E) and the Rayleigh quotients, from G = X^T X and H = X^T S X (Ogita and Aishima,
-// Japan J. Indust. Appl. Math. 35 (2018) 1007): with R = I - G, E_ij = (H_ij + l_j R_ij) / (l_j - l_i),
-// E_jj = R_jj / 2; eigenvalues too close to tell apart only have their vectors orthogonalised.
-__global__ void polish_kernel(int k, int m, const double* __restrict__ G, const double* __restrict__ H, double tol,
-                              double* __restrict__ E, double* __restrict__ lam) {
-    const long long n = (long long)k * m;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % k), j = (int)(t / k);
-        const double li = H[(size_t)i * k + i] / G[(size_t)i * k + i], lj = H[(size_t)j * k + j] / G[(size_t)j * k + j];
-        const size_t o = i >= j ? (size_t)j * k + i : (size_t)i * k + j;  // lower triangles
-        const double r = (i == j ? 1.0 : 0.0) - G[o];
-        double e = 0.5 * r;
-        if (i != j && fabs(lj - li) > tol) {
-            const double v = (H[o] + lj * r) / (lj - li);
-            if (fabs(v) < 1e-5) e = v;
+// Japan J. Indust. Appl. Math. 35 (2018) 1007): with R = I - G, E = R / 2 + K off the diagonal, K_ij =
+// (H_ij + (l_i + l_j) R_ij / 2) / (l_j - l_i) the couplings, and E_jj = R_jj / 2 - sum_i K_ij^2 / 2, which keeps
+// the norms to second order.  Counted are the vectors for which that is not enough (polish.h, which takes
+// them): a coupling above kCloseCoupling that is not rounding, or two with a product above kCloseProduct.
+// One warp a column; the k - m columns past the last only count, their couplings to the first m.
+__global__ void __launch_bounds__(128) polish_kernel(int k, int m, const double* __restrict__ G, const double* __restrict__ H,
+                                                     double* __restrict__ E, double* __restrict__ lam, int* close) {
+    const int lane = threadIdx.x & 31;
+    const double rounding = kCouplingRounding * fabs(H[0] / G[0]);
+    for (int j = blockIdx.x * 4 + (threadIdx.x >> 5); j < k; j += gridDim.x * 4) {
+        const double gj = G[(size_t)j * k + j], lj = H[(size_t)j * k + j] / gj;
+        double s2 = 0.0, a1 = 0.0, a2 = 0.0;  // sum of squares, the two largest
+        bool over = !isfinite(lj);
+        for (int i = lane; i < (j < m ? k : m); i += 32) {
+            if (i == j) continue;
+            const size_t o = i >= j ? (size_t)j * k + i : (size_t)i * k + j;  // lower triangles
+            const double g = G[o], li = H[(size_t)i * k + i] / G[(size_t)i * k + i];
+            const double h = H[o] - 0.5 * (li + lj) * g, d = lj - li;
+            double v = 0.0;
+            if (!(fabs(h) <= kCloseCoupling * fabs(d)))
+                over |= !(fabs(h) <= rounding);
+            else if (d != 0.0)
+                v = h / d;
+            s2 = fma(v, v, s2);
+            a2 = fmax(a2, fmin(a1, fabs(v)));
+            a1 = fmax(a1, fabs(v));
+            if (j < m) E[(size_t)j * k + i] = v - 0.5 * g;
         }
-        E[t] = e;
-        if (i == j) lam[j] = lj;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+            const double b1 = __shfl_xor_sync(0xffffffffu, a1, o), b2 = __shfl_xor_sync(0xffffffffu, a2, o);
+            a2 = fmax(fmax(a2, b2), fmin(a1, b1));
+            a1 = fmax(a1, b1);
+        }
+        over = __any_sync(0xffffffffu, over) || a1 * a2 > kCloseProduct;
+        if (lane) continue;
+        if (j < m) {
+            E[(size_t)j * k + j] = 0.5 * (1.0 - gj - s2);
+            lam[j] = lj;
+        }
+        if (over) atomicAdd(close, 1);
     }
 }
 
@@ -1061,10 +1087,9 @@ void launch_back(const VecArgs& a, const BlockEigVectors& p, int warps, cudaStre
 
 }  // namespace
 
-void launch_polish_coefficients(int k, int m, const double* G, const double* H, double tol, double* E, double* lam,
+void launch_polish_coefficients(int k, int m, const double* G, const double* H, double* E, double* lam, int* close,
                                 cudaStream_t s, long long* launches) {
-    const long long n = (long long)k * m;
-    polish_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 65536), 256, 0, s>>>(k, m, G, H, tol, E, lam);
+    polish_kernel<<<(unsigned)((k + 3) / 4), 128, 0, s>>>(k, m, G, H, E, lam, close);
     OPSEC_CUDA(cudaGetLastError());
     ++*launches;
 }

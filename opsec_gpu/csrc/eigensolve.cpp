@@ -1,6 +1,7 @@
 // eigensolve.cpp -- the KL eigensolve (klt.cpp:173-248): azimuthal blocks by the hand-written
 // block eigensolver or cuSOLVER, dense cuSOLVER syevdx, or the iterative solver.
 #include "context.h"
+#include "polish.h"
 #include "symmetry.h"
 
 bool azimuthal_ok(opsec_gpu* c, int ncells, const opsec_cell* cells) {
@@ -222,8 +223,8 @@ bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
     int kc = M;
     while (kc < n && w[n - 1 - kc] >= cut) kc++;
     kc = std::min(n, std::max(kc, M + std::max(32, M / 8)));  // a margin below the cut for the polish
-    const int hi[3] = {kc, 0, 0};
-    c->bev_i.alloc(3);
+    const int hi[4] = {kc, 0, 0, 0};  // candidates, first column, status, close couplings
+    c->bev_i.alloc(4);
     OPSEC_CUDA(cudaMemcpyAsync(c->bev_i.p, hi, sizeof hi, cudaMemcpyHostToDevice, c->stream));
     const size_t per = (size_t)n * kc;
     c->bev_vec.alloc(3 * per + (size_t)((n + 1) / 2) * kc);
@@ -258,7 +259,8 @@ bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
     if (g_clock) g_clock->end(c->stream);
     // The reduction and the back-transformation are good to 48 bits: vectors of neighbouring
     // eigenvalues are off by 1e-12 of each other.  One first-order correction in FP64 over the kept
-    // vectors and the margin brings them to what an FP64 solve gives.
+    // vectors and the margin brings them to what an FP64 solve gives; groups of eigenvalues closer than
+    // about 1e-6 of the largest are diagonalised (polish.h).
     if (!c->blas) blas_check(cublasCreate(&c->blas), "cublasCreate");
     blas_check(cublasSetStream(c->blas, c->stream), "cublasSetStream");
     const double one = 1.0, zero = 0.0;
@@ -266,19 +268,38 @@ bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
     blas_check(cublasDgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, n, kc, n, &one, c->S.p, n, X, n, &zero, SX, n), "dgemm");
     blas_check(cublasDsyrk(c->blas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, kc, n, &one, X, n, &zero, G, kc), "dsyrk");
     blas_check(cublasDgemm(c->blas, CUBLAS_OP_T, CUBLAS_OP_N, kc, kc, n, &one, X, n, SX, n, &zero, H, kc), "dgemm");
-    launch_polish_coefficients(kc, M, G, H, 1e-12 * sc, E, c->evals.p, c->stream, &c->launches);
-    OPSEC_CUDA(cudaMemcpyAsync(c->modes.p, X, sizeof(double) * (size_t)n * M, cudaMemcpyDeviceToDevice, c->stream));
-    blas_check(cublasDgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, n, M, kc, &one, X, n, E, kc, &one, c->modes.p, n), "dgemm");
+    launch_polish_coefficients(kc, M, G, H, E, c->evals.p, c->bev_i.p + 3, c->stream, &c->launches);
+    auto correct = [&] {
+        OPSEC_CUDA(cudaMemcpyAsync(c->modes.p, X, sizeof(double) * (size_t)n * M, cudaMemcpyDeviceToDevice, c->stream));
+        blas_check(cublasDgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, n, M, kc, &one, X, n, E, kc, &one, c->modes.p, n), "dgemm");
+    };
+    correct();
     c->launches += 4;
     if (g_clock) g_clock->end(c->stream);
-    int st = 0;
+    int st[2] = {0, 0};
     std::vector<double> ev(M);
     OPSEC_CUDA(cudaMemcpyAsync(ev.data(), c->evals.p, sizeof(double) * M, cudaMemcpyDeviceToHost, c->stream));
-    OPSEC_CUDA(cudaMemcpyAsync(&st, p.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    OPSEC_CUDA(cudaMemcpyAsync(st, p.status, sizeof st, cudaMemcpyDeviceToHost, c->stream));
     sync(c);
-    if (st) {
-        c->warning = "dense eigensolver check " + std::to_string(st) + " failed; solved by cuSOLVER instead";
+    if (st[0]) {
+        c->warning = "dense eigensolver check " + std::to_string(st[0]) + " failed; solved by cuSOLVER instead";
         return false;
+    }
+    if (st[1]) {  // eigenvalues too close for a first-order correction: on the host, and the product again
+        const size_t kk = (size_t)kc * kc;
+        std::vector<double> hG(kk), hH(kk), hE((size_t)kc * M);
+        OPSEC_CUDA(cudaMemcpyAsync(hG.data(), G, sizeof(double) * kk, cudaMemcpyDeviceToHost, c->stream));
+        OPSEC_CUDA(cudaMemcpyAsync(hH.data(), H, sizeof(double) * kk, cudaMemcpyDeviceToHost, c->stream));
+        sync(c);
+        if (!polish_close(kc, M, hG.data(), hH.data(), hE.data(), ev.data())) {
+            c->warning = "dense eigensolver: too many close eigenvalues; solved by cuSOLVER instead";
+            return false;
+        }
+        OPSEC_CUDA(cudaMemcpyAsync(E, hE.data(), sizeof(double) * hE.size(), cudaMemcpyHostToDevice, c->stream));
+        correct();
+        sync(c);  // hE goes out of scope
+        c->launches++;
+        c->eig_stats[8] = st[1];
     }
     c->eig_stats[4] = kc;  // only now: the library's solve leaves it 0
     std::stable_sort(ev.begin(), ev.end(), std::greater<double>());  // refined one by one: equal to rounding

@@ -243,9 +243,10 @@ struct BlockEigVectors {
 size_t blockeig_compact_doubles(int n, int nblk);
 size_t blockeig_rows_doubles(int n, int nblk);
 void launch_blockeig_vectors(const BlockEigVectors& p, cudaStream_t s, long long* launches);
-// First-order correction X (I + E) of k approximate eigenvectors from G = X^T X and H = X^T S X
-// (k x k, lower triangles read): the k x m columns of E for the first m and their Rayleigh quotients.
-void launch_polish_coefficients(int k, int m, const double* G, const double* H, double tol, double* E, double* lam,
+// Correction X (I + E) of k approximate eigenvectors from G = X^T X and H = X^T S X (k x k, lower triangles
+// read): the k x m columns of E for the first m and their Rayleigh quotients.  *close += the vectors for which
+// it is not enough (polish.h).
+void launch_polish_coefficients(int k, int m, const double* G, const double* H, double* E, double* lam, int* close,
                                 cudaStream_t s, long long* launches);
 
 // The same for small surveys (blockeig_small.cu): A is overwritten.
