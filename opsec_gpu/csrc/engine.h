@@ -149,6 +149,7 @@ struct XiTableArgs {
     double* xi64;           // [1+nbands][n] out
     float* xi32;            // [1+nbands][n] out
     double band_wmax;       // widest band, max |band_hi - band_lo|
+    double pk_unit;         // power of two that brings max |P| to [128, 256)
     double* scratch;        // xi_scratch_doubles() doubles
 };
 size_t xi_scratch_doubles(const XiTableArgs& a);  // reads xl, nbands and band_wmax

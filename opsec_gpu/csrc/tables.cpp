@@ -31,6 +31,11 @@ void build_tables(opsec_gpu* c) {
     a.nbands = nb;
     a.band_wmax = 0.0;
     for (int p = 0; p < nb; p++) a.band_wmax = std::max(a.band_wmax, std::fabs(c->band_hi[p] - c->band_lo[p]));
+    double pmax = 0.0;
+    for (double P : c->pk_P) pmax = std::max(pmax, std::fabs(P));
+    int e = 8;
+    if (pmax > 0.0) std::frexp(pmax, &e);
+    a.pk_unit = std::ldexp(1.0, std::max(-1000, std::min(1000, 8 - e)));  // it and its inverse are normal numbers
     c->scratch.alloc(xi_scratch_doubles(a));
     a.pk_x = c->pk_dev.p;
     a.pk_y = a.pk_x + npk;

@@ -32,7 +32,9 @@ namespace {
 constexpr int kNkXi = 32768;
 constexpr int kNkBand = 8192;
 constexpr double kTwoPi2 = 2.0 * M_PI * M_PI;
-constexpr double kScale = 1099511627776.0;  // 2^40: keeps the highest moments clear of FP32 underflow
+// 2^40: keeps the highest moments clear of FP32 underflow.  Table 0 is summed in units of P(k) besides
+// (pk_unit), whose own scale FP32's range would not hold: 2^90 times the ordinary one overflows.
+constexpr double kScale = 1099511627776.0;
 constexpr int kP = 24;                      // moments per block
 constexpr int kAnchor = 16;                 // recurrence steps between rotation anchors
 constexpr double kZmax = 2.0;
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(256) xi_moments_kernel(XiPlan p) {
         const double k = s.kmin + j * dk, k2 = k * k;
         df P = wcd;
         if (t == 0)
-            P = df_from(wc * spline_eval(p.a.npk, p.a.pk_x, p.a.pk_y, p.a.pk_b, p.a.pk_c, p.a.pk_d, k));
+            P = df_from(wc * p.a.pk_unit * spline_eval(p.a.npk, p.a.pk_x, p.a.pk_y, p.a.pk_b, p.a.pk_c, p.a.pk_d, k));
         else if (!(k >= s.kmin && k < s.kmax))  // ConstantSpline(1, kmin, kmax)
             P = df{0.f, 0.f};
         const float mult = 2 + 2 * (j % 2) - (j == 0) - (j == s.nk);
@@ -413,6 +415,7 @@ __global__ void __launch_bounds__(128) xi_finish_kernel(XiPlan p) {
             acc -= (double)w * (r2 * r2) * (1.0 / 60.0);
         }
     }
+    if (t == 0) acc *= 1.0 / p.a.pk_unit;
     p.a.xi64[(size_t)t * p.n + i] = acc;
     p.a.xi32[(size_t)t * p.n + i] = (float)acc;
 }
