@@ -664,8 +664,8 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
         // Converged when the correction is below 1e-14 of the block scale (T is scaled to norm < 1) and
         // 1e-10 of the distance to the next eigenvalue: the vector is that of the shift before the
         // correction, off by their quotient (left to the polish where there is one: 0.12 ms at 1,728
-        // rows); or when it stops shrinking at a level below 1e-10 (the
-        // rounding floor of gamma)
+        // rows); or when it stops shrinking at the rounding of gamma.  One that stops shrinking above
+        // that, between eigenvalues some 1e-10 apart, is bracketed by Sturm counts instead.
         const double tol = a.polished ? 1e-14 : fmin(1e-14, fmax(0.5 * DBL_EPSILON, 1e-10 * gaps[j]));
         double s = fmin(fmax(x, lo), hi), prev = 1.0;
         {
@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* _
                 const double dl = rq_step(tm, n, t, dgb, egb, inv, s, a, col, &r, &nz);
                 const double s1 = s + dl;
                 if (!(s1 > lo && s1 < hi)) break;  // left the bracket
-                if (fabs(dl) <= tol || (fabs(dl) <= 1e-10 && fabs(dl) > 0.25 * prev)) {
+                if (fabs(dl) <= tol || (fabs(dl) <= 16.0 * DBL_EPSILON && fabs(dl) > 0.25 * prev)) {
                     lam = s1;
                     done = true;  // the stored solutions belong to s
                     break;

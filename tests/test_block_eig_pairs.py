@@ -20,3 +20,24 @@ def test_vectors_of_close_pairs_are_orthogonal(dims):
     # its shift's error over the distance: two units in the last place of an eigenvalue of that scale,
     # 4.4e-16 / 1e-6, of each of the two
     assert np.max(np.abs(B @ B.T - np.eye(M))) <= 9e-10
+
+
+@pytest.mark.parametrize("dims,thickness,part", [((37, 15, 16), 60.0, 1), ((37, 15, 16), 20.0, 4), ((20, 31, 14), 100.0, 1),
+                                                 ((20, 32, 14), 20.0, 1)])
+def test_thin_shells(dims, thickness, part):
+    """Shells far thinner than the correlation length: most eigenvalues of a block are close to others."""
+    sv, cells = synth.shell_survey(*dims, rmin=200.0, rmax=200.0 + thickness, rc=200.0 + thickness / 2, width=thickness / 2)
+    M = cells.size // part
+    ev = {}
+    for eig in ("own", "batched"):
+        with api.Engine(api.make_config(sv, bands=synth.band_edges(2, 0.0, 0.1), extra=(f"azimuthal.eig = {eig}",))) as e:
+            e.set_pk(*synth.pk_table())
+            ev[eig], B = e.klt(cells, M)
+            if eig == "own":
+                assert e.eig_stats()["iterations"] == 1
+                S, own = e.signal_block(cells), B
+    lam0 = ev["batched"][0]
+    # as the block eigensolver's other tests; orthogonality as above
+    assert np.max(np.abs(ev["own"] - ev["batched"])) <= 1e-11 * lam0
+    assert np.max(np.abs(own @ S - ev["own"][:, None] * own)) <= 1e-11 * lam0
+    assert np.max(np.abs(own @ own.T - np.eye(M))) <= 9e-10
