@@ -82,9 +82,8 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     double* scale = eg + (size_t)nblk * n;
     const bool small = small_survey(npar, (long long)n * npar * Nphi);
     c->bev_err.alloc(1);
-    OPSEC_CUDA(cudaMemsetAsync(c->bev_err.p, 0, sizeof(int), c->stream));
     if (!small) c->bev_D.alloc(tridiag_work_bytes(n, nblk));
-    launch_block_unit(n, nblk, c->S.p, unit, c->stream, &c->launches);
+    launch_block_unit(n, nblk, c->S.p, unit, c->bev_err.p, c->stream, &c->launches);
     if (g_clock) g_clock->begin("blockeig_tridiag", c->stream, 4.0 / 3.0 * n * nn * nblk);
     if (small)
         launch_small_tridiag(n, nblk, c->S.p, unit, c->bev_V.p, tau, dg, eg, c->stream, &c->launches);
@@ -99,10 +98,7 @@ bool own_block_eigensolve(opsec_gpu* c, int n, int nblk, int npar, int Nphi, int
     std::vector<double> w((size_t)nblk * n), sc(nblk);
     OPSEC_CUDA(cudaMemcpyAsync(w.data(), c->W.p, sizeof(double) * w.size(), cudaMemcpyDeviceToHost, c->stream));
     OPSEC_CUDA(cudaMemcpyAsync(sc.data(), scale, sizeof(double) * nblk, cudaMemcpyDeviceToHost, c->stream));
-    int err = 0;
-    OPSEC_CUDA(cudaMemcpyAsync(&err, c->bev_err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    sync(c);
-    if (err) fail(OPSEC_ERR_CUDA, "tridiagonalisation: a wait between CTAs timed out");
+    sync(c);  // no wait between CTAs but the hardware's cluster barrier: no error word to read
     // the M-th largest approximate eigenvalue, counting the (cos, sin) pairs of 0 < m < Nphi/2 twice
     std::vector<double> all;
     all.reserve((size_t)2 * nblk * n);
@@ -203,8 +199,7 @@ bool own_dense_eigensolve(opsec_gpu* c, int n, int M) {
     c->W.alloc(n);
     c->bev_D.alloc(tridiag_work_bytes(n, 1));
     c->bev_err.alloc(1);
-    OPSEC_CUDA(cudaMemsetAsync(c->bev_err.p, 0, sizeof(int), c->stream));
-    launch_block_unit(n, 1, c->S.p, unit, c->stream, &c->launches);
+    launch_block_unit(n, 1, c->S.p, unit, c->bev_err.p, c->stream, &c->launches);
     if (g_clock) g_clock->begin("blockeig_tridiag", c->stream, 4.0 / 3.0 * n * nn);
     launch_tridiag(n, 1, true, c->S.p, unit, c->bev_V.p, tau, dg, eg, c->bev_D.p, c->bev_err.p, c->proj_wait, c->stream,
                    &c->launches);

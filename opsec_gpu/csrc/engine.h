@@ -149,7 +149,7 @@ struct XiTableArgs {
     double* xi64;           // [1+nbands][n] out
     float* xi32;            // [1+nbands][n] out
     double band_wmax;       // widest band, max |band_hi - band_lo|
-    double pk_unit;         // power of two that brings max |P| to [128, 256)
+    double pk_unit, pk_back;  // power of two that brings max |P| to [128, 256), and its inverse
     double* scratch;        // xi_scratch_doubles() doubles
 };
 size_t xi_scratch_doubles(const XiTableArgs& a);  // reads xl, nbands and band_wmax
@@ -209,15 +209,16 @@ void launch_assemble_modes(int H, int Nphi, int Nmu, int npar, int nmodes, const
 bool blockeig_supported(int n);
 // Householder tridiagonalisation (tridiag.cu) of nblk blocks of order n >= 3 (FP64, column-major,
 // lower triangle read): T = (dg, eg), the reflectors V[block][c][i/2] as (hi, hi, lo, lo) floats of
-// entries i and i + 1 (v[c+1] = 1) and tau, each [block][n].  work: tridiag_work_bytes() bytes.  *err (zeroed by the
-// caller) is set when a wait between CTAs ran out.  chip: one block on the whole GPU instead of a
+// entries i and i + 1 (v[c+1] = 1) and tau, each [block][n].  work: tridiag_work_bytes() bytes.  *err (cleared by
+// launch_block_unit) is set when a wait between CTAs ran out.  chip: one block on the whole GPU instead of a
 // cluster (a cooperative launch; tridiag_chip_supported).
 // doubles of one block's reflectors (the small surveys' [n][n] pairs fit as well)
 size_t blockeig_reflector_doubles(int n);
 size_t tridiag_work_bytes(int n, int nblk);
 bool tridiag_chip_supported(int n);
-// unit: [block] (power of two, its inverse) by which the reduction scales A, from launch_block_unit
-void launch_block_unit(int n, int nblk, const double* A, double* unit, cudaStream_t s, long long* launches);
+// unit: [block] (power of two, its inverse) by which the reduction scales A, from launch_block_unit,
+// which also clears *err
+void launch_block_unit(int n, int nblk, const double* A, double* unit, int* err, cudaStream_t s, long long* launches);
 void launch_tridiag(int n, int nblk, bool chip, const double* A, const double* unit, double* V, double* tau, double* dg,
                     double* eg, void* work, int* err, long long wait_cycles, cudaStream_t s, long long* launches);
 void launch_blockeig_spectrum(int n, int nblk, const double* dg, const double* eg, double* w, double* scale,

@@ -94,8 +94,9 @@ struct TridiagArgs {
     long long wait_cycles;
 };
 
-// (2^-e, 2^e) of each block, 2^e > its largest |diagonal entry| >= 2^(e-1): one CTA a block
-__global__ void __launch_bounds__(256) unit_kernel(int n, const double* __restrict__ A, double2* __restrict__ unit) {
+// (2^-e, 2^e) of each block, 2^e > its largest |diagonal entry| >= 2^(e-1): one CTA a block.  Clears the
+// reduction's error word on the way.
+__global__ void __launch_bounds__(256) unit_kernel(int n, const double* __restrict__ A, double2* __restrict__ unit, int* err) {
     __shared__ double red[8];
     const double* Ab = A + (size_t)blockIdx.x * n * n;
     double m = 0.0;
@@ -105,6 +106,7 @@ __global__ void __launch_bounds__(256) unit_kernel(int n, const double* __restri
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x) return;
+    if (blockIdx.x == 0) *err = 0;
     for (int w = 1; w < 8; w++) m = fmax(m, red[w]);
     int e = 0;
     if (m > 0.0 && isfinite(m)) frexp(m, &e);
@@ -642,8 +644,8 @@ bool tridiag_chip_supported(int n) {
            smem_base(n, 152, kChipT / 32, 2) <= (size_t)max_dynamic_smem((const void*)tridiag_kernel<kChipT, 2, 4 * kElems, true>);
 }
 
-void launch_block_unit(int n, int nblk, const double* A, double* unit, cudaStream_t s, long long* launches) {
-    unit_kernel<<<nblk, 256, 0, s>>>(n, A, reinterpret_cast<double2*>(unit));
+void launch_block_unit(int n, int nblk, const double* A, double* unit, int* err, cudaStream_t s, long long* launches) {
+    unit_kernel<<<nblk, 256, 0, s>>>(n, A, reinterpret_cast<double2*>(unit), err);
     OPSEC_CUDA(cudaGetLastError());
     ++*launches;
 }

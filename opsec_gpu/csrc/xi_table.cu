@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(128) xi_finish_kernel(XiPlan p) {
             acc -= (double)w * (r2 * r2) * (1.0 / 60.0);
         }
     }
-    if (t == 0) acc *= 1.0 / p.a.pk_unit;
+    if (t == 0) acc *= p.a.pk_back;
     p.a.xi64[(size_t)t * p.n + i] = acc;
     p.a.xi32[(size_t)t * p.n + i] = (float)acc;
 }
