@@ -581,7 +581,7 @@ __global__ void rows_kernel(int n, int nblk, const double* __restrict__ dg, cons
 // Bound by the FP64 pipe (64 cycles an instruction, measured, with nothing to overlap) and by loads of the stored solutions (32 rows at a time: row by row their latency was half the kernel).
 // Candidates of 34 blocks of 512^2 (4,351): 4.51 -> 1.15 ms against FP64 pivots with a division in
 // every row; 34 of 1024^2 25.5 -> 3.77, 10 of 555^2 12.5 -> 2.01, 18 of 64^2 0.406 -> 0.092; with the lanes in teams
-// 34 of 512^2 0.90 -> 0.45, 10 of 555^2 0.98 -> 0.46, one of 1728^2 5.11 -> 1.61, of 3150^2 6.05 -> 2.69.
+// 34 of 512^2 0.90 -> 0.46, 10 of 555^2 0.98 -> 0.46, one of 1728^2 5.11 -> 1.70, of 3150^2 6.05 -> 2.66.
 // LOCAL: the block's rows in shared memory; otherwise (orders whose rows do not fit) read through L1.
 template <bool LOCAL>
 __global__ void __launch_bounds__(128) vectors_kernel(VecArgs a, const double* __restrict__ R, int per, int team) {

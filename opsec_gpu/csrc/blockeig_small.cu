@@ -2,14 +2,16 @@
 // triangle on clusters of four CTAs for the reduction, FP64 pivots (a division a row) for the
 // candidates and one reflector at a time for the back-transformation.
 //
-// It is slower from about 64 rows a block on.  It stays because the last digits of a small survey's
-// Fisher matrix hang on its vectors: C_p is formed and rounded in FP32 in the basis of the block's
-// eigenvectors, and where a block holds nearly degenerate pairs (an odd number of mu cells leaves
-// the even and the odd modes in one block) rounding decides which basis of a pair that is.  Another
-// solver of equal accuracy moves F, f and q by up to 2e-8 of their norm on surveys under 4,096
-// cells (24 of 58 drawn ones by over 1e-9), by at most 9e-10 to 8,192 cells and 5e-10 beyond; with an
-// even number of mu cells by at most 4e-10 from 1,024 cells on.  The estimates' own error is 1e-7.
-// own_block_eigensolve draws the line.
+// It is slower from about 64 rows a block on: a 37 x 15 x 14 survey (7,770 cells, these kernels) takes 26.1
+// ms a build, a 37 x 15 x 18 one (9,990 cells, the others) 17.3; 12 x 12 x 7 2.75 and 12 x 12 x 8 2.24.  It
+// stays because the last digits of a small survey's Fisher matrix hang on its vectors: C_p is formed and
+// rounded in FP32 in the basis of the block's eigenvectors, and where a block holds nearly degenerate pairs
+// (an odd number of mu cells leaves the even and the odd modes in one block) rounding decides which
+// basis of a pair that is.  Another solver of equal accuracy moves F, f and q by up to 2e-8 of their norm
+// on surveys under 4,096 cells, by at most 9e-10 to 8,192 cells and 5e-10 beyond; with an even number of mu
+// cells by at most 4e-10 from 1,024 cells on.  Neither is nearer the truth (the estimates' own error is
+// 1e-7): own_block_eigensolve draws the line where such a survey's results stay within 1e-9 of what
+// they have been, not where these kernels stop being the faster or the better ones.
 #include <cooperative_groups.h>
 
 #include <cfloat>

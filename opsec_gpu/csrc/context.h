@@ -47,7 +47,7 @@ void launch_fisher64(const FisherArgs& a, const double* Dp64, cudaStream_t s, lo
 void launch_reverse_modes(int n, int m, int lda, const double* A, const double* w, double* modes, double* evals,
                           cudaStream_t s, long long* launches);
 // klt.solver = auto: the subspace iteration from this many cells on (and a block of at most
-// a quarter of them); the dense FP64 syevdx below
+// a quarter of them); below, the own dense solver or syevdx (eigensolve.cpp)
 constexpr int kChfsiMinCells = 16384;
 void blas_check(cublasStatus_t st, const char* what);
 void solver_check(cusolverStatus_t st, const char* what);

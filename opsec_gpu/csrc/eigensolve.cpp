@@ -1,5 +1,6 @@
-// eigensolve.cpp -- the KL eigensolve (klt.cpp:173-248): azimuthal blocks by the hand-written
-// block eigensolver or cuSOLVER, dense cuSOLVER syevdx, or the iterative solver.
+// eigensolve.cpp -- the KL eigensolve (klt.cpp:173-248): azimuthal blocks by the hand-written block
+// eigensolver or cuSOLVER; a dense S by the same kernels on the whole chip, cuSOLVER's syevdx or the
+// iterative solver.
 #include "context.h"
 #include "polish.h"
 #include "symmetry.h"
@@ -55,15 +56,15 @@ void drop_eig_graph(opsec_gpu* c) {
 }
 
 // Dense problems of this order on (to tridiag_chip_supported's limit, 4,096) take the engine's own
-// kernels, open box with all else equal, top 29 %: 512 cells 14.9 -> 4.3 ms, 990 31.5 -> 10.4, 1,728
-// 67.7 -> 30.4, 2,730 156.6 -> 85.  Smaller ones gain as much (294 cells 9.0 -> 2.3 ms) but stay with
-// cuSOLVER: their C_p, rounded to FP32 in few modes, moves q by up to 1e-9 with any other rounding
-// of the vectors.  So do exactly degenerate S (symmetry.h), whose basis rounding picks and two of whose
+// kernels (top quarter of an open box by cuSOLVER and by them: 512 cells 14.9 and 3.5 ms, 990 31.5 and 8.6,
+// 1,728 67.7 and 24, 2,744 157 and 73).  Smaller ones would gain as much (294 cells 9.0 and 2.3 ms) but
+// stay with cuSOLVER, as small_survey's do with their kernels: C_p, rounded to FP32 in few modes, moves
+// q by up to 1e-9 with any other rounding of the vectors.  So do exactly degenerate S (symmetry.h), whose basis rounding picks and two of whose
 // separately computed vectors may come out parallel.
 constexpr int kOwnDenseMin = 512;
 
-// Surveys whose Fisher matrix moves by over 1e-9 with the eigensolver's rounding (blockeig_small.cu):
-// few cells, or blocks that keep the modes even and odd in mu together (npar = 1) and not many cells.
+// Surveys whose Fisher matrix moves by over 1e-9 with the eigensolver's rounding (blockeig_small.cu says
+// why, and what that costs): few cells, or blocks that keep the modes even and odd in mu together (npar = 1) and not many cells.
 bool small_survey(int npar, long long cells) { return cells < 1024 || (npar == 1 && cells < 8192); }
 
 // The hand-written block eigensolver (blockeig.cu, blockeig_small.cu) on the nblk blocks of order n in c->S:
@@ -529,7 +530,8 @@ int eigensolve(opsec_gpu* c, int ncells, const opsec_cell* cells, int M, bool wa
     }
     drop_eig_graph(c);
     c->modes_ok = true;  // the dense and iterative solvers write the modes directly
-    // dense path: S in FP64, top-M by syevdx or by subspace iteration (klt.cpp:173-248 via PARPACK there)
+    // dense path: S in FP64, top-M by the own kernels, syevdx or subspace iteration (klt.cpp:173-248 via
+    // PARPACK there)
     const int N = ncells;
     c->S.alloc((size_t)N * N);
     std::vector<int> all(N);

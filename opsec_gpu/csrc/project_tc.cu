@@ -669,7 +669,7 @@ Layout layout_of(const ProjectArgs& a) {
     L.Npad = (a.ncells + BM - 1) / BM * BM;
     L.Mpad = (a.nmodes + BN - 1) / BN * BN;
     const size_t half_mat = (size_t)L.Mpad * L.Npad * sizeof(__half);
-    // Bands of one launch: a band is few tiles (step 1 26, step 2 5 at 1,575 cells and 588 modes, 101 and
+    // Bands of one launch: a band is few tiles (step 1 26, step 2 5 at 1,575 cells and 300 modes, 101 and
     // 65 us each whatever the number), so bands share launches until step 2, the smaller grid, has kWaves
     // waves of one-CTA SMs, as far as kBatchBytes of T and tables go (a 1,575-cell comma over 20 bands
     // 4.22 ms one at a time, 0.77 ms so; larger batches would fill no more SMs and leave L2 sooner).

@@ -118,8 +118,8 @@ __device__ TableSpec table_spec(const XiPlan& p, int t) {
     return s;
 }
 
-// exp(-x), x = k^2 >= 0, times 2^40, in double-FP32: the argument is reduced by ln 2 in FP64, the
-// Taylor series on |y| <= ln 2 / 2 runs to y^13 (the next term is below 5e-18).
+// exp(-x), x = k^2 >= 0, times 2^40, in double-FP32: the argument is reduced by ln 2 in two parts (Cody and
+// Waite, Software Manual for the Elementary Functions, 1980) in FP64, the Taylor series on |y| <= ln 2 / 2 runs to y^13 (the next term is below 5e-18).
 __device__ __forceinline__ df exp_neg_scaled(double x) {
     constexpr double kMagic = 6755399441055744.0;  // 1.5 2^52: adding it rounds to an integer
     constexpr double kLn2Hi = 6.93147180559945286227e-01, kLn2Lo = 2.31904681384629955842e-17;
