@@ -23,17 +23,14 @@ class Symmetry {
   public:
     // coordsys 1 Cartesian (L > 0: periodic), 2 spherical; b: Min1, Max1, ...; n: cells an axis
     Symmetry(int coordsys, const double* b, const int* n, double L, bool full_phi, int ncells, const opsec_cell* cells)
-        : coordsys_(coordsys), L_(L), full_phi_(full_phi), cells_(cells, cells + ncells) {
+        : coordsys_(coordsys), L_(L), full_phi_(full_phi), cells_(cells), ncells_(ncells) {
         for (int p = 0; p < 3; p++) {
             n_[p] = n[p];
             h_[p] = (b[2 * p + 1] - b[2 * p]) / n[p];
         }
-        at_.reserve(ncells);
-        for (const opsec_cell& c : cells_) at_.emplace_back(id(c.d1, c.d2, c.d3), c.Nbar);
-        std::sort(at_.begin(), at_.end());
     }
 
-    bool forces_degeneracy() const {
+    bool forces_degeneracy() {
         if (coordsys_ == 2) return full_phi_ && shifted(2);
         for (int p = 0; p < 3; p++) {
             const int q = (p + 1) % 3, r = (p + 2) % 3;
@@ -68,16 +65,23 @@ class Symmetry {
     int coordsys_, n_[3];
     double h_[3], L_;
     bool full_phi_;
-    std::vector<opsec_cell> cells_;
-    std::vector<std::pair<long long, double>> at_;  // (grid cell, Nbar), sorted
+    const opsec_cell* cells_;
+    int ncells_;
+    std::vector<std::pair<long long, double>> at_;  // (grid cell, Nbar), sorted; filled for the first motion
 
     static bool close(double x, double y) { return std::fabs(x - y) <= 1e-9 * std::max(std::fabs(x), std::fabs(y)); }
     bool alike(int p, int q) const { return n_[p] == n_[q] && close(h_[p], h_[q]); }
     long long id(int d1, int d2, int d3) const { return ((long long)d1 * n_[1] + d2) * n_[2] + d3; }
 
     template <class Motion>
-    bool maps_onto_itself(Motion g) const {
-        for (const opsec_cell& c : cells_) {
+    bool maps_onto_itself(Motion g) {
+        if (at_.empty()) {
+            at_.reserve(ncells_);
+            for (int a = 0; a < ncells_; a++) at_.emplace_back(id(cells_[a].d1, cells_[a].d2, cells_[a].d3), cells_[a].Nbar);
+            if (!std::is_sorted(at_.begin(), at_.end())) std::sort(at_.begin(), at_.end());
+        }
+        for (int a = 0; a < ncells_; a++) {
+            const opsec_cell& c = cells_[a];
             int d[3] = {c.d1, c.d2, c.d3};
             g(d);
             const std::pair<long long, double> key(id(d[0], d[1], d[2]), -HUGE_VAL);
@@ -88,9 +92,10 @@ class Symmetry {
     }
     // ... and is of order three or more on its cells
     template <class Motion>
-    bool turns(Motion g) const {
+    bool turns(Motion g) {
         if (!maps_onto_itself(g)) return false;
-        for (const opsec_cell& c : cells_) {
+        for (int a = 0; a < ncells_; a++) {
+            const opsec_cell& c = cells_[a];
             int d[3] = {c.d1, c.d2, c.d3};
             g(d);
             g(d);
@@ -100,7 +105,7 @@ class Symmetry {
     }
     // invariant under a cyclic shift of axis p by n/4 or by n over an odd number (every cyclic group of
     // order above two holds one of these)
-    bool shifted(int p) const {
+    bool shifted(int p) {
         const int n = n_[p];
         for (int k = 3; k <= n; k++)
             if (n % k == 0 && (k == 4 || k % 2) && turns([=](int* d) { d[p] = (d[p] + n / k) % n; })) return true;
